@@ -28,6 +28,10 @@ SOURCES = [
     "coo_build.cu",
     "init.cu",
     "sweep_fp32.cu",
+    "sweep_fp32_p32.cu",
+    "sweep_fp32_p64.cu",
+    "sweep_fp32_p128.cu",
+    "sweep_fp32_p192.cu",
     "sweep_tc.cu",
     "sweep_tc_fp32.cu",
     "sweep_tc_fp64.cu",

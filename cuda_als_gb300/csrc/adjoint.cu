@@ -8,10 +8,12 @@
 //           + sum_{u in H(i)} -2 (r_ui - x_u . y_i) x_u
 //   dL/dlambda = -sum_u n_u g_u . x_u
 // Two kernels, each in FP32 or FP64 (T):
-//   adjoint_row_kernel: one CTA per user row — the Gram of [Y | r] in register tiles (as in
-//     sweep_fp32.cu, the right-hand side summed apart with compensation), the L D L^T factor in
-//     shared memory, the forward solve, the row's held-out terms (in order: h_u and the loss),
+//   adjoint_tile_kernel (FP32, f <= 175) and adjoint_row_kernel (FP64, and FP32 above): one CTA
+//     per user row — the Gram (the right-hand side summed apart with compensation), its
+//     L D L^T factor, the forward solve, the row's held-out terms (in order: h_u and the loss),
 //     the second solve with the same factor; writes x_u and g_u, the loss and dL/dlambda parts.
+//     The tile kernel keeps the matrix in registers (tilesolve.cuh), the row kernel factors it in
+//     shared memory a column at a time; FP32 results are the same to the bit.
 //   adjoint_chunk_kernel + adjoint_combine_kernel: dL/dy_i from the item's training column (the
 //     CSC) in chunks of 2,048 ratings (one CTA each: heavy items spread over many) and its
 //     held-out ratings; every sum in a fixed order (warps, then chunks): deterministic, no
@@ -28,6 +30,7 @@
 #include "internal.h"
 #include "solvers.cuh"
 #include "tc.h"
+#include "tilesolve.cuh"
 
 namespace als {
 namespace {
@@ -260,6 +263,119 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 512 : 1024)
     }
 }
 
+template <int P>
+inline size_t tile_smem(int f) {
+    return sizeof(float) * (tile::shared_floats<P>(tile::nb_of(f), false) + 8);
+}
+
+// The FP32 row step for f <= 175 with the matrix in registers, one 8 x 8 tile a thread.
+template <int P>
+__global__ void __launch_bounds__(512) adjoint_tile_kernel(const AdjArgs<float> a, const int nb) {
+    extern __shared__ __align__(16) unsigned char smem_bytes[];
+    __shared__ double dsh[33];
+    const int f = a.f;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
+    const tile::Shared s = tile::carve<P>(reinterpret_cast<float *>(smem_bytes), nb, false);
+    float *red = reinterpret_cast<float *>(s.bad) + 8;  // 8 floats (f <= 175)
+    const int row = blockIdx.x;
+    const int beg = a.ptr[row], end = a.ptr[row + 1], nu = end - beg;
+    const int hbeg = a.hptr[row], hend = a.hptr[row + 1];
+    float *xr = a.X + (int64_t)row * f, *gr = a.G + (int64_t)row * f;
+    float *xo = a.Xout + (int64_t)row * f;
+    double loss = 0.0;
+
+    auto no_gradient = [&]() {  // x = 0: held-out residuals are r itself, no path through x
+        for (int i = tid; i < f; i += nt) {
+            xo[i] = 0.f;
+            xr[i] = 0.f;
+            gr[i] = 0.f;
+        }
+        for (int e = hbeg + tid; e < hend; e += nt) loss += (double)a.hval[e] * a.hval[e];
+        const double l = block_sum_d(loss, dsh);
+        if (tid == 0) {
+            a.loss_part[row] = l;
+            a.dlam_part[row] = 0.0;
+        }
+    };
+    if (nu == 0) {
+        no_gradient();
+        return;
+    }
+    if (tid == 0) *s.bad = 0;
+    const tile::Tile t = tile::tile_of<P>(tid, nb, false);
+    tile::Acc acc;
+    tile::clear(acc);
+    float2 bsum = make_float2(0.f, 0.f), bcomp = bsum;
+    tile::accumulate<P>(a.idx, a.val, a.Y, f, nb, beg, end, t, t.on, acc, bsum, bcomp, s.big, s.rv);
+    tile::add_diagonal(acc, t, f, (float)nu * a.lambda);
+    if (2 * tid < f) *reinterpret_cast<float2 *>(s.vb + 2 * tid) = bsum;
+    for (int i = f + (f & 1) + tid; i < 8 * nb; i += nt) s.vb[i] = 0.f;
+    __syncthreads();
+    const bool ok = tile::factor<false, P>(acc, t, f, nb, s);
+    if (ok) tile::backward<false>(s.vb, s.vx, f, nb, s);
+    int bad = 0;
+    for (int i = tid; ok && i < f; i += nt) bad |= isfinite(s.vx[i]) ? 0 : 1;
+    if (__syncthreads_or(bad) || !ok) {  // non-positive pivot: x = 0, flagged, no gradient
+        if (tid == 0) atomicAdd(&a.flags[0], 1);
+        no_gradient();
+        return;
+    }
+    for (int i = tid; i < 8 * nb; i += nt) {
+        s.vb[i] = 0.f;
+        if (i < f) {
+            const float x = s.vx[i];
+            xr[i] = x;
+            xo[i] = x;
+        }
+    }
+    __syncthreads();
+    // held-out terms: loss and h = dL/dx, walked in order by warp 0 (deterministic)
+    if (warp == 0) {
+        for (int e = hbeg; e < hend; ++e) {
+            const float *y = a.Y + (int64_t)a.hidx[e] * f;
+            float d = 0.f;
+            for (int j = lane; j < f; j += 32) d = fmaf(s.vx[j], y[j], d);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            const float res = a.hval[e] - d;
+            if (lane == 0) loss += (double)res * (double)res;
+            for (int j = lane; j < f; j += 32) s.vb[j] += -2.f * res * y[j];
+            __syncwarp();
+        }
+    }
+    // g = A^-1 h with the same factor (vb <- g)
+    tile::forward_again(s.vb, s.vw, f, nb, s);
+    tile::backward<false>(s.vw, s.vb, f, nb, s);
+    // g . x: 32 features a warp sum, the warps' sums in order
+    for (int i0 = 32 * warp; i0 < f; i0 += nt) {
+        float gx = i0 + lane < f ? s.vb[i0 + lane] * s.vx[i0 + lane] : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) gx += __shfl_xor_sync(0xffffffffu, gx, o);
+        if (lane == 0) red[i0 >> 5] = gx;
+    }
+    for (int i = tid; i < f; i += nt) gr[i] = s.vb[i];
+    const double sl = block_sum_d(loss, dsh);  // (its barrier also orders red)
+    if (tid == 0) {
+        float gx = 0.f;
+        for (int w = 0; 32 * w < f; ++w) gx += red[w];
+        a.loss_part[row] = sl;
+        a.dlam_part[row] = -(double)nu * (double)gx;
+    }
+}
+
+template <int P>
+cudaError_t launch_rows(const AdjArgs<float> &a, int64_t m, cudaStream_t st) {
+    const int nb = tile::nb_of(a.f);
+    const size_t smem = tile_smem<P>(a.f);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            adjoint_tile_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    adjoint_tile_kernel<P><<<(unsigned)m, tile::up32(tile::tiles_of(nb)), smem, st>>>(a, nb);
+    return cudaGetLastError();
+}
+
 // dL/dy_i, in fixed chunks: chunk c covers ratings [cbeg[c], cend[c]) of item citem[c]'s
 // training column (the CSC: users and ratings) and, for the item's first chunk, its held-out
 // ratings.  Warp w of the chunk's CTA takes entries w, w + ITEM_WARPS, ... in order; lane l
@@ -458,11 +574,26 @@ als_status adjoint_impl(als_handle *h, const als_coo_view *held, const T *d_Y, T
         a.flags = h->d_flags;
         a.f = f;
         a.lambda = lambda;
-        const size_t smem = smem_of<T>(FP);
-        if (smem > 48 * 1024)
-            step(cudaFuncSetAttribute(adjoint_row_kernel<T>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (e == cudaSuccess && m > 0) adjoint_row_kernel<T><<<(unsigned)m, nt_of(FP), smem, st>>>(a, FP);
+        bool tiles = false;
+        if constexpr (sizeof(T) == 4) {
+            tiles = tile::fits(f);
+            if (tiles && e == cudaSuccess && m > 0) {
+                switch (tile::pitch_of(f)) {
+                case 32: step(launch_rows<32>(a, m, st)); break;
+                case 64: step(launch_rows<64>(a, m, st)); break;
+                case 128: step(launch_rows<128>(a, m, st)); break;
+                default: step(launch_rows<192>(a, m, st)); break;
+                }
+            }
+        }
+        if (!tiles) {
+            const size_t smem = smem_of<T>(FP);
+            if (smem > 48 * 1024)
+                step(cudaFuncSetAttribute(adjoint_row_kernel<T>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (e == cudaSuccess && m > 0)
+                adjoint_row_kernel<T><<<(unsigned)m, nt_of(FP), smem, st>>>(a, FP);
+        }
         step(cudaGetLastError());
         const size_t ismem = sizeof(T) * ITEM_WARPS * (size_t)f;
         if (e == cudaSuccess && n > 0) {

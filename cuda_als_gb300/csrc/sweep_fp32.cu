@@ -11,23 +11,24 @@
 // The reference writes every f x f Gram to HBM (d_xtxs) and reads it back in the solver; here
 // the Gram lives in shared memory only.
 //
-// Layout.  The gathered panel Z (KC ratings x FP features, FP32) carries the rating itself as
-// feature f.  Each thread owns a 4 x 8 register tile of the lower block triangle of the Gram
-// (8 x 8 blocks, split in two), so the FMA work is the lower triangle only; each Gram entry is
-// one sequential FMA chain over the row's ratings, in rating order (the order of the reference's
+// Two layouts.  f <= 175: the matrix in registers, one 8 x 8 tile a thread (tilesolve.cuh), the
+// direct solvers in place there, CG on the Gram stored to shared memory.  Larger f (the "wide"
+// kernels; a tile a thread would take more than 512 threads of 128 registers): 4 x 8 register
+// tiles for the Gram, which is stored to shared memory (stride FP + 1, conflict-free column
+// walks) and solved there.  Both do the same arithmetic in the same order: each Gram entry is one
+// sequential FMA chain over the row's ratings, in rating order (the order of the reference's
 // calculate_vtvs, als_model.cu:137-155).  The right-hand side is summed apart, more accurately:
-// thread j sums r_k y_kj over each KC-rating chunk and adds the chunk sums with compensated
-// (Kahan) addition, so b_u carries about one rounding instead of the n_u of a sequential sum.
+// thread j sums r_k y_kj over each 32 ratings and adds those sums with compensated (Kahan)
+// addition, so b_u carries about one rounding instead of the n_u of a sequential sum.
 // (An FP32 sequential right-hand side costs ALS up to 4x in accuracy against FP64 after ten
-// iterations at f = 100-128: its error meets the Gram's condition number in every solve.)  After
-// the last chunk the tiles are stored to shared memory (stride FP+1, conflict-free column walks)
-// and the CTA solves in place.
+// iterations at f = 100-128: its error meets the Gram's condition number in every solve.)
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
 
 #include "internal.h"
 #include "solvers.cuh"
+#include "sweep_fp32_tile.cuh"
 
 namespace als {
 
@@ -36,13 +37,6 @@ namespace {
 constexpr int KC = 32;      // ratings gathered per chunk
 constexpr int MAX_FP = 232; // shared-memory bound of the Gram (FP x (FP+1) floats)
 
-__host__ __device__ inline int fp_of(int f) { return ((f + 1 + 7) / 8) * 8; }
-__host__ __device__ inline int nt_of(int fp) {
-    int nb = fp / 8;
-    int t = nb * (nb + 1);
-    t = (t + 31) / 32 * 32;
-    return t < 64 ? 64 : t;
-}
 __host__ __device__ inline size_t zsize_of(int fp) {
     size_t z = (size_t)KC * fp, g = (size_t)fp * (fp + 1);
     return z > g ? z : g;
@@ -121,12 +115,11 @@ __device__ void accumulate(const SweepArgs &a, int FP, int beg, int end, const T
     }
 }
 
-// From the finished Gram tiles and b: regularise, solve with the selected solver (CG warm-started
+// The wide kernels: from the finished Gram tiles and b: regularise, solve with the selected solver (CG warm-started
 // from the current x), write x (or x = 0 and a flag for a non-SPD / non-finite row).
 __device__ void solve_and_write(const SweepArgs &a, int FP, int row, int nu, const Tile &t,
                                 const float (&acc)[4][8], float b_tid, float *smem) {
-    const int f = a.f, GS = FP + 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int f = a.f, GS = FP + 1, tid = threadIdx.x;
     float *G = smem;  // the Gram of [Y | r] replaces the panel
     int32_t *scol = (int32_t *)(smem + zsize_of(FP));
     float *sval = (float *)(scol + KC);
@@ -147,39 +140,11 @@ __device__ void solve_and_write(const SweepArgs &a, int FP, int row, int nu, con
         vx[tid] = xo[tid];
     }
     __syncthreads();
-
-    bool ok = true;
-    const int nt = blockDim.x;
-    if (a.solve == ALS_SOLVE_CG_FP32 || a.solve == ALS_SOLVE_CG_FP16) {
-        if (a.solve == ALS_SOLVE_CG_FP16) {  // the Gram rounded to binary16 (cg.cu:236-430)
-            for (int i = warp; i < f; i += nwarps)
-                for (int j = lane; j <= i; j += 32)
-                    G[i * GS + j] = __half2float(__float2half_rn(G[i * GS + j]));
-            __syncthreads();
-        }
-        cg_solve<CtaSync>(G, GS, f, vb, vx, vr, vp, vap, red, a.cg_iters, a.cg_tol, tid, nt);
-    } else if (a.solve == ALS_SOLVE_LU) {
-        ok = lu_nopivot_solve<CtaSync>(G, GS, f, vb, tid, nt);
-        for (int i = tid; i < f; i += blockDim.x) vx[i] = vb[i];
-    } else {
-        ok = ldlt_factor<CtaSync>(G, GS, f, tid, nt);
-        if (ok) ldlt_solve<CtaSync>(G, GS, f, vb, tid);
-        for (int i = tid; i < f; i += blockDim.x) vx[i] = vb[i];
-    }
-    __syncthreads();
-    float bad = 0.f;
-    for (int i = tid; i < f; i += blockDim.x) bad += isfinite(vx[i]) ? 0.f : 1.f;
-    bad = group_sum<CtaSync>(bad, red, tid, nt);
-    if (!ok || bad > 0.f) {
-        for (int i = tid; i < f; i += blockDim.x) xo[i] = 0.f;
-        if (tid == 0 && a.flags) atomicAdd(&a.flags[0], 1);
-        return;
-    }
-    for (int i = tid; i < f; i += blockDim.x) xo[i] = vx[i];
+    solve_shared(a, G, GS, vb, vx, vr, vp, vap, red, xo);
 }
 
 // Rows of the order slice [row_begin, row_end), one CTA each: Gram, right-hand side, solve.
-__global__ void __launch_bounds__(1024) sweep_fp32_kernel(const SweepArgs a, const int FP) {
+__global__ void __launch_bounds__(1024) sweep_wide_kernel(const SweepArgs a, const int FP) {
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x;
     const int slot = a.row_begin + blockIdx.x;
@@ -205,7 +170,7 @@ __global__ void __launch_bounds__(1024) sweep_fp32_kernel(const SweepArgs a, con
 // Heavy rows: part p accumulates ratings [beg[p], end[p]) of its row and stores its tiles (FP x GS
 // floats, the lower block triangle) and its compensated right-hand side (sum, compensation).
 __global__ void __launch_bounds__(1024)
-    gram_part_kernel(const SweepArgs a, const int FP, const int32_t *__restrict__ part_beg,
+    gram_part_wide_kernel(const SweepArgs a, const int FP, const int32_t *__restrict__ part_beg,
                      const int32_t *__restrict__ part_end, float *__restrict__ part) {
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, GS = FP + 1;
@@ -236,7 +201,7 @@ __global__ void __launch_bounds__(1024)
 // Heavy row at order position h: its parts first[h]..first[h+1] added in order (the tiles
 // plainly, the right-hand sides with compensation), then the common regularise / solve / write.
 __global__ void __launch_bounds__(1024)
-    combine_solve_kernel(const SweepArgs a, const int FP, const int32_t *__restrict__ first,
+    combine_solve_wide_kernel(const SweepArgs a, const int FP, const int32_t *__restrict__ first,
                          const float *__restrict__ part) {
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, GS = FP + 1;
@@ -276,18 +241,26 @@ bool fp32_supported(int f) { return f >= 1 && fp_of(f) <= MAX_FP; }
 
 cudaError_t launch_sweep_fp32(const SweepArgs &a, const Fp32Split *sp, cudaStream_t st,
                               int *launches) {
+    if (tile::fits(a.f)) {
+        switch (tile::pitch_of(a.f)) {
+        case 32: return launch_tiles_32(a, sp, st, launches);
+        case 64: return launch_tiles_64(a, sp, st, launches);
+        case 128: return launch_tiles_128(a, sp, st, launches);
+        default: return launch_tiles_192(a, sp, st, launches);
+        }
+    }
     const int FP = fp_of(a.f);
     if (nt_of(FP) < a.f) return cudaErrorInvalidConfiguration;  // thread j owns b_j
     const size_t smem = smem_of(FP);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(sweep_fp32_kernel,
+        cudaError_t e = cudaFuncSetAttribute(sweep_wide_kernel,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gram_part_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(gram_part_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(combine_solve_kernel,
+            e = cudaFuncSetAttribute(combine_solve_wide_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
@@ -295,21 +268,22 @@ cudaError_t launch_sweep_fp32(const SweepArgs &a, const Fp32Split *sp, cudaStrea
     SweepArgs b = a;
     if (sp && sp->nheavy > 0 && a.row_begin == 0 && a.order) {
         const int32_t nh = sp->nheavy < a.row_end ? sp->nheavy : a.row_end;
-        gram_part_kernel<<<(unsigned)sp->first_host[nh], nt_of(FP), smem, st>>>(
+        gram_part_wide_kernel<<<(unsigned)sp->first_host[nh], nt_of(FP), smem, st>>>(
             a, FP, sp->part_beg, sp->part_end, sp->part);
-        combine_solve_kernel<<<(unsigned)nh, nt_of(FP), smem, st>>>(a, FP, sp->first, sp->part);
+        combine_solve_wide_kernel<<<(unsigned)nh, nt_of(FP), smem, st>>>(a, FP, sp->first, sp->part);
         if (launches) *launches += 2;
         b.row_begin = nh;
     }
     const int n = b.row_end - b.row_begin;
     if (n > 0) {
-        sweep_fp32_kernel<<<(unsigned)n, nt_of(FP), smem, st>>>(b, FP);
+        sweep_wide_kernel<<<(unsigned)n, nt_of(FP), smem, st>>>(b, FP);
         if (launches) ++*launches;
     }
     return cudaGetLastError();
 }
 
 size_t fp32_part_floats(int f) {
+    if (tile::fits(f)) return tile_part_floats(f);
     const int FP = fp_of(f);
     return (size_t)FP * (FP + 1) + 2 * (size_t)FP;
 }
