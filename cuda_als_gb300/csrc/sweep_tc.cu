@@ -3,7 +3,7 @@
 //
 // Reference path replaced (per half-sweep, als_model.cu:1797-2029 / :2030-2267):
 //   float2half_array (als_model.cu:54-60)            -> quantise_bf16 below (padded BF16 table)
-//   csrmm2 + geam RHS (als_model.cu:1816-1852)      -> second MMA against the rating tile
+//   csrmm2 + geam RHS (als_model.cu:1816-1852)      -> the ratings as a feature column
 //   calculate_vtvs_smem_row_major_tensor* (:428-1490, wmma 16x16x16, f <= 112 only)
 //                                                    -> tcgen05.mma M=128, N=roundup(f,16)
 //   LU_solve / updateXWithCGHost (:1570-1720, cg.cu) -> register solvers (regsolve.cuh) or the
@@ -16,15 +16,22 @@
 //            selected solver (registers / shared memory, or the tensor core for the FP16-Gram CG);
 //            Cholesky refinement re-reads A from TMEM for the residual b - A x (in FP64 for rows
 //            whose Cholesky diagonal ratio exceeds cond_threshold).
-//   producer: walks the rows' stages (KC = 64 ratings each) and copies each stage's column ids
-//            and ratings into a metadata ring MD stages ahead with cp.async, then publishes it.
-//   MMA issuer: per 16 ratings one M=128 x N=Ng x K=16 MMA (Gram: A = B = the gathered panel,
-//            both MN-major) and one M=128 x N=16 MMA (RHS: B = the rating tile), into one of
-//            NBUF TMEM accumulators; tcgen05.commit frees the stage / publishes the row.  (The
-//            tensor-core CG at f <= 112 fuses the two: one N=Ng+16 MMA, the ratings written into
-//            feature column Ng of the panel by the gather warp once its rows have landed.)
-//   NGATHER gather warps: take the published stages round-robin, write the rating tile (row 0 of
-//            a K-major tile), arm the stage's barrier and issue one tile::gather4 per lane.
+//   producer: cuts rows into stages (KC = 64 ratings each) and publishes their descriptors, up
+//            to 32 at once.
+//   NGATHER gather warps: take the stages round-robin; each loads its stage's column ids and
+//            ratings a turn ahead, copies the factor rows by 16-byte cp.async to their swizzled
+//            places, writes the ratings (into feature column Ng of the panel, at f > 112 into row
+//            0 of a K-major tile) and marks the stage full.
+//   MMA issuer: per 16 ratings one M=128 x N=Ng+16 x K=16 MMA (A = B = the gathered panel, both
+//            MN-major: Gram and right-hand side together; at f > 112 a Gram MMA and an N = 16
+//            MMA against the rating tile), into one of NBUF TMEM accumulators; tcgen05.commit
+//            frees the stage / publishes the row.
+// What bounds it, measured on one GB300 (98.6M ratings, f = 100, cycles a 64-rating stage an SM):
+// V half, FP16-Gram CG 680: the issuer's MMAs 300 (76 each, 64 at the tensor core's rate) and,
+// one after another, its wait, the stage's descriptor and the commits; 1,000 while one warp
+// published stage by stage and the rows came by TMA tile::gather4 (7 cycles a 128-byte row box, a
+// second limit at 900-1,000 cycles; cp.async takes 320).  U half, FP32 CG: the solves (an
+// accumulator is awaited for 780 of 1,770 cycles).
 // Operand layout (one stage): 2 atoms of 64 features x KC ratings; atom a, rating k, feature chunk
 // c (8 features, 16 B) sits at a*8192 + (k/8)*1024 + (k%8)*128 + ((c%8) ^ (k%8))*16, i.e. the
 // canonical SWIZZLE_128B MN-major layout with LBO = 8192 (between 64-feature atoms) and
@@ -134,7 +141,6 @@ static int tcg_solver(int solve_type) {
     }
 }
 struct TcState {
-    CUtensorMap tmap[2];   // [side]: TMA map of the side's 16- or 8-bit table (64-byte aligned)
     tcg::Geometry geo[tcg::NSOLVER];  // per solver (CG, Cholesky, LU, tensor-core CG)
     bool f8 = false;                   // FP8 (e4m3) operands instead of BF16
     __nv_bfloat16 *d_bf[2] = {nullptr, nullptr};  // [side]: table gathered by that side
@@ -147,52 +153,6 @@ struct TcState {
 };
 
 bool tc_path_supported(int f) { return f >= 1 && f <= tcg::MAXF; }
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-    static const EncodeTiledFn fn = []() -> EncodeTiledFn {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                             &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
-// The gather map of a BF16 table of `rows` x fst: box = 64 features (128 bytes, the swizzle
-// span) x 1 row, as tile::gather4 requires; features past fst read as zero.
-static bool encode_table_map(CUtensorMap *map, void *table, int64_t rows, int fst) {
-    EncodeTiledFn fn = encode_tiled();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)fst, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)fst * sizeof(__nv_bfloat16)};
-    const cuuint32_t box[2] = {64, 1};
-    const cuuint32_t estride[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, table, dims, strides, box, estride,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// The gather map of an FP8 table of `rows` x 128 bytes: box = 128 features (one 128-byte line,
-// the swizzle span) x 1 row.
-static bool encode_table_map_f8(CUtensorMap *map, void *table, int64_t rows) {
-    EncodeTiledFn fn = encode_tiled();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)tcg::F8_ROW_BYTES, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)tcg::F8_ROW_BYTES};
-    const cuuint32_t box[2] = {(cuuint32_t)tcg::F8_ROW_BYTES, 1};
-    const cuuint32_t estride[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, table, dims, strides, box, estride,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 
 als_status tc_prepare(als_handle *h, std::string *why) {
     if (!tc_path_supported(h->f)) {
@@ -227,10 +187,6 @@ als_status tc_prepare(als_handle *h, std::string *why) {
             *why = "out of memory for the FP8 factor tables";
             return ALS_ERR_OUT_OF_MEMORY;
         }
-        if (!encode_table_map_f8(&t->tmap[s], t->d_f8[s], opp[s] + 1)) {
-            *why = "cuTensorMapEncodeTiled failed for the FP8 table";
-            return ALS_ERR_CUDA;
-        }
     }
     if (t->f8 && cudaMalloc(&t->d_cmax, sizeof(unsigned int) * tcg::MAXF) != cudaSuccess) {
         *why = "out of memory";
@@ -242,10 +198,6 @@ als_status tc_prepare(als_handle *h, std::string *why) {
             cudaMemset(t->d_bf[s], 0, bytes) != cudaSuccess) {
             *why = "out of memory for the BF16 factor tables";
             return ALS_ERR_OUT_OF_MEMORY;
-        }
-        if (!encode_table_map(&t->tmap[s], t->d_bf[s], opp[s] + 1, t->geo[0].fst)) {
-            *why = "cuTensorMapEncodeTiled failed for the BF16 table";
-            return ALS_ERR_CUDA;
         }
     }
     if (cudaMalloc(&t->d_work, sizeof(int32_t) * 8) != cudaSuccess) {
@@ -345,12 +297,12 @@ cudaError_t tc_launch_bucket(const als_handle *h, int side, int32_t lo, int32_t 
     cudaError_t e = cudaMemsetAsync(t->d_work + slot, 0, sizeof(int32_t), st);
     if (e != cudaSuccess) return e;
     tcg::Params p{};
-    p.tmap = t->tmap[side];
     p.ptr = side == 0 ? h->d_csr_ptr : h->d_csc_ptr;
     p.idx = side == 0 ? h->d_csr_idx : h->d_csc_idx;
     p.val = side == 0 ? h->d_csr_val : h->d_csc_val;
     p.order = h->d_order[side] + lo;
-    p.Ybf = t->d_bf[side];
+    p.table = t->f8 ? t->d_f8[side] : reinterpret_cast<const uint8_t *>(t->d_bf[side]);
+    p.row_bytes = t->f8 ? tcg::F8_ROW_BYTES : 2 * g.fst;
     p.dscale = t->d_scale[side];
     p.X = side == 0 ? h->d_U : h->d_V;
     p.work = t->d_work + slot;

@@ -2,7 +2,6 @@
 // design); instantiated per padded size by sweep_tc_fp*.cu.
 #pragma once
 
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -29,24 +28,25 @@ constexpr int ATOM_BYTES = 1024;             // 8 ratings x 128 B
 constexpr int ATOM_STRIDE = (KC / 8) * ATOM_BYTES;  // 8192: LBO between 64-feature atoms
 constexpr int TILE_BYTES = 2 * ATOM_STRIDE;  // 128 features
 constexpr int R_BYTES = 2 * ATOM_BYTES;      // K-major rating tile, N = 16 rows x 64 ratings
-constexpr int STAGE_BYTES = TILE_BYTES + R_BYTES;
-// FP8 stages: one 128-feature atom of KC ratings (8 KB) and the rating tile
+// FP8 stages: one 128-feature atom of KC ratings (8 KB)
 constexpr int TILE_BYTES_F8 = ATOM_STRIDE;
-constexpr int STAGE_BYTES_F8 = TILE_BYTES_F8 + R_BYTES;
-__host__ __device__ constexpr int stage_bytes(bool f8) { return f8 ? STAGE_BYTES_F8 : STAGE_BYTES; }
 __host__ __device__ constexpr int tile_bytes(bool f8) { return f8 ? TILE_BYTES_F8 : TILE_BYTES; }
+// The ratings ride in the panel's feature column ng (sweep_tc_kernel, FUSED) where there is one.
+__host__ __device__ constexpr bool fused_of(int fp) { return fp <= 112; }
+__host__ __device__ constexpr int stage_bytes(int fp, bool f8) {
+    return tile_bytes(f8) + (fused_of(fp) ? 0 : R_BYTES);
+}
 constexpr int MAXF = 128;
 constexpr int MAX_NBUF = 4;
-// Producer metadata ring: each stage's column ids and ratings are copied into shared memory MD
-// stages ahead of its gathers (MR slots, MR > MD), so their HBM latency never stalls the gathers.
-constexpr int MD = 12;
-constexpr int MR = 16;
+// Ring of stage descriptors (row, first rating, ratings of the row, count and flags) from the
+// producer to the gather warps.
+constexpr int MR = 32;
 // Warp roles: the solver warpgroups come first (group g = warps 4g..4g+3, so warp w reads TMEM
-// lanes 32 (w % 4) ..), then the producer (metadata look-ahead), the MMA issuer and the gather
-// warps.  One warp issues a tile::gather4 only every ~90 cycles, so the stages go round-robin to
-// several gather warps, which also write each stage's rating tile and arm its barrier.
+// lanes 32 (w % 4) ..), then the producer (which cuts the rows into stages), the MMA issuer and
+// the gather warps, which take the stages round-robin: a gather warp loads its stage's column ids
+// and ratings one stage ahead, copies the factor rows and marks the stage full.
 constexpr int MAX_NGATHER = 6;
-constexpr int MRING_BYTES = MR * KC * 8 + MR * 16;   // column ids, ratings, Meta per slot
+constexpr int MRING_BYTES = MR * 16 + MAX_NGATHER * KC * 4;  // descriptors, a gather warp's ids
 // SOLVER_CGTC: CG on the Gram rounded to binary16's significand (the reference's FP16-Gram CG),
 // its products A p run on the tensor core from the accumulator left in TMEM.
 enum { SOLVER_CG = 0, SOLVER_CHOL = 1, SOLVER_LU = 2, SOLVER_CGTC = 3 };
@@ -74,19 +74,16 @@ __host__ __device__ constexpr int nepi_of(int solver, int fp) {
     return solver == 1 || solver == 3 || cg_quad_rows(solver, fp) ? nbuf_of(solver, fp)
                                                                    : nbuf_of(solver, fp) / 2;
 }
-// Gather warps: one warp issues a tile::gather4 only every ~90 cycles, so the gathers want several
-// warps, up to about six (ten made the tensor-core CG slower: the SM's gathers are then saturated
-// and the extra warps only add hand-offs).  A launch's registers are shared out per four warps, so
-// above 640 threads a thread keeps 80 and at 640 it keeps 96.  The tensor-core CG (about 60 a
-// thread) takes six gather warps; the Cholesky factor, LU and the four-group quad-blocked CG (84
-// to 96 a thread) two.  The three-group quad-blocked CG at FP = 128 splits the registers
-// (setmaxnreg): launched with six gather warps at 96 a thread, its solver warpgroups take 128 and
-// the two service warpgroups (producer, MMA issuer, gather warps) give theirs back down to
-// SERVICE_REGS, the sum being exactly what the launch holds (launch_regs_of x threads).  (The same
-// split for the four groups at FP = 64 and 112, 80 a thread at launch, made their light rows,
-// bound by the solves, 1-8% slower.)
+// Gather warps: six take a stage in the time of its MMAs (two: V half of 98.6M ratings at f = 100
+// with the FP32 CG 5.69 ms, six 3.57).  A launch's registers are shared out per four warps, so
+// above 640 threads a thread keeps 80 and at 640 it keeps 96.  The tensor-core CG (about 70 a
+// thread) takes six as it is; the Cholesky factor and LU (96 and more) two.  The quad-blocked CG
+// splits its registers (setmaxnreg): launched with six gather warps at 80 a thread (FP = 128, three
+// groups: 96), its solver warpgroups take 96 (128) and the two service warpgroups (producer, MMA
+// issuer, gather warps) give theirs back down to SERVICE_REGS, the sum being exactly what the
+// launch holds (launch_regs_of x threads).
 __host__ __device__ constexpr bool regsplit_of(int solver, int fp) {
-    return cg_quad_rows(solver, fp) && fp == 128;
+    return cg_quad_rows(solver, fp);
 }
 __host__ __device__ constexpr int ngather_of(int solver, int fp) {
     return solver == 3 || regsplit_of(solver, fp) ? 6 : 2;
@@ -107,20 +104,16 @@ __host__ __device__ constexpr int launch_regs_of(int solver, int fp) {
 // WAIT_NS, so that a CTA that gave up still lets every copy it issued land before it exits.
 constexpr unsigned long long WAIT_NS = 10ull * 1000 * 1000 * 1000;  // 10 s
 
-struct Meta {  // per stage / per accumulator
-    int32_t row;    // -1 = end of work
-    int32_t cnt;    // ratings in this stage
-    int32_t flags;  // 1 = first stage of the row, 2 = last stage of the row
-    int32_t nu;     // ratings of the row
+struct Meta {  // per accumulator
+    int32_t row;  // -1 = end of work
+    int32_t nu;   // ratings of the row
 };
 
 struct Params {
-    // 2-D map of the BF16 table (fst features x n_opp + 1 rows), box 64 features x 1 row,
-    // 128-byte swizzle: the producer's tile::gather4 loads read 4 rows of it per instruction
-    CUtensorMap tmap;
     const int32_t *ptr, *idx, *order;
     const float *val;
-    const __nv_bfloat16 *Ybf;  // (n_opp + 1) x fst, row n_opp all zero
+    const uint8_t *table;      // the gathered table, n_opp + 1 rows (row n_opp all zero) of
+    int32_t row_bytes;         // row_bytes: BF16 2 fst, FP8 128
     const float *dscale;       // FP8 operands: the table's per-feature scales (powers of two)
     float *X;                  // this side's FP32 factors (in: CG warm start, out: solution)
     int32_t *work;             // atomic row counter (zeroed before the launch)
@@ -183,15 +176,15 @@ __host__ __device__ constexpr size_t group_floats(int fp, int solver) {
                          : (size_t)fp * (fp + 4) + 8 * (size_t)fp + 2 * (size_t)fp + 16 + 5 * 128 + 64;
 }
 // Stage-ring depth: as many stages as the shared memory left beside the solver groups' scratch,
-// the metadata ring and the barriers holds (at most MAX_NSTAGE).  On Gram-bound rows a stage's
-// life (gather issue, the rows' L2 round trip, the MMAs, the commit that frees the slot) is
-// long against its MMA time, so the stages in flight set the rate; on solve-bound rows more
-// stages cost nothing (one CTA per SM).  FP8 stages are 10 KB instead of 18 KB.
+// the descriptor ring and the barriers holds (at most MAX_NSTAGE).  On Gram-bound rows a stage's
+// life (the copies' issue, their L2 round trip, the MMAs, the commit that frees the slot) is
+// long against its MMA time; on solve-bound rows more stages cost nothing (one CTA per SM).  FP8
+// stages are half as large.
 constexpr size_t SMEM_BUDGET = 232448 - 2048;  // the opt-in limit per CTA, less alignment slack
 __host__ __device__ constexpr int nstage_fit(int solver, int fp, bool f8) {
     return (int)((SMEM_BUDGET - sizeof(float) * group_floats(fp, solver) * nepi_of(solver, fp) -
                   (size_t)MRING_BYTES - 1024 - (f8 ? sizeof(float) * MAXF : 0)) /
-                 (size_t)stage_bytes(f8));
+                 (size_t)stage_bytes(fp, f8));
 }
 __host__ __device__ constexpr int nstage_of(int solver, int fp, bool f8) {
     return nstage_fit(solver, fp, f8) > MAX_NSTAGE ? MAX_NSTAGE : nstage_fit(solver, fp, f8);
@@ -213,7 +206,7 @@ inline Geometry geometry(int f, int solver, bool f8 = false) {
     g.tmem_cols = cols;
     g.nthreads = nthreads_of(solver, g.fp);
     const int ns = nstage_of(solver, g.fp, f8);
-    size_t bytes = (size_t)ns * stage_bytes(f8);                     // operand ring
+    size_t bytes = (size_t)ns * stage_bytes(g.fp, f8);                     // operand ring
     bytes += sizeof(float) * group_floats(g.fp, solver) * g.nepi;    // per-group scratch
     if (f8) bytes += sizeof(float) * MAXF;                            // per-feature scales
     bytes += MRING_BYTES;                                            // metadata ring
@@ -276,40 +269,55 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
     __syncwarp();
     return ok != 0;
 }
+// The same by votes, every lane trying (and acquiring) itself: no broadcast on the path of a
+// phase already complete.
+__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile int *abort,
+                                              unsigned long long limit) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+    const unsigned long long t0 = now_ns();
+    for (uint32_t i = 0;; ++i) {
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+        if ((i & 15) == 15) {
+            const int stop = (threadIdx.x & 31) == 0 && (*abort || now_ns() - t0 > limit);
+            if (__any_sync(0xffffffffu, stop)) return false;
+        }
+    }
+}
+// A shared-memory word written after what it announces (__threadfence_block before the store).
+__device__ __forceinline__ uint32_t ld_acquire(const volatile int *word) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];"
+                 : "=r"(v)
+                 : "r"(smem_u32(const_cast<const int *>(word)))
+                 : "memory");
+    return v;
+}
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-// 4-byte asynchronous global -> shared copy (the ratings of a stage have no alignment), with an
-// L2 cache policy: the column ids and ratings stream through once per half-sweep (evict first),
-// so they do not push the gathered factor table (evict last) out of L2.
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, uint64_t policy) {
-    asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 4, %2;" ::"r"(dst),
-                 "l"(src), "l"(policy)
-                 : "memory");
+// Load with an L2 cache policy: the column ids and ratings stream through once per half-sweep
+// (evict first), so they do not push the gathered factor table (evict last) out of L2.
+__device__ __forceinline__ int32_t ld_stream(const int32_t *src, uint64_t policy) {
+    int32_t v;
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(src), "l"(policy));
+    return v;
+}
+__device__ __forceinline__ float ld_stream(const float *src, uint64_t policy) {
+    float v;
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;" : "=f"(v) : "l"(src), "l"(policy));
+    return v;
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-// Arrive on `bar` and add `bytes` to the transaction count its current phase waits for.
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+// 16-byte copy of a factor row's chunk, L2 to shared memory; `policy`: the gathered table is re-read
+// by every SM for the whole half-sweep.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint64_t policy) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
+                 "l"(policy)
                  : "memory");
-}
-// TMA gather: rows r0..r3 of the 2-D tensor map, features x .. x+63 (x * 2 bytes a multiple of
-// 16), land as four consecutive 128-byte rows at dst (128-byte swizzle by address); the bytes
-// count against `bar`'s transaction count.  `policy` is an L2 cache policy: the gathered table is
-// re-read by every SM for the whole half-sweep.
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap *tmap, int x, int r0,
-                                            int r1, int r2, int r3, uint32_t bar,
-                                            uint64_t policy) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes"
-        ".L2::cache_hint [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar),
-        "l"(policy)
-        : "memory");
 }
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t pol;
@@ -345,12 +353,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool a_mn, bool 
            ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// (`lead`: nonzero in the one lane that issues)
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
+                                         uint32_t idesc, uint32_t accumulate, uint32_t lead) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 // Instruction descriptor of tcgen05.mma kind::f8f6f4: D F32, A/B E4M3 (format 0), majors, N, M.
@@ -359,16 +368,18 @@ __host__ __device__ constexpr uint32_t idesc_e4m3(int M, int N, bool a_mn, bool 
            ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 __device__ __forceinline__ void mma_e4m3(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
+                                         uint32_t idesc, uint32_t accumulate, uint32_t lead) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
+__device__ __forceinline__ void mma_commit(uint32_t bar, uint32_t lead = 1u) {
     asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(lead)
         : "memory");
 }
 // Shared-memory descriptor without swizzle (canonical layout of 8-row x 16-byte core matrices):
@@ -569,9 +580,12 @@ __device__ float cg_tc(const Params &p, uint32_t tcol, uint32_t trow, float bi, 
         gs.sync();
         if (et == lead && !*abort) {
             tc_fence_after();
-            for (int kk = 0; kk < ng / 16; ++kk)
-                mma_f16_tmem_a(tcol + (uint32_t)ng, tcol + 8u * kk,
-                               sdesc_plain(bt + 512u * kk, 256, 128), idesc, kk > 0 ? 1u : 0u);
+            const uint64_t bd = sdesc_plain(bt, 256, 128);
+#pragma unroll
+            for (int kk = 0; kk < FP / 16; ++kk)
+                if (16 * kk < ng)
+                    mma_f16_tmem_a(tcol + (uint32_t)ng, tcol + 8u * kk, bd + (uint64_t)(32 * kk),
+                                   idesc, kk > 0 ? 1u : 0u);
             mma_commit(bar);
             st.unconfirmed = true;
             st.committed = st.phase;
@@ -900,23 +914,21 @@ template <int FP, int SOLVER, bool F8>
 __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
     sweep_tc_kernel(const __grid_constant__ Params p) {
     constexpr int NSTAGE = nstage_of(SOLVER, FP, F8);
-    constexpr int SBYTES = stage_bytes(F8), TBYTES = tile_bytes(F8);
+    constexpr int SBYTES = stage_bytes(FP, F8), TBYTES = tile_bytes(F8);
     static_assert(NSTAGE >= 2 && NSTAGE <= MAX_NSTAGE, "stage ring");
     constexpr int NEPI = nepi_of(SOLVER, FP);
     constexpr int WP = 4 * NEPI;  // producer warp; then the MMA issuer and the gather warps
     constexpr int WM = WP + 1;
     constexpr int WG = WP + 2;
     constexpr int NGATHER = ngather_of(SOLVER, FP);
-    // One MMA per 16 ratings for the Gram and the right-hand side together: the gather warp of a
-    // stage waits for its bytes, writes the stage's ratings into feature column ng of the panel
-    // (the gather left it zero: ng >= fst) and marks the stage ready; the MMA issuer waits for
-    // ready and issues M=128 x N=ng+16 (Gram in columns [0, ng), b in column ng; row ng of the
-    // accumulator then holds b^T, a padded row the solvers ignore).  Where the gather warps have
-    // the time: the tensor-core CG's six; FP = 128 (ng = 128) has no free column.  FP8 stages
-    // take the e4m3 rating into byte ng of each 128-byte row: one MMA per 32 ratings instead of
-    // a Gram MMA and an N = 16 right-hand-side MMA (the same e4m3 products, summed in one pass).
-    constexpr bool FUSED = SOLVER == SOLVER_CGTC && FP <= 112;
-    static_assert(NGATHER <= MAX_NGATHER, "");
+    // One MMA per 16 ratings for the Gram and the right-hand side together: the gather warp
+    // writes the stage's ratings into feature column ng of the panel, which no copied chunk
+    // covers (ng >= fst), and the MMA is M=128 x N=ng+16 (Gram in columns [0, ng), b in column
+    // ng; row ng of the accumulator then holds b^T, a padded row the solvers ignore).  FP = 128
+    // (ng = 128) has no free column: a second, N = 16 MMA against the rating tile.  FP8 stages
+    // take the e4m3 rating into byte ng of each 128-byte row: one MMA per 32 ratings.
+    constexpr bool FUSED = fused_of(FP);
+    static_assert(NGATHER <= MAX_NGATHER && NGATHER <= NSTAGE, "");
     // Register split: setmaxnreg acts per warpgroup, so the solver warps and the service warps
     // each form whole warpgroups, and the registers the solvers take are exactly those the
     // service warps give back out of the launch's own (a larger .inc would wait forever; the host
@@ -935,26 +947,22 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
     uint8_t *ring = smem;
     float *gscratch = (float *)(ring + NSTAGE * SBYTES);
     float *dsc = gscratch + GroupLayout<FP, SOLVER>::floats * NEPI;  // [MAXF] FP8 scales
-    int32_t *mcol = (int32_t *)(dsc + (F8 ? MAXF : 0));                             // [MR][KC]
-    float *mval = reinterpret_cast<float *>(mcol + MR * KC);                            // [MR][KC]
-    Meta *mmeta = reinterpret_cast<Meta *>(mval + MR * KC);                             // [MR]
-    Meta *smeta = reinterpret_cast<Meta *>(mmeta + MR);                                 // [NSTAGE]
-    Meta *ameta = smeta + NSTAGE;
-    uint64_t *bars = (uint64_t *)(ameta + MAX_NBUF);  // 16-byte aligned: Meta is 16 bytes
+    int4 *desc = reinterpret_cast<int4 *>(dsc + (F8 ? MAXF : 0));           // [MR]
+    int32_t *wids = reinterpret_cast<int32_t *>(desc + MR);                 // [MAX_NGATHER][KC]
+    int4 *sdes = reinterpret_cast<int4 *>(wids + MAX_NGATHER * KC);         // [NSTAGE]
+    Meta *ameta = reinterpret_cast<Meta *>(sdes + NSTAGE);                  // [MAX_NBUF]
+    uint64_t *bars = (uint64_t *)(ameta + MAX_NBUF);
     uint64_t *full = bars, *empty = bars + NSTAGE;
     uint64_t *acc_full = bars + 2 * NSTAGE;
     uint64_t *acc_empty = acc_full + MAX_NBUF, *acc_meta = acc_empty + MAX_NBUF;
     uint64_t *drain = acc_meta + MAX_NBUF;
     uint64_t *mvbar = drain + 1;  // [MAX_NBUF]: the tensor-core CG's product barrier per group
-    uint64_t *ready = mvbar + MAX_NBUF;  // [MAX_NSTAGE]: stage's ratings in the panel (FUSED)
-    uint32_t *tmem_slot = (uint32_t *)(ready + MAX_NSTAGE);
+    uint32_t *tmem_slot = (uint32_t *)(mvbar + MAX_NBUF);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
     volatile int *grp_ok = abort + 1;  // per-group broadcast of the leader's wait outcome
-    volatile int *pub = grp_ok + MAX_NBUF;  // stages whose metadata has landed (producer)
+    volatile int *pub = grp_ok + MAX_NBUF;  // stages described (producer)
     volatile int *fin = pub + 1;            // the producer has published its last stage
-    volatile int *done = fin + 1;               // [NGATHER]: stages gather warp h has taken its
-                                                // metadata from (slot t % MR free again)
-    volatile int *armed = done + MAX_NGATHER;   // [NSTAGE]: the last stage armed in each slot
+    volatile int *done = fin + 1;  // [NGATHER]: the next stage gather warp h reads
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nbuf = p.nbuf;
@@ -971,12 +979,10 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
     }
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
-            // the gathering warp's arrive.expect_tx; the TMA bytes complete the phase
             mbar_init(smem_u32(&full[s]), 1);
             mbar_init(smem_u32(&empty[s]), 1);
-            armed[s] = -1;
         }
-        for (int h = 0; h < NGATHER; ++h) done[h] = 0;
+        for (int h = 0; h < NGATHER; ++h) done[h] = h;
         for (int b = 0; b < MAX_NBUF; ++b) {
             mbar_init(smem_u32(&acc_full[b]), 1);
             mbar_init(smem_u32(&acc_empty[b]), 1);
@@ -984,7 +990,6 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
             mbar_init(smem_u32(&mvbar[b]), 1);
         }
         mbar_init(smem_u32(drain), 1);
-        for (int u = 0; u < MAX_NSTAGE; ++u) mbar_init(smem_u32(&ready[u]), 1);
         *abort = 0;
         *pub = 0;
         *fin = 0;
@@ -1003,6 +1008,10 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // a bounded wait by a whole warp, on warp-uniform outcomes
+    auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool {
+        return mbar_wait_all(bar, parity, abort, p.wait_ns);
+    };
     // (the solver warpgroups first: each role's register budget covers the code it runs)
     if (warp < WP) {
         if constexpr (REGSPLIT)
@@ -1065,11 +1074,10 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
             asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SERVICE_REGS) : "memory");
         if (warp == WP) {
             // ------------------------------------------------------------------ producer
-            // Two cursors walk the same sequence of stages (KC ratings of one row each).  The
-            // look-ahead cursor issues a stage's column ids and ratings as 4-byte cp.async into the
-            // metadata ring MD stages ahead, with its Meta; the publishing cursor waits for that
-            // cp.async group and publishes the stage to the gather warps, which do the rest.  Rows
-            // come in chunks from the atomic counter (one at a time among the first `head` slots, the
+            // Cuts rows into stages of KC ratings and publishes their descriptors, up to 32 of a
+            // row at once (one stage at a time, its ids and ratings copied here too, this warp
+            // took ~1,000 cycles a stage and set the pace of every Gram-bound launch).  Rows come
+            // in chunks from the atomic counter (one at a time among the first `head` slots, the
             // heaviest rows, then CH at a time), pipelined two chunks ahead so the dependent
             // order[] -> ptr[] loads have landed when a chunk starts.
             constexpr int CH = 8;
@@ -1098,107 +1106,62 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                 n1beg = lane < n1cnt ? p.ptr[n1row] : 0;
                 n1end = lane < n1cnt ? p.ptr[n1row + 1] : 0;
             }
-            const uint64_t stream_pol = l2_evict_first_policy();  // column ids and ratings: once
-            int aj = 0;                                          // look-ahead cursor: row of chunk
-            int abase = __shfl_sync(0xffffffffu, cbeg, 0);       // and first rating of its stage
-            uint32_t gen = 0;                                    // stages issued by the look-ahead
-            // the metadata slot of stage g is free once the gather warp of stage g - MR has taken the
-            // column ids, ratings and Meta out of it (bounded wait; false on timeout or abort)
-            auto slot_free = [&](uint32_t g) -> bool {
-                if (g < (uint32_t)MR) return true;
-                const uint32_t old = g - MR;
-                int r = 1;
-                if (lane == 0) {
-                    const volatile int *d = done + old % NGATHER;
-                    const unsigned long long t0 = now_ns();
-                    for (uint32_t k = 0;; ++k) {
-                        if ((uint32_t)*d > old) break;
-                        if ((k & 255) == 255 && (*abort || now_ns() - t0 > p.wait_ns)) {
-                            r = 0;
-                            break;
-                        }
-                    }
-                    __threadfence_block();
-                }
-                return __shfl_sync(0xffffffffu, r, 0) != 0;
-            };
-            // issue the metadata of stage `gen`: 1 issued, 0 no rows left, -1 its slot never freed
-            auto generate = [&]() -> int {
-                while (aj >= ccnt) {
-                    if (ccnt <= 0) return 0;
-                    ccnt = n1cnt; crow = n1row; cbeg = n1beg; cend = n1end;
-                    n1cnt = n2cnt; n1row = n2row;
-                    n1beg = lane < n1cnt ? p.ptr[n1row] : 0;     // n2's row ids landed a chunk ago
-                    n1end = lane < n1cnt ? p.ptr[n1row + 1] : 0;
-                    int cb;
-                    grab(cb, n2cnt);
-                    n2row = lane < n2cnt ? p.order[cb + lane] : 0;
-                    aj = 0;
-                    if (ccnt <= 0) return 0;
-                    abase = __shfl_sync(0xffffffffu, cbeg, 0);
-                }
-                if (!slot_free(gen)) return -1;
-                const int row = __shfl_sync(0xffffffffu, crow, aj);
-                const int beg = __shfl_sync(0xffffffffu, cbeg, aj);
-                const int end = __shfl_sync(0xffffffffu, cend, aj);
-                const int cnt = min(KC, end - abase);
-                const int slot = (int)(gen % MR);
-                int32_t *mc = mcol + slot * KC;
-                float *mv = mval + slot * KC;
-    #pragma unroll
-                for (int h = 0; h < KC; h += 32) {
-                    if (lane + h < cnt) {
-                        cp_async4(smem_u32(mc + lane + h), p.idx + abase + lane + h, stream_pol);
-                        cp_async4(smem_u32(mv + lane + h), p.val + abase + lane + h, stream_pol);
-                    } else {
-                        mc[lane + h] = p.zero_row;   // the ragged tail gathers the all-zero row
-                        mv[lane + h] = 0.f;
+            int gen = 0, limit = 0;  // stages published; stages below `limit` have a free slot
+            // descriptor slots free from stage gen on, at least one (bounded wait; 0 on timeout
+            // or abort): slot g is free once stage g - MR has been read by its gather warp, and
+            // every stage below the least of their next stages has been
+            auto space = [&]() -> int {
+                if (gen < limit) return limit - gen;
+                const unsigned long long t0 = now_ns();
+                for (uint32_t k = 0;; ++k) {
+                    limit = MR + __reduce_min_sync(0xffffffffu, lane < NGATHER ? done[lane] : 0x3fffffff);
+                    if (gen < limit) break;
+                    if ((k & 255) == 255) {
+                        int stop = 0;
+                        if (lane == 0) stop = (*abort || now_ns() - t0 > p.wait_ns) ? 1 : 0;
+                        if (__shfl_sync(0xffffffffu, stop, 0)) return 0;
                     }
                 }
-                cp_commit();
-                if (lane == 0) {
-                    Meta m;
-                    m.row = row;
-                    m.cnt = cnt;
-                    m.flags = (abase == beg ? 1 : 0) | (abase + KC >= end ? 2 : 0);
-                    m.nu = end - beg;
-                    mmeta[slot] = m;
-                }
-                abase += KC;
-                if (abase >= end) {
-                    ++aj;
-                    abase = aj < ccnt ? __shfl_sync(0xffffffffu, cbeg, aj < ccnt ? aj : 0) : 0;
-                }
-                ++gen;
-                return 1;
+                __threadfence_block();
+                return limit - gen;
             };
             bool ok = true;
-            int more = 1;
-            for (int k = 0; k < MD && more == 1; ++k) more = generate();
-            if (more < 0) ok = false;
-            uint32_t it = 0;  // stages published
-            while (ok && it < gen) {
-                // stage it's metadata group: at most gen - it - 1 younger groups may stay pending
-                if (gen - it - 1 >= (uint32_t)(MD - 1))
-                    cp_wait<MD - 1>();
-                else
-                    cp_wait<0>();
-                __syncwarp();  // every lane's copies (and tail fills) of the stage are in place
-                if (lane == 0) {
-                    __threadfence_block();
-                    *pub = (int)(it + 1);
+            while (ok && ccnt > 0) {
+                for (int j = 0; j < ccnt && ok; ++j) {
+                    const int row = __shfl_sync(0xffffffffu, crow, j);
+                    const int beg = __shfl_sync(0xffffffffu, cbeg, j);
+                    const int end = __shfl_sync(0xffffffffu, cend, j);
+                    int base = beg;
+                    do {  // (a row without ratings is one empty stage)
+                        const int room = space();
+                        if (room <= 0) { ok = false; break; }
+                        const int n = min(max(1, (end - base + KC - 1) / KC), min(room, 32));
+                        if (lane < n) {
+                            const int b = base + lane * KC;
+                            const int flags = (b == beg ? 1 : 0) | (b + KC >= end ? 2 : 0);
+                            desc[(gen + lane) % MR] =
+                                make_int4(row, b, end - beg, min(KC, end - b) | flags << 16);
+                        }
+                        __threadfence_block();
+                        __syncwarp();
+                        gen += n;
+                        base += n * KC;
+                        if (lane == 0) *pub = gen;
+                    } while (base < end);
                 }
-                __syncwarp();
-                ++it;
-                if (more == 1) {
-                    more = generate();
-                    if (more < 0) ok = false;
-                }
+                ccnt = n1cnt; crow = n1row; cbeg = n1beg; cend = n1end;
+                n1cnt = n2cnt; n1row = n2row;
+                n1beg = lane < n1cnt ? p.ptr[n1row] : 0;     // n2's row ids landed a chunk ago
+                n1end = lane < n1cnt ? p.ptr[n1row + 1] : 0;
+                int cb;
+                grab(cb, n2cnt);
+                n2row = lane < n2cnt ? p.order[cb + lane] : 0;
             }
-            // nothing of this warp may be in flight when the CTA tears down
-            cp_wait<0>();
-            __syncwarp();
-            if (lane == 0) {  // *pub is now the number of stages; the gather warps add the end marker
+            if (ok && space() <= 0) ok = false;
+            if (ok && lane == 0) {  // the end of work, a stage of its own
+                desc[gen % MR] = make_int4(-1, 0, 0, 4 << 16);
+                __threadfence_block();
+                *pub = gen + 1;
                 __threadfence_block();
                 *fin = 1;
             }
@@ -1208,88 +1171,97 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
             }
         } else if (warp == WM) {
             // ------------------------------------------------------------------ MMA issuer
-            if (lane == 0) {
-                const int ng_mma = FUSED ? p.ng + 16 : p.ng;
-                const uint32_t idesc_g = F8 ? idesc_e4m3(128, ng_mma, true, true)
-                                            : idesc_bf16(128, ng_mma, true, true);
-                const uint32_t idesc_r = F8 ? idesc_e4m3(128, 16, true, false)
-                                            : idesc_bf16(128, 16, true, false);
-                const uint32_t ring_s = smem_u32(ring);
-                uint32_t it = 0, acc_it = 0, buf = 0;
-                bool ok = true;
-                auto take_buffer = [&]() -> bool {  // wait until accumulator acc_it % nbuf is free
-                    buf = acc_it % nbuf;
-                    const uint32_t use = acc_it / nbuf;
-                    if (use >= 1 &&
-                        !mbar_wait(smem_u32(&acc_empty[buf]), (use - 1) & 1, abort, p.wait_ns))
-                        return false;
-                    tc_fence_after();
-                    return true;
-                };
-                for (;;) {
-                    const int s = it % NSTAGE;
-                    // (every writer of the stage's operands fenced its generic stores into the async
-                    // proxy before it arrived: the acquire of this wait is all the MMA needs)
-                    if (!mbar_wait(smem_u32(FUSED ? &ready[s] : &full[s]), (it / NSTAGE) & 1, abort,
-                                   p.wait_ns)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const Meta m = smeta[s];
-                    if (m.row < 0) {  // end of work: one end marker per solver warpgroup
-                        for (int g = 0; g < NEPI && ok; ++g) {
-                            if (!take_buffer()) { ok = false; break; }
+            // The whole warp walks the stages on warp-uniform values (votes, a shuffled stage
+            // word, counters), so the MMAs' descriptors live in uniform registers; lane 0 alone
+            // issues, by predicate.
+            const uint32_t lead = lane == 0 ? 1u : 0u;
+            const int ng_mma = FUSED ? p.ng + 16 : p.ng;
+            const uint32_t idesc_g = F8 ? idesc_e4m3(128, ng_mma, true, true)
+                                        : idesc_bf16(128, ng_mma, true, true);
+            const uint32_t idesc_r = F8 ? idesc_e4m3(128, 16, true, false)
+                                        : idesc_bf16(128, 16, true, false);
+            const uint32_t ring_s = smem_u32(ring);
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+            bool ok = true;
+            int s = 0, buf = 0;                  // ring slot, accumulator
+            uint32_t s_phase = 0, b_phase = 1;   // (an accumulator's first use waits for nothing)
+            bool first_uses = true;  // until every accumulator has been used once
+            auto take_buffer = [&]() -> bool {  // wait until accumulator `buf` is free
+                if (!first_uses && !wait_all(smem_u32(&acc_empty[buf]), b_phase)) return false;
+                tc_fence_after();
+                return true;
+            };
+            auto next_buffer = [&]() {
+                if (++buf == nbuf) {
+                    buf = 0;
+                    first_uses = false;
+                    b_phase ^= 1u;
+                }
+            };
+            for (;;) {
+                // (every writer of the stage's operands fenced its generic stores into the async
+                // proxy before it arrived: the acquire of this wait is all the MMA needs)
+                if (!wait_all(smem_u32(&full[s]), s_phase)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const int4 d = sdes[s];
+                const int word = __shfl_sync(0xffffffffu, d.w, 0);  // cnt | flags << 16
+                const int cnt = word & 0xffff, flags = word >> 16;
+                const Meta m = {(flags & 4) ? -1 : d.x, d.z};
+                if (flags & 4) {  // end of work: one end marker per solver warpgroup
+                    for (int g = 0; g < NEPI; ++g) {
+                        if (!take_buffer()) { ok = false; break; }
+                        if (lane == 0) {
                             ameta[buf] = m;
                             mbar_arrive(smem_u32(&acc_meta[buf]));
-                            ++acc_it;
                         }
-                        break;
+                        __syncwarp();
+                        next_buffer();
                     }
-                    if ((m.flags & 1) && !take_buffer()) { ok = false; break; }
-                    const uint32_t dg = tmem_base + buf * p.acc_stride;
-                    const uint32_t db = dg + p.ng;
-                    const uint32_t tile_s = ring_s + s * SBYTES;
-                    if constexpr (F8) {
-                        // K = 32 ratings (four 8-rating groups, 4 KB of the one-atom panel) and the
-                        // matching 32 bytes of the rating tile's row per MMA
-                        const int nk = (m.cnt + F8_K - 1) / F8_K;
-                        for (int kk = 0; kk < nk; ++kk) {
-                            const uint64_t ad =
-                                sdesc(tile_s + kk * 4 * ATOM_BYTES, ATOM_STRIDE, ATOM_BYTES);
-                            const uint32_t accum = ((m.flags & 1) && kk == 0) ? 0u : 1u;
-                            mma_e4m3(dg, ad, ad, idesc_g, accum);
-                            if (!FUSED) {
-                                const uint64_t rd = sdesc(tile_s + TBYTES + kk * 32, 16, ATOM_BYTES);
-                                mma_e4m3(db, ad, rd, idesc_r, accum);
-                            }
-                        }
-                    } else {
-                        const int nk = (m.cnt + 15) >> 4;
-                        for (int kk = 0; kk < nk; ++kk) {
-                            const uint64_t ad =
-                                sdesc(tile_s + kk * 2 * ATOM_BYTES, ATOM_STRIDE, ATOM_BYTES);
-                            const uint32_t accum = ((m.flags & 1) && kk == 0) ? 0u : 1u;
-                            mma_bf16(dg, ad, ad, idesc_g, accum);
-                            if (!FUSED) {
-                                const uint64_t rd =
-                                    sdesc(tile_s + TBYTES + kk * 32, 16, ATOM_BYTES);
-                                mma_bf16(db, ad, rd, idesc_r, accum);
-                            }
-                        }
-                    }
-                    mma_commit(smem_u32(&empty[s]));
-                    if (m.flags & 2) {
-                        ameta[buf] = m;
-                        // committed for empty rows too, so buffer b's phase count is its use count
-                        mma_commit(smem_u32(&acc_full[buf]));
-                        mbar_arrive(smem_u32(&acc_meta[buf]));
-                        ++acc_it;
-                    }
-                    ++it;
+                    break;
                 }
-                // drain: every MMA issued so far has completed before TMEM is released
-                mma_commit(smem_u32(drain));
+                if ((flags & 1) && !take_buffer()) { ok = false; break; }
+                const uint32_t dg = tmem_u + buf * p.acc_stride;
+                const uint32_t db = dg + p.ng;
+                const uint32_t tile_s = ring_s + s * SBYTES;
+                // one MMA per 16 ratings (FP8: 32, four 8-rating groups)
+                const uint64_t ad = sdesc(tile_s, ATOM_STRIDE, ATOM_BYTES);
+                const uint64_t rd = sdesc(tile_s + TBYTES, 16, ATOM_BYTES);
+                const int nk = F8 ? (cnt + F8_K - 1) / F8_K : (cnt + 15) >> 4;
+#pragma unroll
+                for (int kk = 0; kk < (F8 ? 2 : 4); ++kk) {
+                    if (kk < nk) {
+                        const uint64_t a = ad + (uint64_t)(kk * (F8 ? 4 : 2) * (ATOM_BYTES >> 4));
+                        const uint64_t r = rd + (uint64_t)(kk * 2);  // 32 bytes a step
+                        const uint32_t accum = kk == 0 && (flags & 1) ? 0u : 1u;
+                        if constexpr (F8) {
+                            mma_e4m3(dg, a, a, idesc_g, accum, lead);
+                            if (!FUSED) mma_e4m3(db, a, r, idesc_r, accum, lead);
+                        } else {
+                            mma_bf16(dg, a, a, idesc_g, accum, lead);
+                            if (!FUSED) mma_bf16(db, a, r, idesc_r, accum, lead);
+                        }
+                    }
+                }
+                mma_commit(smem_u32(&empty[s]), lead);
+                if (flags & 2) {
+                    if (lane == 0) ameta[buf] = m;
+                    // committed for empty rows too, so buffer b's phase count is its use count
+                    mma_commit(smem_u32(&acc_full[buf]), lead);
+                    if (lane == 0) mbar_arrive(smem_u32(&acc_meta[buf]));
+                    __syncwarp();
+                    next_buffer();
+                }
+                if (++s == NSTAGE) {
+                    s = 0;
+                    s_phase ^= 1u;
+                }
+            }
+            // drain: every MMA issued so far has completed before TMEM is released
+            mma_commit(smem_u32(drain), lead);
+            if (lane == 0) {
                 if (!mbar_wait(smem_u32(drain), 0, nullptr, WAIT_NS)) ok = false;
                 if (!ok) {
                     *abort = 1;
@@ -1299,176 +1271,144 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
             __syncwarp();
         } else {
             // ------------------------------------------------------------------ gather warps
-            // Warp h takes every NGATHER-th stage from t = h once the producer has published it:
-            // it waits for the stage's ring slot, writes the rating tile, reads the column ids and
-            // Meta out of the metadata slot (handing the slot back), arms the stage's full barrier
-            // with the byte count and issues one tile::gather4 per lane (4 ratings x 64 features).
-            // The warp whose turn comes after the last stage writes the end marker (row = -1).
+            // Warp h takes every NGATHER-th stage from t = h once the producer has described it.
+            // It loads the stage's column ids and ratings into registers one turn ahead (their
+            // HBM latency passes behind the stage before), then waits for the stage's ring slot,
+            // copies the factor rows by 16-byte cp.async to their swizzled places, writes the
+            // ratings and, when the copies have landed, marks the stage full.
             const int h = warp - WG;
-            const int natoms = F8 ? 1 : (p.fst > 64 ? 2 : 1);
-            const int gq = lane & 15, ga = lane >> 4;  // this lane's 4-rating quad, atom
-            const uint64_t keep = l2_evict_last_policy();
-            bool ok = true;
-            for (uint32_t t = (uint32_t)h;; t += NGATHER) {
-                int go = 0;  // 1: stage t is published, 0: no more stages, -1: timed out or aborted
-                uint32_t total = 0;
-                if (lane == 0) {
+            const int nch = F8 ? p.ng >> 4 : p.fst >> 3;  // 16-byte chunks of a factor row
+            constexpr int LPR = F8 || FP <= 64 ? 8 : 16;  // lanes a factor row
+            const int gl = lane % LPR, gr = lane / LPR;     // this lane's chunk, its row group
+            const bool mine = gl < nch;
+            // Row group gr copies four consecutive rows of every 16 (LPR = 8) or 8 (LPR = 16):
+            // one 16-byte load gives their ids.  The chunk's place in the swizzled panel:
+            const int r4 = 4 * gr;  // first row of the four among 16 (LPR = 8) or 8
+            uint32_t place[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int k7 = (r4 + i) & 7;
+                place[i] = (uint32_t)((gl >> 3) * ATOM_STRIDE + (r4 >> 3) * ATOM_BYTES + k7 * 128 +
+                                      (((gl & 7) ^ k7) << 4));
+            }
+            const uint8_t *src0 = p.table + 16 * gl;
+            const uint32_t rb = (uint32_t)p.row_bytes;
+            const uint64_t keep = l2_evict_last_policy(), stream = l2_evict_first_policy();
+            int32_t *ids = wids + h * KC;
+            // stage t's descriptor: 1 taken, 0 no more stages, -1 timed out or aborted; then its
+            // ids and ratings are on their way
+            int4 d = make_int4(0, 0, 0, 0);
+            int32_t i0 = 0, i1 = 0;
+            float v0 = 0.f, v1 = 0.f;
+            uint32_t known = 0;  // stages this warp has seen published
+            auto take = [&](uint32_t t) -> int {
+                if (known <= t) {
                     const unsigned long long t0 = now_ns();
                     for (uint32_t k = 0;; ++k) {
-                        if ((uint32_t)*pub > t) { go = 1; break; }
-                        if (*fin) {
-                            total = (uint32_t)*pub;
-                            go = total > t ? 1 : 0;
-                            break;
-                        }
-                        if ((k & 255) == 255 && (*abort || now_ns() - t0 > p.wait_ns)) {
-                            go = -1;
-                            break;
+                        // *fin before *pub: then *pub is the final count
+                        const int last = __shfl_sync(0xffffffffu, ld_acquire(fin), 0);
+                        known = __shfl_sync(0xffffffffu, ld_acquire(pub), 0);
+                        if (known > t) break;
+                        if (last) return 0;
+                        if ((k & 63) == 63) {
+                            const int stop = lane == 0 && (*abort || now_ns() - t0 > p.wait_ns);
+                            if (__any_sync(0xffffffffu, stop)) return -1;
                         }
                     }
-                    __threadfence_block();
                 }
-                go = __shfl_sync(0xffffffffu, go, 0);
-                total = __shfl_sync(0xffffffffu, total, 0);
-                __syncwarp();  // the lanes' reads of the stage's metadata follow lane 0's acquire
-                if (go < 0) {
-                    ok = false;
+                d = desc[t % MR];
+                __syncwarp();
+                if (lane == 0) done[h] = (int)(t + NGATHER);  // the slot may be refilled
+                const int cnt = d.w & 0xffff;  // the ragged tail gathers the all-zero row
+                const int32_t *ip = p.idx + d.y + lane;
+                const float *vp = p.val + d.y + lane;
+                i0 = lane < cnt ? ld_stream(ip, stream) : p.zero_row;
+                i1 = lane + 32 < cnt ? ld_stream(ip + 32, stream) : p.zero_row;
+                v0 = lane < cnt ? ld_stream(vp, stream) : 0.f;
+                v1 = lane + 32 < cnt ? ld_stream(vp + 32, stream) : 0.f;
+                return 1;
+            };
+            bool ok = true;
+            int go = take((uint32_t)h);
+            for (uint32_t t = (uint32_t)h;; t += NGATHER) {
+                if (go <= 0) {
+                    ok = go == 0;
                     break;
                 }
-                if (go == 0 && t != total) break;  // another warp writes the end marker
+                // The slot's previous stage has been consumed (bounded wait).  Its barrier is at
+                // most one phase behind the one waited for, so the parity is unambiguous: this
+                // warp's last stage, t - NGATHER, waited for t - NGATHER - NSTAGE, stages are
+                // consumed in order and NGATHER <= NSTAGE.
                 const int s = t % NSTAGE;
-                if (t >= NSTAGE) {
-                    // the slot's previous stage (another warp's) is armed first: then the slot's
-                    // empty barrier is at most one phase behind the one waited for below, so its
-                    // parity cannot match an older phase
-                    int armed_ok = 1;
-                    if (lane == 0) {
-                        const unsigned long long t0 = now_ns();
-                        for (uint32_t k = 0;; ++k) {
-                            if (armed[s] >= (int)(t - NSTAGE)) break;
-                            if ((k & 255) == 255 && (*abort || now_ns() - t0 > p.wait_ns)) {
-                                armed_ok = 0;
-                                break;
-                            }
-                            }
-                        __threadfence_block();
-                    }
-                    if (!__shfl_sync(0xffffffffu, armed_ok, 0)) {
-                        ok = false;
-                        break;
-                    }
-                }
-                if (t >= NSTAGE &&
-                    !mbar_wait_warp(smem_u32(&empty[s]), ((t / NSTAGE) - 1) & 1, abort, p.wait_ns)) {
+                if (t >= NSTAGE && !wait_all(smem_u32(&empty[s]), ((t / NSTAGE) - 1) & 1)) {
                     ok = false;
                     break;
                 }
-                if (go == 0) {  // t == total: the end marker, one stage with row = -1
-                    if (lane == 0) {
-                        Meta m;
-                        m.row = -1;
-                        m.cnt = 0;
-                        m.flags = 3;
-                        m.nu = 0;
-                        smeta[s] = m;
-                        armed[s] = (int)t;  // (its phase completes on this arrive: no bytes)
-                        mbar_arrive(smem_u32(&full[s]));
-                        if (FUSED) mbar_arrive(smem_u32(&ready[s]));
-                    }
-                    __syncwarp();
+                const int cnt = d.w & 0xffff;
+                if (lane == 0) sdes[s] = d;
+                if (d.w >> 16 & 4) {  // the end of work: nothing to copy
+                    if (lane == 0) mbar_arrive(smem_u32(&full[s]));
                     break;
                 }
-                const int slot = (int)(t % MR);
-                Meta m;  // read by lane 0 (which saw the stage published), handed to the warp
-                {
-                    int4 w = make_int4(0, 0, 0, 0);
-                    if (lane == 0) w = *reinterpret_cast<const int4 *>(&mmeta[slot]);
-                    m.row = __shfl_sync(0xffffffffu, w.x, 0);
-                    m.cnt = __shfl_sync(0xffffffffu, w.y, 0);
-                    m.flags = __shfl_sync(0xffffffffu, w.z, 0);
-                    m.nu = __shfl_sync(0xffffffffu, w.w, 0);
-                }
+                ids[lane] = i0;
+                ids[lane + 32] = i1;
+                const float r0 = v0, r1 = v1;
+                __syncwarp();
+                go = take(t + NGATHER);  // the next stage's ids and ratings, behind this one
                 uint8_t *tile = ring + s * SBYTES;
-                __nv_bfloat16 *rt = reinterpret_cast<__nv_bfloat16 *>(tile + TBYTES);
-                if constexpr (F8) {  // e4m3 ratings (star ratings are exact), bytes 0..63 of row 0
-                    uint8_t *rt8 = tile + TBYTES;
-                    rt8[lane] = __nv_cvt_float_to_fp8(mval[slot * KC + lane], __NV_SATFINITE, __NV_E4M3);
-                    rt8[lane + 32] =
-                        __nv_cvt_float_to_fp8(mval[slot * KC + lane + 32], __NV_SATFINITE, __NV_E4M3);
-                } else {
-                    rt[lane] = __float2bfloat16_rn(mval[slot * KC + lane]);
-                    rt[lane + 32] = __float2bfloat16_rn(mval[slot * KC + lane + 32]);
-                }
-                // the MMA reads ratings [0, 16 nk) (FP8: [0, 32 nk)): gather their quads (the ragged
-                // tail's column ids point at the zero row), 512 bytes per quad and atom
-                const int nq = F8 ? ((m.cnt + F8_K - 1) / F8_K) * (F8_K / 4) : ((m.cnt + 15) >> 4) * 4;
-                const bool mine = gq < nq && ga < natoms;
-                int32_t r0 = 0, r1 = 0, r2 = 0, r3 = 0;
+                // the MMA reads ratings [0, 16 n16) (the ragged tail's column ids point at the
+                // zero row; FP8 contracts 32 at a time)
+                const int n16 = F8 ? ((cnt + F8_K - 1) / F8_K) * 2 : (cnt + 15) >> 4;
                 if (mine) {
-                    const int32_t *q = mcol + slot * KC + 4 * gq;
-                    r0 = q[0];
-                    r1 = q[1];
-                    r2 = q[2];
-                    r3 = q[3];
-                }
-                // the rating tile is a generic store: visible to the tensor core (async proxy)
-                // before the stage can complete
-                fence_async_smem();
-                __syncwarp();  // every lane has read the metadata slot and written its ratings
-                if (lane == 0) {
-                    __threadfence_block();
-                    done[h] = (int)(t + 1);  // the metadata slot may be refilled
-                    smeta[s] = m;
-                    armed[s] = (int)t;
-                    mbar_arrive_expect_tx(smem_u32(&full[s]), (uint32_t)(nq * natoms * 512));
-                }
-                __syncwarp();
-                if (mine) {
-                    const uint32_t dst = smem_u32(tile) + ga * ATOM_STRIDE + (gq >> 1) * ATOM_BYTES +
-                                         (gq & 1) * 512;
-                    tma_gather4(dst, &p.tmap, 64 * ga, r0, r1, r2, r3, smem_u32(&full[s]), keep);
-                }
-                __syncwarp();
-                if constexpr (FUSED) {
-                    // the stage's ratings into feature column ng, once its gathered rows have landed
-                    if (!mbar_wait_warp(smem_u32(&full[s]), (t / NSTAGE) & 1, abort, p.wait_ns)) {
-                        ok = false;
-                        break;
+                    constexpr int QUADS = LPR / 8;  // id loads for 16 ratings
+                    const int4 *iq = reinterpret_cast<const int4 *>(ids + r4);
+                    for (int g16 = 0; g16 < n16; ++g16) {
+                        const uint32_t dst = smem_u32(tile) + g16 * 2 * ATOM_BYTES;
+#pragma unroll
+                        for (int q = 0; q < QUADS; ++q) {
+                            const int4 id = iq[4 * g16 + 2 * q];
+                            const uint8_t *src[4] = {src0 + (uint64_t)(uint32_t)id.x * rb,
+                                                     src0 + (uint64_t)(uint32_t)id.y * rb,
+                                                     src0 + (uint64_t)(uint32_t)id.z * rb,
+                                                     src0 + (uint64_t)(uint32_t)id.w * rb};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                cp_async16(dst + q * ATOM_BYTES + place[i], src[i], keep);
+                        }
                     }
+                }
+                cp_commit();
+                // the ratings: into feature column ng of the panel (no chunk covers it), or the
+                // K-major rating tile's row 0 (e4m3: star ratings are exact)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int k = lane + 32 * e;
+                    const float r = e ? r1 : r0;
+                    uint8_t *row = tile + (k >> 3) * ATOM_BYTES + (k & 7) * 128;
                     if constexpr (F8) {
-                        // one 128-feature atom of bytes: column ng (a multiple of 16) starts
-                        // 16-byte chunk ng / 16 of each row, before the 128-byte swizzle
-                        const int rc = p.ng >> 4;
-                        const uint8_t *rt8 = tile + TBYTES;
-                        for (int k = lane; k < 4 * nq; k += 32)
-                            tile[(k >> 3) * ATOM_BYTES + (k & 7) * 128 + ((rc ^ (k & 7)) << 4)] =
-                                rt8[k];
+                        const uint8_t v = __nv_cvt_float_to_fp8(r, __NV_SATFINITE, __NV_E4M3);
+                        if (FUSED) row[((p.ng >> 4) ^ (k & 7)) << 4] = v;
+                        else tile[TBYTES + k] = v;
                     } else {
-                        const int ra = p.ng >> 6, rc = (p.ng & 63) >> 3;  // column ng: atom, chunk
-                        for (int k = lane; k < 4 * nq; k += 32)
-                            *reinterpret_cast<__nv_bfloat16 *>(tile + ra * ATOM_STRIDE +
-                                                               (k >> 3) * ATOM_BYTES + (k & 7) * 128 +
-                                                               ((rc ^ (k & 7)) << 4)) = rt[k];
+                        const __nv_bfloat16 v = __float2bfloat16_rn(r);
+                        if (FUSED)
+                            *reinterpret_cast<__nv_bfloat16 *>(
+                                row + (p.ng >> 6) * ATOM_STRIDE +
+                                ((((p.ng & 63) >> 3) ^ (k & 7)) << 4)) = v;
+                        else
+                            reinterpret_cast<__nv_bfloat16 *>(tile + TBYTES)[k] = v;
                     }
-                    fence_async_smem();  // generic stores, read by the tensor core
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&ready[s]));
                 }
+                // every lane's copies landed and its stores visible to the tensor core (async
+                // proxy) before the stage is marked full
+                cp_wait<0>();
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&full[s]));
             }
             if (!ok) {
                 *abort = 1;
                 if (lane == 0) atomicAdd(&p.flags[2], 1);
-            }
-            // no gather may be in flight when the CTA tears down: once every gather warp is done,
-            // wait for the last stage armed in each ring slot (a slot is re-armed only after the
-            // MMA consumed its previous stage, so only the last can still be landing; bounded)
-            asm volatile("bar.sync %0, %1;" ::"r"(15), "r"(32 * NGATHER) : "memory");
-            if (h == 0 && lane == 0) {
-                for (int u = 0; u < NSTAGE; ++u) {
-                    const int a = armed[u];
-                    if (a >= 0)
-                        mbar_wait(smem_u32(&full[u]), (uint32_t)(a / NSTAGE) & 1, nullptr, WAIT_NS);
-                }
             }
             __syncwarp();
         }
