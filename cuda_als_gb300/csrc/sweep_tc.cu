@@ -16,7 +16,7 @@
 //            selected solver (registers / shared memory, or the tensor core for the FP16-Gram CG);
 //            Cholesky refinement re-reads A from TMEM for the residual b - A x (in FP64 for rows
 //            whose Cholesky diagonal ratio exceeds cond_threshold).
-//   producer: cuts rows into stages (KC = 64 ratings each) and publishes their descriptors, up
+//   producer: cuts rows into stages (KC = 64 or 128 ratings each) and publishes their descriptors, up
 //            to 32 at once.
 //   NGATHER gather warps: take the stages round-robin; each loads its stage's column ids and
 //            ratings a turn ahead, copies the factor rows by 16-byte cp.async to their swizzled
@@ -26,15 +26,15 @@
 //            MN-major: Gram and right-hand side together; at f > 112 a Gram MMA and an N = 16
 //            MMA against the rating tile), into one of NBUF TMEM accumulators; tcgen05.commit
 //            frees the stage / publishes the row.
-// What bounds it, measured on one GB300 (98.6M ratings, f = 100, cycles a 64-rating stage an SM):
-// V half, FP16-Gram CG 680: the issuer's MMAs 300 (76 each, 64 at the tensor core's rate) and,
-// one after another, its wait, the stage's descriptor and the commits; 1,000 while one warp
-// published stage by stage and the rows came by TMA tile::gather4 (7 cycles a 128-byte row box, a
-// second limit at 900-1,000 cycles; cp.async takes 320).  U half, FP32 CG: the solves (an
-// accumulator is awaited for 780 of 1,770 cycles).
+// What bounds it, measured on one GB300 (98.6M ratings, f = 100, cycles per 64 ratings an SM): V
+// half, FP16-Gram CG 510: the issuer's MMAs 300 (76 each, 64 at the tensor core's rate) and, one
+// after another, its wait, the stage's descriptor and the commits; 1,000 while one warp published
+// stage by stage and the rows came by TMA tile::gather4 (7 cycles a 128-byte row box, a second
+// limit at 900-1,000 cycles; cp.async takes 320).  U half, FP32 CG: the solves (an accumulator is
+// awaited for 780 of 1,770 cycles).
 // Operand layout (one stage): 2 atoms of 64 features x KC ratings; atom a, rating k, feature chunk
-// c (8 features, 16 B) sits at a*8192 + (k/8)*1024 + (k%8)*128 + ((c%8) ^ (k%8))*16, i.e. the
-// canonical SWIZZLE_128B MN-major layout with LBO = 8192 (between 64-feature atoms) and
+// c (8 features, 16 B) sits at a*128*KC + (k/8)*1024 + (k%8)*128 + ((c%8) ^ (k%8))*16, i.e. the
+// canonical SWIZZLE_128B MN-major layout with LBO = 128 KC (between 64-feature atoms) and
 // SBO = 1024 (between 8-rating groups).  Features f..127 are zero (written once).
 //
 // Every wait is bounded by %globaltimer: a wait that runs out sets the status word, the kernel

@@ -15,7 +15,6 @@
 namespace als {
 namespace tcg {
 
-constexpr int KC = 64;                       // ratings per stage
 constexpr int MAX_NSTAGE = 16;
 // CG at FP = 64, 112 and 128 quad-blocks its rows (cg_quad): half of a row's values in
 // registers, half in shared memory (2 FP/16 slots of CGQ_SLOT float4 a group), so four groups
@@ -25,16 +24,28 @@ __host__ __device__ constexpr bool cg_quad_rows(int solver, int fp) {
 }
 __host__ __device__ constexpr int cgq_floats(int fp) { return 2 * (fp / 16) * 130 * 4; }
 constexpr int ATOM_BYTES = 1024;             // 8 ratings x 128 B
-constexpr int ATOM_STRIDE = (KC / 8) * ATOM_BYTES;  // 8192: LBO between 64-feature atoms
-constexpr int TILE_BYTES = 2 * ATOM_STRIDE;  // 128 features
-constexpr int R_BYTES = 2 * ATOM_BYTES;      // K-major rating tile, N = 16 rows x 64 ratings
-// FP8 stages: one 128-feature atom of KC ratings (8 KB)
-constexpr int TILE_BYTES_F8 = ATOM_STRIDE;
-__host__ __device__ constexpr int tile_bytes(bool f8) { return f8 ? TILE_BYTES_F8 : TILE_BYTES; }
 // The ratings ride in the panel's feature column ng (sweep_tc_kernel, FUSED) where there is one.
 __host__ __device__ constexpr bool fused_of(int fp) { return fp <= 112; }
-__host__ __device__ constexpr int stage_bytes(int fp, bool f8) {
-    return tile_bytes(f8) + (fused_of(fp) ? 0 : R_BYTES);
+// Ratings a stage.  The issuer's wait, descriptor and commits cost about 370 cycles a stage beside
+// its MMAs, so where the ring still holds five stages they are of 128 ratings: V half of 98.6M
+// ratings, f = 100, FP16-Gram CG 3.47 -> 2.70 ms; FP8, f = 128, FP32 CG 3.71 -> 2.93 ms.  The
+// BF16 FP32 CG, Cholesky and LU keep their groups' rows in shared memory and stay at 64.
+__host__ __device__ constexpr int kc_of(int solver, int fp, bool f8) {
+    return f8 || solver == 3 ? 128 : 64;
+}
+// LBO between the panel's 64-feature atoms; a BF16 panel has two (128 features), FP8 one.
+__host__ __device__ constexpr int atom_stride_of(int kc) { return kc / 8 * ATOM_BYTES; }
+__host__ __device__ constexpr int tile_bytes(int kc, bool f8) {
+    return (f8 ? 1 : 2) * atom_stride_of(kc);
+}
+// K-major rating tile: N = 16 rows of 128-byte lines, 64 BF16 ratings or 128 FP8 ones a line.
+constexpr int R_ATOM = 2 * ATOM_BYTES;
+__host__ __device__ constexpr int rating_bytes(int kc, bool f8) {
+    return f8 ? R_ATOM : kc / 64 * R_ATOM;
+}
+__host__ __device__ constexpr int stage_bytes(int solver, int fp, bool f8) {
+    const int kc = kc_of(solver, fp, f8);
+    return tile_bytes(kc, f8) + (fused_of(fp) ? 0 : rating_bytes(kc, f8));
 }
 constexpr int MAXF = 128;
 constexpr int MAX_NBUF = 4;
@@ -46,7 +57,8 @@ constexpr int MR = 32;
 // the gather warps, which take the stages round-robin: a gather warp loads its stage's column ids
 // and ratings one stage ahead, copies the factor rows and marks the stage full.
 constexpr int MAX_NGATHER = 6;
-constexpr int MRING_BYTES = MR * 16 + MAX_NGATHER * KC * 4;  // descriptors, a gather warp's ids
+constexpr int MAX_KC = 128;
+constexpr int MRING_BYTES = MR * 16 + MAX_NGATHER * MAX_KC * 4;  // descriptors, a gather warp's ids
 // SOLVER_CGTC: CG on the Gram rounded to binary16's significand (the reference's FP16-Gram CG),
 // its products A p run on the tensor core from the accumulator left in TMEM.
 enum { SOLVER_CG = 0, SOLVER_CHOL = 1, SOLVER_LU = 2, SOLVER_CGTC = 3 };
@@ -76,8 +88,8 @@ __host__ __device__ constexpr int nepi_of(int solver, int fp) {
 }
 // Gather warps: six take a stage in the time of its MMAs (two: V half of 98.6M ratings at f = 100
 // with the FP32 CG 5.69 ms, six 3.57).  A launch's registers are shared out per four warps, so
-// above 640 threads a thread keeps 80 and at 640 it keeps 96.  The tensor-core CG (about 70 a
-// thread) takes six as it is; the Cholesky factor and LU (96 and more) two.  The quad-blocked CG
+// above 640 threads a thread keeps 80 and at 640 it keeps 96.  The tensor-core CG (80 a thread)
+// takes five, as many as its ring has stages; the Cholesky factor and LU (96 and more) two.  The quad-blocked CG
 // splits its registers (setmaxnreg): launched with six gather warps at 80 a thread (FP = 128, three
 // groups: 96), its solver warpgroups take 96 (128) and the two service warpgroups (producer, MMA
 // issuer, gather warps) give theirs back down to SERVICE_REGS, the sum being exactly what the
@@ -86,7 +98,7 @@ __host__ __device__ constexpr bool regsplit_of(int solver, int fp) {
     return cg_quad_rows(solver, fp);
 }
 __host__ __device__ constexpr int ngather_of(int solver, int fp) {
-    return solver == 3 || regsplit_of(solver, fp) ? 6 : 2;
+    return solver == 3 ? 5 : regsplit_of(solver, fp) ? 6 : 2;
 }
 __host__ __device__ constexpr int nthreads_of(int solver, int fp) {
     return 128 * nepi_of(solver, fp) + 32 * (2 + ngather_of(solver, fp));
@@ -184,7 +196,7 @@ constexpr size_t SMEM_BUDGET = 232448 - 2048;  // the opt-in limit per CTA, less
 __host__ __device__ constexpr int nstage_fit(int solver, int fp, bool f8) {
     return (int)((SMEM_BUDGET - sizeof(float) * group_floats(fp, solver) * nepi_of(solver, fp) -
                   (size_t)MRING_BYTES - 1024 - (f8 ? sizeof(float) * MAXF : 0)) /
-                 (size_t)stage_bytes(fp, f8));
+                 (size_t)stage_bytes(solver, fp, f8));
 }
 __host__ __device__ constexpr int nstage_of(int solver, int fp, bool f8) {
     return nstage_fit(solver, fp, f8) > MAX_NSTAGE ? MAX_NSTAGE : nstage_fit(solver, fp, f8);
@@ -206,7 +218,7 @@ inline Geometry geometry(int f, int solver, bool f8 = false) {
     g.tmem_cols = cols;
     g.nthreads = nthreads_of(solver, g.fp);
     const int ns = nstage_of(solver, g.fp, f8);
-    size_t bytes = (size_t)ns * stage_bytes(g.fp, f8);                     // operand ring
+    size_t bytes = (size_t)ns * stage_bytes(solver, g.fp, f8);                     // operand ring
     bytes += sizeof(float) * group_floats(g.fp, solver) * g.nepi;    // per-group scratch
     if (f8) bytes += sizeof(float) * MAXF;                            // per-feature scales
     bytes += MRING_BYTES;                                            // metadata ring
@@ -914,7 +926,9 @@ template <int FP, int SOLVER, bool F8>
 __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
     sweep_tc_kernel(const __grid_constant__ Params p) {
     constexpr int NSTAGE = nstage_of(SOLVER, FP, F8);
-    constexpr int SBYTES = stage_bytes(FP, F8), TBYTES = tile_bytes(F8);
+    constexpr int KC = kc_of(SOLVER, FP, F8), ATOM_STRIDE = atom_stride_of(KC);
+    constexpr int SBYTES = stage_bytes(SOLVER, FP, F8), TBYTES = tile_bytes(KC, F8);
+    static_assert(KC % 64 == 0 && KC <= MAX_KC, "stage");
     static_assert(NSTAGE >= 2 && NSTAGE <= MAX_NSTAGE, "stage ring");
     constexpr int NEPI = nepi_of(SOLVER, FP);
     constexpr int WP = 4 * NEPI;  // producer warp; then the MMA issuer and the gather warps
@@ -1231,10 +1245,10 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                 const uint64_t rd = sdesc(tile_s + TBYTES, 16, ATOM_BYTES);
                 const int nk = F8 ? (cnt + F8_K - 1) / F8_K : (cnt + 15) >> 4;
 #pragma unroll
-                for (int kk = 0; kk < (F8 ? 2 : 4); ++kk) {
+                for (int kk = 0; kk < KC / (F8 ? 32 : 16); ++kk) {
                     if (kk < nk) {
                         const uint64_t a = ad + (uint64_t)(kk * (F8 ? 4 : 2) * (ATOM_BYTES >> 4));
-                        const uint64_t r = rd + (uint64_t)(kk * 2);  // 32 bytes a step
+                        const uint64_t r = rd + (uint64_t)(F8 ? 2 * kk : (kk & 3) * 2 + (kk >> 2) * (R_ATOM >> 4));
                         const uint32_t accum = kk == 0 && (flags & 1) ? 0u : 1u;
                         if constexpr (F8) {
                             mma_e4m3(dg, a, a, idesc_g, accum, lead);
@@ -1298,8 +1312,9 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
             // stage t's descriptor: 1 taken, 0 no more stages, -1 timed out or aborted; then its
             // ids and ratings are on their way
             int4 d = make_int4(0, 0, 0, 0);
-            int32_t i0 = 0, i1 = 0;
-            float v0 = 0.f, v1 = 0.f;
+            constexpr int PER = KC / 32;  // ids and ratings a lane
+            int32_t iv[PER];
+            float vv[PER];
             uint32_t known = 0;  // stages this warp has seen published
             auto take = [&](uint32_t t) -> int {
                 if (known <= t) {
@@ -1322,10 +1337,11 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                 const int cnt = d.w & 0xffff;  // the ragged tail gathers the all-zero row
                 const int32_t *ip = p.idx + d.y + lane;
                 const float *vp = p.val + d.y + lane;
-                i0 = lane < cnt ? ld_stream(ip, stream) : p.zero_row;
-                i1 = lane + 32 < cnt ? ld_stream(ip + 32, stream) : p.zero_row;
-                v0 = lane < cnt ? ld_stream(vp, stream) : 0.f;
-                v1 = lane + 32 < cnt ? ld_stream(vp + 32, stream) : 0.f;
+#pragma unroll
+                for (int e = 0; e < PER; ++e) {
+                    iv[e] = lane + 32 * e < cnt ? ld_stream(ip + 32 * e, stream) : p.zero_row;
+                    vv[e] = lane + 32 * e < cnt ? ld_stream(vp + 32 * e, stream) : 0.f;
+                }
                 return 1;
             };
             bool ok = true;
@@ -1350,9 +1366,12 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                     if (lane == 0) mbar_arrive(smem_u32(&full[s]));
                     break;
                 }
-                ids[lane] = i0;
-                ids[lane + 32] = i1;
-                const float r0 = v0, r1 = v1;
+                float rv[PER];
+#pragma unroll
+                for (int e = 0; e < PER; ++e) {
+                    ids[lane + 32 * e] = iv[e];
+                    rv[e] = vv[e];
+                }
                 __syncwarp();
                 go = take(t + NGATHER);  // the next stage's ids and ratings, behind this one
                 uint8_t *tile = ring + s * SBYTES;
@@ -1381,9 +1400,9 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                 // the ratings: into feature column ng of the panel (no chunk covers it), or the
                 // K-major rating tile's row 0 (e4m3: star ratings are exact)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
+                for (int e = 0; e < PER; ++e) {
                     const int k = lane + 32 * e;
-                    const float r = e ? r1 : r0;
+                    const float r = rv[e];
                     uint8_t *row = tile + (k >> 3) * ATOM_BYTES + (k & 7) * 128;
                     if constexpr (F8) {
                         const uint8_t v = __nv_cvt_float_to_fp8(r, __NV_SATFINITE, __NV_E4M3);
@@ -1396,7 +1415,7 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                                 row + (p.ng >> 6) * ATOM_STRIDE +
                                 ((((p.ng & 63) >> 3) ^ (k & 7)) << 4)) = v;
                         else
-                            reinterpret_cast<__nv_bfloat16 *>(tile + TBYTES)[k] = v;
+                            reinterpret_cast<__nv_bfloat16 *>(tile + TBYTES + (k >> 6) * R_ATOM)[k & 63] = v;
                     }
                 }
                 // every lane's copies landed and its stores visible to the tensor core (async
