@@ -70,12 +70,11 @@ __host__ __device__ constexpr int cgtc_tile_floats(int fp) { return (fp / 8) * 6
 
 // TMEM accumulators (ng + 16 columns: four fit in 512 columns unless FP = 128, whose rows have
 // ng = 128: two at a 256-column stride, or three at 160 for the quad-blocked CG, whose stride
-// need not be a power of two) and solver groups: CG and LU read their row out of TMEM into
-// registers at once and release the buffer, so the MMA fills the next row while they solve;
-// their register-resident rows allow two groups per SM.  A Cholesky group keeps its buffer until
-// refinement has re-read A, and its factor lives in shared memory: one group per buffer; so does
-// the quad-blocked CG (half of each row in shared memory), and the tensor-core CG, whose products
-// read A from the buffer until the solve ends.
+// need not be a power of two) and solver groups, one per accumulator: a Cholesky group keeps its
+// buffer until refinement has re-read A and the tensor-core CG until its solve ends (its products
+// read A there); the FP32 CG reads its row out at once and hands the buffer back, but four solves
+// side by side hide each other's latency (f = 32, 98.6M ratings, users: two groups 10.5 ms, four
+// 6.6).  LU keeps whole rows in registers: two groups.
 __host__ __device__ constexpr int nbuf_of(int solver, int fp) {
     return fp != 128 ? 4 : cg_quad_rows(solver, fp) ? 3 : 2;
 }
@@ -83,8 +82,7 @@ __host__ __device__ constexpr int acc_stride_of(int solver, int fp, int ng) {
     return ng + 16 <= 128 ? 128 : nbuf_of(solver, fp) == 3 ? 160 : 256;
 }
 __host__ __device__ constexpr int nepi_of(int solver, int fp) {
-    return solver == 1 || solver == 3 || cg_quad_rows(solver, fp) ? nbuf_of(solver, fp)
-                                                                   : nbuf_of(solver, fp) / 2;
+    return solver == 2 ? nbuf_of(solver, fp) / 2 : nbuf_of(solver, fp);
 }
 // Gather warps: six take a stage in the time of its MMAs (two: V half of 98.6M ratings at f = 100
 // with the FP32 CG 5.69 ms, six 3.57).  A launch's registers are shared out per four warps, so
@@ -98,7 +96,7 @@ __host__ __device__ constexpr bool regsplit_of(int solver, int fp) {
     return cg_quad_rows(solver, fp);
 }
 __host__ __device__ constexpr int ngather_of(int solver, int fp) {
-    return solver == 3 ? 5 : regsplit_of(solver, fp) ? 6 : 2;
+    return solver == 3 ? 5 : solver == 0 ? 6 : 2;
 }
 __host__ __device__ constexpr int nthreads_of(int solver, int fp) {
     return 128 * nepi_of(solver, fp) + 32 * (2 + ngather_of(solver, fp));
