@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "handle.h"
@@ -39,7 +40,7 @@ constexpr int KC = 32;
 constexpr int MAX_FP = 232;      // FP32: the Gram of FP x (FP+1) floats in shared memory
 constexpr int MAX_F_F64 = 128;   // FP64: the Gram of 136 x 137 doubles (149 KB)
 constexpr int ITEM_WARPS = 8;
-constexpr int ITEM_Q = (MAX_FP + 31) / 32;  // feature slots per lane in the item kernel
+constexpr int AHEAD = 2;  // entries of an item whose rows a warp has in flight
 constexpr int32_t ITEM_CHUNK = 2048;        // training ratings per chunk of an item's column
 
 __host__ __device__ inline int fp_of(int f) { return ((f + 1 + 7) / 8) * 8; }
@@ -381,7 +382,8 @@ cudaError_t launch_rows(const AdjArgs<float> &a, int64_t m, cudaStream_t st) {
 // ratings.  Warp w of the chunk's CTA takes entries w, w + ITEM_WARPS, ... in order; lane l
 // holds features l, l + 32, ...; the warps' partial vectors are added in warp order into
 // part[c].  Heavy items (hundreds of thousands of ratings) spread over many CTAs this way.
-template <typename T>
+// ITEM_Q: features a lane, ceil(f / 32).
+template <typename T, int ITEM_Q>
 __global__ void __launch_bounds__(32 * ITEM_WARPS)
     adjoint_chunk_kernel(int64_t nchunks, int f, const int32_t *__restrict__ citem,
                          const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cend,
@@ -403,36 +405,58 @@ __global__ void __launch_bounds__(32 * ITEM_WARPS)
             y[q] = q < nq && j < f ? Y[it * f + j] : T(0);
             acc[q] = T(0);
         }
-        auto dot = [&](const T *v) -> T {
+        auto dot = [&](const T (&v)[ITEM_Q]) -> T {
             T s = T(0);
 #pragma unroll
-            for (int q = 0; q < ITEM_Q; ++q) {
-                const int j = lane + 32 * q;
-                if (q < nq && j < f) s = fma_t<T>(y[q], v[j], s);
-            }
+            for (int q = 0; q < ITEM_Q; ++q)
+                if (q < nq && lane + 32 * q < f) s = fma_t<T>(y[q], v[q], s);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             return s;
         };
-        for (int e = cbeg[ch] + warp; e < cend[ch]; e += ITEM_WARPS) {
-            const T *xu = X + (int64_t)cusr[e] * f;
-            const T *gu = G + (int64_t)cusr[e] * f;
-            const T yx = dot(xu), gy = dot(gu);
-            const T c = (T)cval[e] - yx;
+        auto load = [&](const T *row, T (&v)[ITEM_Q]) {
 #pragma unroll
             for (int q = 0; q < ITEM_Q; ++q) {
                 const int j = lane + 32 * q;
-                if (q < nq && j < f) acc[q] = fma_t<T>(c, gu[j], fma_t<T>(-gy, xu[j], acc[q]));
+                v[q] = q < nq && j < f ? row[j] : T(0);
+            }
+        };
+        // AHEAD entries' rows in flight, then their contributions in order
+        const int end = cend[ch];
+        for (int e0 = cbeg[ch] + warp; e0 < end; e0 += AHEAD * ITEM_WARPS) {
+            T xu[AHEAD][ITEM_Q], gu[AHEAD][ITEM_Q], c[AHEAD];
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                const int e = e0 + k * ITEM_WARPS;
+                if (e < end) {  // (warp-uniform)
+                    const int64_t u = cusr[e];
+                    c[k] = (T)cval[e];
+                    load(X + u * f, xu[k]);
+                    load(G + u * f, gu[k]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                if (e0 + k * ITEM_WARPS >= end) continue;
+                const T yx = dot(xu[k]), gy = dot(gu[k]);
+                const T ck = c[k] - yx;
+#pragma unroll
+                for (int q = 0; q < ITEM_Q; ++q) {
+                    const int j = lane + 32 * q;
+                    if (q < nq && j < f)
+                        acc[q] = fma_t<T>(ck, gu[k][q], fma_t<T>(-gy, xu[k][q], acc[q]));
+                }
             }
         }
         if (first) {
             for (int e = hptr[it] + warp; e < hptr[it + 1]; e += ITEM_WARPS) {
-                const T *xu = X + (int64_t)husr[e] * f;
+                T xu[ITEM_Q];
+                load(X + (int64_t)husr[e] * f, xu);
                 const T res = (T)hval[e] - dot(xu);
 #pragma unroll
                 for (int q = 0; q < ITEM_Q; ++q) {
                     const int j = lane + 32 * q;
-                    if (q < nq && j < f) acc[q] = fma_t<T>(T(-2) * res, xu[j], acc[q]);
+                    if (q < nq && j < f) acc[q] = fma_t<T>(T(-2) * res, xu[q], acc[q]);
                 }
             }
         }
@@ -465,12 +489,22 @@ __global__ void adjoint_combine_kernel(int64_t n, int f, const int32_t *__restri
     }
 }
 
+// out[k] = sum of v[k n .. k n + n), k = blockIdx.x, in a fixed order (eight loads in flight).
 __global__ void sum_doubles_kernel(const double *__restrict__ v, int64_t n, double *out) {
     __shared__ double sh[33];
+    v += blockIdx.x * n;
     double acc = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) acc += v[i];
+    int64_t i = threadIdx.x;
+    for (; i + 7 * (int64_t)blockDim.x < n; i += 8 * (int64_t)blockDim.x) {
+        double x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = v[i + k * (int64_t)blockDim.x];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc += x[k];
+    }
+    for (; i < n; i += blockDim.x) acc += v[i];
     const double s = block_sum_d(acc, sh);
-    if (threadIdx.x == 0) *out = s;
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 __global__ void f64_to_f32_kernel(const double *__restrict__ a, int64_t n, float *__restrict__ b) {
@@ -479,22 +513,78 @@ __global__ void f64_to_f32_kernel(const double *__restrict__ a, int64_t n, float
         b[i] = (float)a[i];
 }
 
-// Counting sort of the held-out triples by `key` (rows or columns), stable: ptr (nkeys + 1),
-// the other index and the value per entry.
-void group_by(int64_t nkeys, int64_t nh, const int32_t *key, const int32_t *other,
-              const float *vals, std::vector<int32_t> &ptr, std::vector<int32_t> &oth,
-              std::vector<float> &val) {
-    ptr.assign((size_t)nkeys + 1, 0);
-    oth.assign((size_t)(nh > 0 ? nh : 1), 0);
-    val.assign((size_t)(nh > 0 ? nh : 1), 0.f);
-    for (int64_t e = 0; e < nh; ++e) ptr[key[e] + 1]++;
-    for (int64_t r = 0; r < nkeys; ++r) ptr[r + 1] += ptr[r];
-    std::vector<int32_t> cur(ptr.begin(), ptr.end() - 1);
-    for (int64_t e = 0; e < nh; ++e) {
-        const int32_t p = cur[key[e]]++;
-        oth[p] = other[e];
-        val[p] = vals[e];
+// dst[p] = src[perm[p]] for an index and a value array.
+__global__ void gather_held_kernel(int64_t n, const int32_t *__restrict__ perm,
+                                   const int32_t *__restrict__ idx, const float *__restrict__ val,
+                                   int32_t *__restrict__ didx, float *__restrict__ dval) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
+         p += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t q = perm[p];
+        didx[p] = idx[q];
+        dval[p] = val[q];
     }
+}
+
+// Held-out triples grouped by `key` (rows or columns), stable: ptr (nkeys + 1), the other index
+// and the value per entry.
+cudaError_t group_held(int64_t nkeys, int64_t nh, const int32_t *key, const int32_t *other,
+                       const float *val, int32_t *skey, int32_t *perm, void *scratch,
+                       int32_t *ptr, int32_t *oth, float *gval, cudaStream_t st) {
+    if (nh > 0) {
+        const cudaError_t e = radix_sort_pairs(key, nullptr, skey, perm, nh,
+                                               (int32_t)(nkeys > 0 ? nkeys - 1 : 0), scratch, st);
+        if (e != cudaSuccess) return e;
+        gather_held_kernel<<<(unsigned)std::min<int64_t>((nh + 255) / 256, 152 * 16), 256, 0, st>>>(
+            nh, perm, other, val, oth, gval);
+    }
+    return ptrs_from_sorted(nh, nkeys, skey, ptr, st);
+}
+
+// Chunks of at most ITEM_CHUNK training ratings per item (one for an item without any): item,
+// first and last rating (nchunks each), then the first chunk of every item (n + 1).
+cudaError_t build_chunks(als_handle *h) {
+    als_handle::Adjoint &ad = h->adj;
+    if (ad.built) return cudaSuccess;
+    const std::vector<int32_t> &cp = h->host_ptr[1];
+    const int64_t n = h->n;
+    int64_t nchunks = 0;
+    for (int64_t i = 0; i < n; ++i)
+        nchunks += std::max<int64_t>(1, ((int64_t)cp[i + 1] - cp[i] + ITEM_CHUNK - 1) / ITEM_CHUNK);
+    std::vector<int32_t> tab((size_t)(3 * nchunks + n + 1));
+    int32_t *citem = tab.data(), *cbeg = citem + nchunks, *cend = cbeg + nchunks, *cfirst = cend + nchunks;
+    int64_t c = 0;
+    for (int64_t i = 0; i < n; ++i) {
+        cfirst[i] = (int32_t)c;
+        int32_t s = cp[i];
+        do {
+            citem[c] = (int32_t)i;
+            cbeg[c] = s;
+            cend[c++] = std::min(cp[i + 1], s + ITEM_CHUNK);
+            s += ITEM_CHUNK;
+        } while (s < cp[i + 1]);
+    }
+    cfirst[n] = (int32_t)c;
+    cudaError_t e = cudaMalloc(&ad.d_chunks, sizeof(int32_t) * tab.size());
+    if (e == cudaSuccess)
+        e = cudaMemcpy(ad.d_chunks, tab.data(), sizeof(int32_t) * tab.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    ad.nchunks = nchunks;
+    ad.built = true;
+    return cudaSuccess;
+}
+
+// The first held-out entry out of range or not finite, or nnz.
+int64_t first_bad_heldout(const als_handle *h, const als_coo_view *held) {
+    int64_t e = 0;
+    for (; e < held->nnz; ++e) {
+        const int32_t r = held->row_idxs[e], c = held->col_idxs[e];
+        if (r < 0 || r >= h->m || c < 0 || c >= h->n || !std::isfinite(held->vals[e])) break;
+    }
+    return e;
+}
+als_status bad_heldout(const als_handle *h, const als_coo_view *held) {
+    return set_global_error(ALS_ERR_INVALID_ARG, "held-out entry out of range at " +
+                                                     std::to_string(first_bad_heldout(h, held)));
 }
 
 // The adjoint in precision T.  Y: device item factors in T (n x f); dLdY: host, n x f of
@@ -505,59 +595,83 @@ als_status adjoint_impl(als_handle *h, const als_coo_view *held, const T *d_Y, T
     const int f = h->f;
     const int FP = fp_of(f);
     const int64_t m = h->m, n = h->n, nh = held->nnz;
-    std::vector<int32_t> hptr_u, hcol_u, hptr_i, hrow_i;
-    std::vector<float> hval_u, hval_i;
-    group_by(m, nh, held->row_idxs, held->col_idxs, held->vals, hptr_u, hcol_u, hval_u);
-    group_by(n, nh, held->col_idxs, held->row_idxs, held->vals, hptr_i, hrow_i, hval_i);
-    // chunks of at most ITEM_CHUNK training ratings per item (one for an item without any)
-    const std::vector<int32_t> &cp = h->host_ptr[1];
-    std::vector<int32_t> citem, cbeg, cend, cfirst((size_t)n + 1, 0);
-    for (int64_t i = 0; i < n; ++i) {
-        cfirst[i] = (int32_t)citem.size();
-        const int32_t b = cp[i], e = cp[i + 1];
-        int32_t s = b;
-        do {
-            citem.push_back((int32_t)i);
-            cbeg.push_back(s);
-            cend.push_back(std::min(e, s + ITEM_CHUNK));
-            s += ITEM_CHUNK;
-        } while (s < e);
-    }
-    cfirst[n] = (int32_t)citem.size();
-    const int64_t nchunks = (int64_t)citem.size();
     cudaStream_t st = h->stream;
-    int32_t *d_hptr_u = nullptr, *d_hcol_u = nullptr, *d_hptr_i = nullptr, *d_hrow_i = nullptr;
-    float *d_hval_u = nullptr, *d_hval_i = nullptr;
-    T *d_X = nullptr, *d_G = nullptr, *d_dY = nullptr, *d_part = nullptr;
-    int32_t *d_chunks = nullptr;  // citem, cbeg, cend (nchunks each), cfirst (n + 1)
-    double *d_parts = nullptr;
     cudaError_t e = cudaSuccess;
     auto step = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    const size_t nhp = hcol_u.size();
-    step(cudaMalloc(&d_hptr_u, sizeof(int32_t) * (m + 1)));
-    step(cudaMalloc(&d_hcol_u, sizeof(int32_t) * nhp));
-    step(cudaMalloc(&d_hval_u, sizeof(float) * nhp));
-    step(cudaMalloc(&d_hptr_i, sizeof(int32_t) * (n + 1)));
-    step(cudaMalloc(&d_hrow_i, sizeof(int32_t) * nhp));
-    step(cudaMalloc(&d_hval_i, sizeof(float) * nhp));
-    step(cudaMalloc(&d_X, sizeof(T) * (size_t)(m * f)));
-    step(cudaMalloc(&d_G, sizeof(T) * (size_t)(m * f)));
-    step(cudaMalloc(&d_dY, sizeof(T) * (size_t)(n * f)));
-    step(cudaMalloc(&d_parts, sizeof(double) * (size_t)(2 * m + 2)));
-    step(cudaMalloc(&d_chunks, sizeof(int32_t) * (size_t)(3 * nchunks + n + 1)));
-    step(cudaMalloc(&d_part, sizeof(T) * (size_t)(nchunks * f + 1)));
+    auto failed = [&]() {
+        h->last_error = std::string("adjoint: ") + cudaGetErrorString(e);
+        return set_global_error(e == cudaErrorMemoryAllocation ? ALS_ERR_OUT_OF_MEMORY : ALS_ERR_CUDA,
+                                h->last_error);
+    };
+    step(build_chunks(h));
+    if (e != cudaSuccess) return failed();
+    const int64_t nchunks = h->adj.nchunks;
+    const int32_t *d_chunks = h->adj.d_chunks;
+    // the workspace, carved twice: once for its size
+    int32_t *d_in[2] = {nullptr, nullptr}, *d_skey = nullptr, *d_perm = nullptr;
+    int32_t *d_hptr_u = nullptr, *d_hcol_u = nullptr, *d_hptr_i = nullptr, *d_hrow_i = nullptr;
+    float *d_inv = nullptr, *d_hval_u = nullptr, *d_hval_i = nullptr;
+    T *d_X = nullptr, *d_G = nullptr, *d_dY = nullptr, *d_part = nullptr;
+    double *d_parts = nullptr;
+    void *d_sort = nullptr;
+    const size_t nhp = (size_t)(nh > 0 ? nh : 1);
+    auto carve = [&](char *base) -> size_t {
+        size_t off = 0;
+        auto take = [&](auto *&p, size_t count) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + off);
+            off += (count * sizeof(*p) + 255) / 256 * 256;
+        };
+        take(d_in[0], nhp);
+        take(d_in[1], nhp);
+        take(d_inv, nhp);
+        take(d_skey, nhp);
+        take(d_perm, nhp);
+        take(d_hptr_u, (size_t)m + 1);
+        take(d_hcol_u, nhp);
+        take(d_hval_u, nhp);
+        take(d_hptr_i, (size_t)n + 1);
+        take(d_hrow_i, nhp);
+        take(d_hval_i, nhp);
+        take(d_X, (size_t)(m * f));
+        take(d_G, (size_t)(m * f));
+        take(d_dY, (size_t)(n * f));
+        take(d_part, (size_t)(nchunks * f + 1));
+        take(d_parts, (size_t)(2 * m + 2));
+        char *sort = nullptr;
+        take(sort, radix_sort_scratch_bytes(nh));
+        d_sort = sort;
+        return off;
+    };
+    const size_t need = carve(nullptr);
+    if (need > h->adj.work_bytes) {
+        if (h->adj.d_work) {
+            cudaFree(h->adj.d_work);
+            h->adj.d_work = nullptr;
+            h->adj.work_bytes = 0;
+        }
+        step(cudaMalloc(&h->adj.d_work, need));
+        if (e != cudaSuccess) return failed();
+        h->adj.work_bytes = need;
+    }
+    carve(h->adj.d_work);
+    step(cudaMemsetAsync(h->d_flags, 0, sizeof(int32_t) * 8, st));
+    if (nh > 0) {
+        step(cudaMemcpyAsync(d_in[0], held->row_idxs, sizeof(int32_t) * nh, cudaMemcpyHostToDevice, st));
+        step(cudaMemcpyAsync(d_in[1], held->col_idxs, sizeof(int32_t) * nh, cudaMemcpyHostToDevice, st));
+        step(cudaMemcpyAsync(d_inv, held->vals, sizeof(float) * nh, cudaMemcpyHostToDevice, st));
+        step(count_bad_entries(nh, d_in[0], (int32_t)m, d_inv, h->d_flags + 4, st));
+        step(count_bad_entries(nh, d_in[1], (int32_t)n, nullptr, h->d_flags + 4, st));
+        int32_t bad = 0;
+        step(cudaMemcpyAsync(&bad, h->d_flags + 4, sizeof(bad), cudaMemcpyDeviceToHost, st));
+        step(cudaStreamSynchronize(st));
+        if (e != cudaSuccess) return failed();
+        if (bad) return bad_heldout(h, held);
+    }
+    step(group_held(m, nh, d_in[0], d_in[1], d_inv, d_skey, d_perm, d_sort, d_hptr_u, d_hcol_u,
+                    d_hval_u, st));
+    step(group_held(n, nh, d_in[1], d_in[0], d_inv, d_skey, d_perm, d_sort, d_hptr_i, d_hrow_i,
+                    d_hval_i, st));
     if (e == cudaSuccess) {
-        step(cudaMemcpyAsync(d_hptr_u, hptr_u.data(), sizeof(int32_t) * (m + 1), cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_hcol_u, hcol_u.data(), sizeof(int32_t) * nhp, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_hval_u, hval_u.data(), sizeof(float) * nhp, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_hptr_i, hptr_i.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_hrow_i, hrow_i.data(), sizeof(int32_t) * nhp, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_hval_i, hval_i.data(), sizeof(float) * nhp, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_chunks, citem.data(), sizeof(int32_t) * nchunks, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_chunks + nchunks, cbeg.data(), sizeof(int32_t) * nchunks, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_chunks + 2 * nchunks, cend.data(), sizeof(int32_t) * nchunks, cudaMemcpyHostToDevice, st));
-        step(cudaMemcpyAsync(d_chunks + 3 * nchunks, cfirst.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice, st));
-        step(cudaMemsetAsync(h->d_flags, 0, sizeof(int32_t) * 4, st));
         AdjArgs<T> a{};
         a.ptr = h->d_csr_ptr;
         a.idx = h->d_csr_idx;
@@ -597,16 +711,23 @@ als_status adjoint_impl(als_handle *h, const als_coo_view *held, const T *d_Y, T
         step(cudaGetLastError());
         const size_t ismem = sizeof(T) * ITEM_WARPS * (size_t)f;
         if (e == cudaSuccess && n > 0) {
-            adjoint_chunk_kernel<T><<<(unsigned)std::min<int64_t>(nchunks, 152 * 8),
-                                      32 * ITEM_WARPS, ismem, st>>>(
-                nchunks, f, d_chunks, d_chunks + nchunks, d_chunks + 2 * nchunks, h->d_csc_idx,
-                h->d_csc_val, d_hptr_i, d_hrow_i, d_hval_i, d_Y, d_X, d_G, d_part);
+            auto items = [&](auto kernel) {
+                kernel<<<(unsigned)std::min<int64_t>(nchunks, 152 * 8), 32 * ITEM_WARPS, ismem, st>>>(
+                    nchunks, f, d_chunks, d_chunks + nchunks, d_chunks + 2 * nchunks, h->d_csc_idx,
+                    h->d_csc_val, d_hptr_i, d_hrow_i, d_hval_i, d_Y, d_X, d_G, d_part);
+            };
+            switch ((f + 31) / 32) {
+            case 1: items(adjoint_chunk_kernel<T, 1>); break;
+            case 2: items(adjoint_chunk_kernel<T, 2>); break;
+            case 3: items(adjoint_chunk_kernel<T, 3>); break;
+            case 4: items(adjoint_chunk_kernel<T, 4>); break;
+            default: items(adjoint_chunk_kernel<T, (MAX_FP + 31) / 32>); break;
+            }
             adjoint_combine_kernel<T><<<(unsigned)std::min<int64_t>((n * f + 255) / 256, 152 * 16),
                                         256, 0, st>>>(n, f, d_chunks + 3 * nchunks, d_part, d_dY);
         }
         step(cudaGetLastError());
-        sum_doubles_kernel<<<1, 256, 0, st>>>(d_parts, m, d_parts + 2 * m);
-        sum_doubles_kernel<<<1, 256, 0, st>>>(d_parts + m, m, d_parts + 2 * m + 1);
+        sum_doubles_kernel<<<2, 256, 0, st>>>(d_parts, m, d_parts + 2 * m);
         double out[2] = {0.0, 0.0};
         step(cudaMemcpyAsync(out, d_parts + 2 * m, sizeof(out), cudaMemcpyDeviceToHost, st));
         if (dLdY) {
@@ -620,15 +741,7 @@ als_status adjoint_impl(als_handle *h, const als_coo_view *held, const T *d_Y, T
         if (loss) *loss = out[0];
         if (dLdlambda) *dLdlambda = out[1];
     }
-    void *all[] = {d_hptr_u, d_hcol_u, d_hval_u, d_hptr_i, d_hrow_i, d_hval_i, d_X, d_G, d_dY,
-                   d_parts, d_chunks, d_part};
-    for (void *p : all)
-        if (p) cudaFree(p);
-    if (e != cudaSuccess) {
-        h->last_error = std::string("adjoint: ") + cudaGetErrorString(e);
-        return set_global_error(e == cudaErrorMemoryAllocation ? ALS_ERR_OUT_OF_MEMORY : ALS_ERR_CUDA,
-                                h->last_error);
-    }
+    if (e != cudaSuccess) return failed();
     int32_t flags[4] = {0, 0, 0, 0};
     if (cudaMemcpy(flags, h->d_flags, sizeof(flags), cudaMemcpyDeviceToHost) == cudaSuccess)
         h->counters[1] = flags[0];
@@ -639,12 +752,6 @@ als_status check_heldout(const als_handle *h, const als_coo_view *held) {
     if (held->rows != h->m || held->cols != h->n || held->nnz < 0 || held->nnz > INT32_MAX ||
         (held->nnz > 0 && (!held->row_idxs || !held->col_idxs || !held->vals)))
         return set_global_error(ALS_ERR_INVALID_ARG, "held-out COO shape differs from the model");
-    for (int64_t e = 0; e < held->nnz; ++e) {
-        const int32_t r = held->row_idxs[e], c = held->col_idxs[e];
-        if (r < 0 || r >= h->m || c < 0 || c >= h->n || !std::isfinite(held->vals[e]))
-            return set_global_error(ALS_ERR_INVALID_ARG, "held-out entry out of range at " +
-                                                             std::to_string(e));
-    }
     return ALS_OK;
 }
 
@@ -652,6 +759,18 @@ als_status check_heldout(const als_handle *h, const als_coo_view *held) {
 }  // namespace als
 
 using namespace als;
+
+void release_adjoint(als_handle *h, bool workspace) {
+    als_handle::Adjoint &ad = h->adj;
+    if (ad.d_chunks) cudaFree(ad.d_chunks);
+    ad.d_chunks = nullptr;
+    ad.built = false;
+    if (workspace && ad.d_work) {
+        cudaFree(ad.d_work);
+        ad.d_work = nullptr;
+        ad.work_bytes = 0;
+    }
+}
 
 als_status run_adjoint(als_handle *h, const als_coo_view *held, double *loss, float *dLdY,
                        double *dLdlambda) {
@@ -666,6 +785,8 @@ als_status run_adjoint_f64(als_handle *h, const als_coo_view *held, const double
                            double lambda, double *loss, double *dLdY, double *dLdlambda) {
     als_status s = check_heldout(h, held);
     if (s != ALS_OK) return s;
+    // (before the handle's V is overwritten; the FP32 form checks on the device)
+    if (first_bad_heldout(h, held) < held->nnz) return bad_heldout(h, held);
     if (!Y) return set_global_error(ALS_ERR_INVALID_ARG, "null item factors");
     if (h->f > MAX_F_F64)
         return set_global_error(ALS_ERR_UNSUPPORTED, "the FP64 adjoint supports f <= 128");

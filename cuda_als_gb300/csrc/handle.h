@@ -83,6 +83,16 @@ struct als_handle {
         float *d_part = nullptr;
     } split[2];
 
+    // adjoint: chunk table of the item side (built from the ratings, dropped when they change) and
+    // device workspace (grown to the largest call, kept until als_destroy)
+    struct Adjoint {
+        bool built = false;
+        int64_t nchunks = 0;
+        int32_t *d_chunks = nullptr;  // item, first and last rating per chunk; first chunk per item
+        char *d_work = nullptr;
+        size_t work_bytes = 0;
+    } adj;
+
     // event log attached by als_set_log (not owned): training lines, per-iteration test RMSE
     als_log *log = nullptr;
     bool log_iter_rmse = false, log_cout = false;
@@ -102,6 +112,7 @@ void reset_tuning(als_handle *h);
 als_status read_stage_ms(als_handle *h, int side);
 als_status check_sweep_flags(als_handle *h);
 bool tc_supported(int f);
+void release_adjoint(als_handle *h, bool workspace);  // adjoint.cu
 
 // eventlog.cpp
 namespace als {

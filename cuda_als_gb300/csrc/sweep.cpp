@@ -47,6 +47,7 @@ void release_split(als_handle *h);
 
 void release_precision_path(als_handle *h) {
     release_split(h);
+    release_adjoint(h, true);
     for (int s = 0; s < 2; ++s)
         for (int k = 0; k < 2; ++k)
             if (h->ev_half[s][k]) cudaEventDestroy(h->ev_half[s][k]);
@@ -144,6 +145,7 @@ void data_changed(als_handle *h) {
     invalidate_graphs(h);
     for (auto &pl : h->plan) pl.clear();
     release_split(h);
+    release_adjoint(h, false);
 }
 
 // Forget the autotuner's decisions (als_init_factors with autotune = 1).
