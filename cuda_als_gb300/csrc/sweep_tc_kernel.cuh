@@ -243,8 +243,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
                  : "memory");
 }
 // A try suspends the thread until the phase completes (the hardware wakes it then) or
-// MBAR_SUSPEND_NS pass, so a waiting warp takes no issue slots from the warps that work.
-constexpr uint32_t MBAR_SUSPEND_NS = 20000;
+// MBAR_SUSPEND_NS pass, so a waiting warp takes next to no issue slots from the warps that work
+// (1 us and 20 us time the same; at 20 us a whole small half-sweep ends within the 16 tries below,
+// and no limit, however short, is ever checked).
+constexpr uint32_t MBAR_SUSPEND_NS = 1000;
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -255,7 +257,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait (`limit` ns, checked every 16 failed tries, i.e. within ~0.3 ms); false on
+// Bounded wait (`limit` ns, checked every 16 failed tries, i.e. within ~20 us); false on
 // timeout or (when abort != nullptr) once another role aborted.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort,
                                           unsigned long long limit) {
