@@ -957,7 +957,9 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                                 launch_regs_of(SOLVER, FP) * nthreads_of(SOLVER, FP) <= 65536),
                   "register split");
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    // (aligned by an offset, not through an integer: the pointer stays known as shared memory, and
+    // the solvers' accesses are LDS / STS instead of generic loads and stores)
+    uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t *ring = smem;
     float *gscratch = (float *)(ring + NSTAGE * SBYTES);
     float *dsc = gscratch + GroupLayout<FP, SOLVER>::floats * NEPI;  // [MAXF] FP8 scales
