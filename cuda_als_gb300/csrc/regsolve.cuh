@@ -11,10 +11,11 @@
 //   cg_quad       the same CG with four rows shared by a lane quad (half of them in shared
 //                 memory): a quarter of the p reads, for rows too long to keep in registers.
 //   chol_fac      Cholesky A = L L^T of the Gram copied to a packed lower triangle in shared
-//                 memory, left-looking in blocks of 8 columns: the dot products are spread over
-//                 all 128 threads as (row, column-half) items, one thread factors and inverts
-//                 each 8 x 8 diagonal block in registers, three barriers per block.
-//   chol_solve_group  L y = b and L^T x = y by the group, one barrier per 8-row block.
+//                 memory, left-looking in blocks of 8 columns, with the forward solve beside it:
+//                 the dot products are spread over the threads as (row, column half) items,
+//                 one thread factors each 8 x 8 diagonal block in registers and eight lanes invert
+//                 it, three barriers per block.
+//   chol_forward, chol_backward  L y = b and L^T x = y by the group, one barrier per 16 rows.
 // Sums over threads are combined in a fixed order (deterministic).
 #pragma once
 
@@ -201,34 +202,42 @@ struct TriLayout {
 };
 
 // Cholesky A = L L^T of the padded FP x FP matrix held in Ls (packed, tri_off rows; entry (i, j)
-// for j <= i must be set, the rest of each row's blocks is scratch).  On exit entry (i, j <= i)
-// holds L[i][j], Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for r >= c (the inverse of each 8 x 8
-// diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128 threads of a group (et = 0..127);
-// thread `lead` factors the diagonal blocks.
+// for j <= i must be set, the rest of each row's blocks is scratch), and the forward solve L y = b
+// beside it: `bv` holds b on entry (FP floats, scratch afterwards), `yv` receives y.  On exit entry
+// (i, j <= i) holds L[i][j], Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for r >= c (the inverse of each
+// 8 x 8 diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128 threads of a group (et =
+// 0..127); warp `lead` / 32 works on the diagonal blocks.
 //
 // Left-looking in blocks of 8 columns, three barriers per block:
-//  (a) every (row r >= k0, half h) pair subtracts L[r][0:k0] . L[k0+4h+kk][0:k0], kk < 4, from
-//      its 4 entries: work spread evenly over the 128 threads whatever the row count left;
-//  (b) one thread (lead) factors the 8 x 8 diagonal block in registers (rsqrt pivots) and
-//      inverts it;
-//  (c) every row below takes its block columns as s L_KK^-T.
+//  (a) the block's entries lose L[r][0:k0] . L[k0+4h+kk][0:k0], a (row, column half) item a thread;
+//  (b) thread `lead` factors the 8 x 8 diagonal block in registers (rsqrt pivots) and eight lanes
+//      of its warp invert it, a column each;
+//  (c) every row below takes its block columns as s L_KK^-T; each thread also forms the block's
+//      y = L_KK^-1 b and folds it into its own row's b.
+// Work is dealt from the lead warp on, so that the groups' few busy warps sit on different
+// schedulers.  Half-sweep over 480,189 rows and 98.6M ratings, ms at f = 64 / 100 / 128: 24.0 / 50.9
+// / 91.5 with separate solves and work dealt from warp 0 (and one buffer less at 128), now 18.0 /
+// 36.1 / 51.8.  Two rows an item: 18.8 / 38.5 / 53.8; (a) for the next block by the warps that idle
+// in (b): 19.1 / 38.2 / 50.5.
 // Returns false (on thread lead) if a pivot was not positive and finite.
 template <int FP>
-__device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, const GroupSync &gs) {
+__device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, float *bv, float *yv,
+                         const GroupSync &gs) {
     constexpr int B = 8;
     bool ok = true;
+    const int ev = (et + 128 - lead) & 127;
 #pragma unroll 1
     for (int K = 0; K < FP / B; ++K) {
         const int k0 = K * B;
         if (k0 > 0) {
             const int nitems = 2 * (FP - k0);
-            for (int t = et; t < nitems; t += 128) {
+            for (int t = ev; t < nitems; t += 128) {
                 const int r = k0 + (t >> 1), c0 = k0 + 4 * (t & 1);
                 float *lr = Ls + tri_off(r);
                 const float *l0 = Ls + tri_off(c0), *l1 = Ls + tri_off(c0 + 1);
                 const float *l2 = Ls + tri_off(c0 + 2), *l3 = Ls + tri_off(c0 + 3);
                 float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll 2
+#pragma unroll 4
                 for (int q = 0; q < k0; q += 4) {
                     const float4 o = *reinterpret_cast<const float4 *>(lr + q);
                     const float4 a0 = *reinterpret_cast<const float4 *>(l0 + q);
@@ -251,175 +260,230 @@ __device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, co
             }
             gs.sync();
         }
-        if (et == lead) {
-            // (b) factor: right-looking inside the block, everything in registers
-            float m[B][B];
+        float *dv = Dv + K * B * B;
+        if (ev < 32) {
+            if (et == lead) {
+                // (b) factor: right-looking inside the block, everything in registers
+                float m[B][B];
 #pragma unroll
-            for (int r = 0; r < B; ++r) {
-                const float *lr = Ls + tri_off(k0 + r) + k0;
-                const float4 x = *reinterpret_cast<const float4 *>(lr);
-                const float4 y = *reinterpret_cast<const float4 *>(lr + 4);
-                m[r][0] = x.x; m[r][1] = x.y; m[r][2] = x.z; m[r][3] = x.w;
-                m[r][4] = y.x; m[r][5] = y.y; m[r][6] = y.z; m[r][7] = y.w;
+                for (int r = 0; r < B; ++r) {
+                    const float *lr = Ls + tri_off(k0 + r) + k0;
+                    const float4 x = *reinterpret_cast<const float4 *>(lr);
+                    const float4 y = *reinterpret_cast<const float4 *>(lr + 4);
+                    m[r][0] = x.x; m[r][1] = x.y; m[r][2] = x.z; m[r][3] = x.w;
+                    m[r][4] = y.x; m[r][5] = y.y; m[r][6] = y.z; m[r][7] = y.w;
+                }
+                float iv[B];
+#pragma unroll
+                for (int k = 0; k < B; ++k) {
+                    const float dk2 = m[k][k];
+                    const bool good = dk2 > 0.f && isfinite(dk2);
+                    ok = ok && good;
+                    const float inv = good ? rsqrtf(dk2) : 1.f;
+                    m[k][k] = good ? dk2 * inv : 1.f;
+                    iv[k] = inv;
+#pragma unroll
+                    for (int r = k + 1; r < B; ++r) m[r][k] *= inv;
+#pragma unroll
+                    for (int r = k + 1; r < B; ++r)
+#pragma unroll
+                        for (int j = k + 1; j <= r; ++j) m[r][j] = fmaf(-m[r][k], m[j][k], m[r][j]);
+                }
+#pragma unroll
+                for (int r = 0; r < B; ++r) {  // L rows (entries right of the diagonal: zero)
+                    float *lr = Ls + tri_off(k0 + r) + k0;
+                    *reinterpret_cast<float4 *>(lr) =
+                        make_float4(m[r][0], r >= 1 ? m[r][1] : 0.f, r >= 2 ? m[r][2] : 0.f,
+                                    r >= 3 ? m[r][3] : 0.f);
+                    *reinterpret_cast<float4 *>(lr + 4) =
+                        make_float4(r >= 4 ? m[r][4] : 0.f, r >= 5 ? m[r][5] : 0.f,
+                                    r >= 6 ? m[r][6] : 0.f, r >= 7 ? m[r][7] : 0.f);
+                }
+                *reinterpret_cast<float4 *>(invd + k0) = make_float4(iv[0], iv[1], iv[2], iv[3]);
+                *reinterpret_cast<float4 *>(invd + k0 + 4) = make_float4(iv[4], iv[5], iv[6], iv[7]);
             }
-            float iv[B];
+            __syncwarp();
+            const int c = et & 31;
+            if (c < B) {
+                // inverse, lane c its column: D[c][c] = 1 / L_cc,
+                // D[r][c] = -(sum_{c <= t < r} L[r][t] D[t][c]) / L[r][r]
+                float iv[B], d[B];
+                const float4 i0 = *reinterpret_cast<const float4 *>(invd + k0);
+                const float4 i1 = *reinterpret_cast<const float4 *>(invd + k0 + 4);
+                iv[0] = i0.x; iv[1] = i0.y; iv[2] = i0.z; iv[3] = i0.w;
+                iv[4] = i1.x; iv[5] = i1.y; iv[6] = i1.z; iv[7] = i1.w;
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const float dk2 = m[k][k];
-                const bool good = dk2 > 0.f && isfinite(dk2);
-                ok = ok && good;
-                const float inv = good ? rsqrtf(dk2) : 1.f;
-                m[k][k] = good ? dk2 * inv : 1.f;
-                iv[k] = inv;
+                for (int r = 0; r < B; ++r) {
+                    const float *lr = Ls + tri_off(k0 + r) + k0;
+                    const float4 x = *reinterpret_cast<const float4 *>(lr);
+                    const float4 y = *reinterpret_cast<const float4 *>(lr + 4);
+                    const float m[B] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+                    float acc = 0.f;
 #pragma unroll
-                for (int r = k + 1; r < B; ++r) m[r][k] *= inv;
-#pragma unroll
-                for (int r = k + 1; r < B; ++r)
-#pragma unroll
-                    for (int j = k + 1; j <= r; ++j) m[r][j] = fmaf(-m[r][k], m[j][k], m[r][j]);
-            }
-#pragma unroll
-            for (int r = 0; r < B; ++r) {  // L rows (entries right of the diagonal: zero)
-                float *lr = Ls + tri_off(k0 + r) + k0;
-                *reinterpret_cast<float4 *>(lr) = make_float4(
-                    m[r][0], r >= 1 ? m[r][1] : 0.f, r >= 2 ? m[r][2] : 0.f, r >= 3 ? m[r][3] : 0.f);
-                *reinterpret_cast<float4 *>(lr + 4) =
-                    make_float4(r >= 4 ? m[r][4] : 0.f, r >= 5 ? m[r][5] : 0.f,
-                                r >= 6 ? m[r][6] : 0.f, r >= 7 ? m[r][7] : 0.f);
-            }
-            *reinterpret_cast<float4 *>(invd + k0) = make_float4(iv[0], iv[1], iv[2], iv[3]);
-            *reinterpret_cast<float4 *>(invd + k0 + 4) = make_float4(iv[4], iv[5], iv[6], iv[7]);
-            // inverse, one column at a time: D[c][c] = 1 / L_cc,
-            // D[r][c] = -(sum_{c <= t < r} L[r][t] D[t][c]) / L[r][r]
-            float *dv = Dv + K * B * B;
-#pragma unroll
-            for (int c = 0; c < B; ++c) {
-                float d[B];
-#pragma unroll
-                for (int r = c; r < B; ++r) {
-                    if (r == c) {
-                        d[r] = iv[c];
-                    } else {
-                        float acc = 0.f;
-#pragma unroll
-                        for (int t = c; t < r; ++t) acc = fmaf(m[r][t], d[t], acc);
-                        d[r] = -acc * iv[r];
-                    }
-                    dv[r * B + c] = d[r];
+                    for (int t = 0; t < r; ++t) acc = fmaf(m[t], d[t], acc);  // (d[t < c] is zero)
+                    d[r] = r < c ? 0.f : r == c ? iv[r] : -acc * iv[r];
+                    if (r >= c) dv[r * B + c] = d[r];
                 }
             }
         }
         gs.sync();
-        // (c) rows below the block
-        const float *dv = Dv + K * B * B;
-        for (int t = et; t < FP - k0 - B; t += 128) {
-            float *lr = Ls + tri_off(k0 + B + t) + k0;
-            const float4 x = *reinterpret_cast<const float4 *>(lr);
-            const float4 y = *reinterpret_cast<const float4 *>(lr + 4);
-            const float sb[B] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-            float o[B];
+        // (c) rows below the block; b's block by every thread, the first keeps it
+        const int row = k0 + B + ev;
+        if (row < FP || ev == 0) {
+            float rb[B], y[B], sb[B], o[B];
+            const float4 b0 = *reinterpret_cast<const float4 *>(bv + k0);
+            const float4 b1 = *reinterpret_cast<const float4 *>(bv + k0 + 4);
+            rb[0] = b0.x; rb[1] = b0.y; rb[2] = b0.z; rb[3] = b0.w;
+            rb[4] = b1.x; rb[5] = b1.y; rb[6] = b1.z; rb[7] = b1.w;
+            float *lr = Ls + tri_off(row < FP ? row : k0) + k0;
+            const float4 x0 = *reinterpret_cast<const float4 *>(lr);
+            const float4 x1 = *reinterpret_cast<const float4 *>(lr + 4);
+            sb[0] = x0.x; sb[1] = x0.y; sb[2] = x0.z; sb[3] = x0.w;
+            sb[4] = x1.x; sb[5] = x1.y; sb[6] = x1.z; sb[7] = x1.w;
 #pragma unroll
             for (int kk = 0; kk < B; ++kk) {
-                float acc = 0.f;
+                float acc = 0.f, accy = 0.f;
 #pragma unroll
-                for (int q = 0; q <= kk; ++q) acc = fmaf(sb[q], dv[kk * B + q], acc);
+                for (int q = 0; q <= kk; ++q) {
+                    const float dq = dv[kk * B + q];
+                    acc = fmaf(sb[q], dq, acc);
+                    accy = fmaf(dq, rb[q], accy);
+                }
                 o[kk] = acc;
+                y[kk] = accy;
             }
-            *reinterpret_cast<float4 *>(lr) = make_float4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<float4 *>(lr + 4) = make_float4(o[4], o[5], o[6], o[7]);
+            if (row < FP) {
+                *reinterpret_cast<float4 *>(lr) = make_float4(o[0], o[1], o[2], o[3]);
+                *reinterpret_cast<float4 *>(lr + 4) = make_float4(o[4], o[5], o[6], o[7]);
+                float t = bv[row];
+#pragma unroll
+                for (int q = 0; q < B; ++q) t = fmaf(-o[q], y[q], t);
+                bv[row] = t;
+            }
+            if (ev == 0) {
+                *reinterpret_cast<float4 *>(yv + k0) = make_float4(y[0], y[1], y[2], y[3]);
+                *reinterpret_cast<float4 *>(yv + k0 + 4) = make_float4(y[4], y[5], y[6], y[7]);
+            }
         }
         gs.sync();
     }
     return ok;
 }
 
-// x = (L L^T)^-1 v for the factor left by chol_fac, by the whole group: thread t keeps the
-// running value of row t.  Per 8-row block (forward, then backward from the bottom) the warp that
-// owns the block's rows forms its 8 results with the block's inverse (lane l0 + c computes result
-// c from shuffles of the block rows' running values) and publishes them in `xb`; after one barrier
-// every thread folds them into its own row: forward L[t][k0..k0+7] . y, backward
-// L[k0..k0+7][t] . x.  Each row sees the same FMA sequence as in a one-warp solve.  Blocks use the
-// two 8-float halves of `xb` in turn (the backward sweep starting on the half the forward sweep did
-// not end on), so a block's writer never overwrites values a thread has yet to read.  v (FP floats
-// of shared memory) holds b on entry and x on exit, each thread reading and writing its own row.
+// The triangular solves by the whole group: thread t keeps the running value of row t.  Blocks of
+// 16 rows, one barrier each: the warp that owns the rows solves the block's two 8-row halves with
+// their inverses (lane l0 + c computes result c from shuffles of the rows' running values), folds
+// the first half into its own later rows in between, and publishes the 16 results in `xb`; after
+// the barrier every other row folds them into its own.  Each row sees the same FMA sequence as in
+// a one-warp solve.  Blocks use the two 16-float halves of `xb` in turn, so a block's writer never
+// overwrites values a thread has yet to read, from one solve to the next either.
+__device__ __forceinline__ void fold8(const float *l, int stride, const float (&y)[8], float &t) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t = fmaf(-l[q * stride], y[q], t);
+}
+__device__ __forceinline__ void read8(const float *p, float (&y)[8]) {
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
+    y[4] = b.x; y[5] = b.y; y[6] = b.z; y[7] = b.w;
+}
+// `acc` <- the row's y with L y = acc (et >= FP: no row).
 template <int FP>
-__device__ void chol_solve_group(int et, const float *Ls, const float *Dv, float *v, float *xb,
-                                 const GroupSync &gs) {
-    constexpr int B = 8;
-    constexpr int NB = FP / B;
+__device__ __forceinline__ void chol_forward(int et, const float *Ls, const float *Dv, float *xb,
+                                             float &acc, const GroupSync &gs) {
     const int lane = et & 31, w = et >> 5;
     const bool live = et < FP;
-    float acc = live ? v[et] : 0.f;
-    // forward: L y = b
+    const float *own = Ls + tri_off(live ? et : 0);
 #pragma unroll 1
-    for (int K = 0; K < NB; ++K) {
-        const int k0 = K * B;
-        float *yb = xb + (K & 1) * B;
-        if (w == (k0 >> 5)) {  // warp-uniform: the warp holding rows k0..k0+7
-            const int l0 = k0 & 31, c = lane - l0;
-            float r[B];
+    for (int b = 0; b < FP / 16; ++b) {
+        const int k0 = 16 * b;
+        float *xk = xb + (b & 1) * 16;
+        float y[8], l[8];
+        if (w == (k0 >> 5)) {  // warp-uniform: the warp holding rows k0..k0+15
 #pragma unroll
-            for (int q = 0; q < B; ++q) r[q] = __shfl_sync(0xffffffffu, acc, l0 + q);
-            if (c >= 0 && c < B) {
-                const float *dr = Dv + K * B * B + c * B;  // row c of the block's inverse, q <= c
-                float y = 0.f;
+            for (int h = 0; h < 2; ++h) {
+                const int l0 = (k0 & 31) + 8 * h, c = lane - l0;
+                float r[8];
 #pragma unroll
-                for (int q = 0; q < B; ++q)
-                    if (q <= c) y = fmaf(dr[q], r[q], y);
-                acc = y;
-                yb[c] = y;
+                for (int q = 0; q < 8; ++q) r[q] = __shfl_sync(0xffffffffu, acc, l0 + q);
+                if (c >= 0 && c < 8) {
+                    const float *dr = Dv + (2 * b + h) * 64 + c * 8;  // row c of the inverse, q <= c
+                    float v = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (q <= c) v = fmaf(dr[q], r[q], v);
+                    acc = v;
+                    xk[8 * h + c] = v;
+                }
+                if (h == 0) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) y[q] = __shfl_sync(0xffffffffu, acc, l0 + q);
+                    if (live && et >= k0 + 8) {
+                        read8(own + k0, l);
+                        fold8(l, 1, y, acc);
+                    }
+                }
             }
         }
         gs.sync();
-        if (live && et >= k0 + B) {
-            const float4 a0 = *reinterpret_cast<const float4 *>(Ls + tri_off(et) + k0);
-            const float4 a1 = *reinterpret_cast<const float4 *>(Ls + tri_off(et) + k0 + 4);
-            const float4 y0 = *reinterpret_cast<const float4 *>(yb);
-            const float4 y1 = *reinterpret_cast<const float4 *>(yb + 4);
-            float t = acc;
-            t = fmaf(-a0.x, y0.x, t);
-            t = fmaf(-a0.y, y0.y, t);
-            t = fmaf(-a0.z, y0.z, t);
-            t = fmaf(-a0.w, y0.w, t);
-            t = fmaf(-a1.x, y1.x, t);
-            t = fmaf(-a1.y, y1.y, t);
-            t = fmaf(-a1.z, y1.z, t);
-            t = fmaf(-a1.w, y1.w, t);
-            acc = t;
+        if (live && et >= k0 + 16) {
+            if (w != (k0 >> 5)) {
+                read8(xk, y);
+                read8(own + k0, l);
+                fold8(l, 1, y, acc);
+            }
+            read8(xk + 8, y);
+            read8(own + k0 + 8, l);
+            fold8(l, 1, y, acc);
         }
     }
-    // backward: L^T x = y, blocks from the bottom
+}
+// `acc` <- the row's x with L^T x = acc.
+template <int FP>
+__device__ __forceinline__ void chol_backward(int et, const float *Ls, const float *Dv, float *xb,
+                                              float &acc, const GroupSync &gs) {
+    const int lane = et & 31, w = et >> 5;
+    auto fold = [&](int r0, const float (&x)[8]) {  // the results of rows r0..r0+7
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc = fmaf(-Ls[tri_off(r0 + q) + et], x[q], acc);
+    };
 #pragma unroll 1
-    for (int K = NB - 1; K >= 0; --K) {
-        const int k0 = K * B;
-        float *xk = xb + ((K + 1) & 1) * B;
+    for (int b = FP / 16 - 1; b >= 0; --b) {
+        const int k0 = 16 * b;
+        float *xk = xb + ((b + 1) & 1) * 16;
+        float x[8];
         if (w == (k0 >> 5)) {
-            const int l0 = k0 & 31, c = lane - l0;
-            float r[B];
 #pragma unroll
-            for (int q = 0; q < B; ++q) r[q] = __shfl_sync(0xffffffffu, acc, l0 + q);
-            if (c >= 0 && c < B) {
-                const float *dc = Dv + K * B * B + c;  // column c of the block's inverse, q >= c
-                float x = 0.f;
+            for (int h = 1; h >= 0; --h) {
+                const int l0 = (k0 & 31) + 8 * h, c = lane - l0;
+                float r[8];
 #pragma unroll
-                for (int q = 0; q < B; ++q)
-                    if (q >= c) x = fmaf(dc[q * B], r[q], x);
-                acc = x;
-                xk[c] = x;
+                for (int q = 0; q < 8; ++q) r[q] = __shfl_sync(0xffffffffu, acc, l0 + q);
+                if (c >= 0 && c < 8) {
+                    const float *dc = Dv + (2 * b + h) * 64 + c;  // column c of the inverse, q >= c
+                    float v = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (q >= c) v = fmaf(dc[q * 8], r[q], v);
+                    acc = v;
+                    xk[8 * h + c] = v;
+                }
+                if (h == 1) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) x[q] = __shfl_sync(0xffffffffu, acc, l0 + q);
+                    if (et < k0 + 8) fold(k0 + 8, x);
+                }
             }
         }
         gs.sync();
-        if (live && et < k0) {
-            const float4 x0 = *reinterpret_cast<const float4 *>(xk);
-            const float4 x1 = *reinterpret_cast<const float4 *>(xk + 4);
-            const float xs[B] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-            float t = acc;
-#pragma unroll
-            for (int kk = 0; kk < B; ++kk) t = fmaf(-Ls[tri_off(k0 + kk) + et], xs[kk], t);
-            acc = t;
+        if (et < k0) {
+            if (w != (k0 >> 5)) {
+                read8(xk + 8, x);
+                fold(k0 + 8, x);
+            }
+            read8(xk, x);
+            fold(k0, x);
         }
     }
-    if (live) v[et] = acc;
 }
 
 }  // namespace als

@@ -76,7 +76,7 @@ __host__ __device__ constexpr int cgtc_tile_floats(int fp) { return (fp / 8) * 6
 // side by side hide each other's latency (f = 32, 98.6M ratings, users: two groups 10.5 ms, four
 // 6.6).  LU keeps whole rows in registers: two groups.
 __host__ __device__ constexpr int nbuf_of(int solver, int fp) {
-    return fp != 128 ? 4 : cg_quad_rows(solver, fp) ? 3 : 2;
+    return fp != 128 ? 4 : cg_quad_rows(solver, fp) || solver == 1 ? 3 : 2;
 }
 __host__ __device__ constexpr int acc_stride_of(int solver, int fp, int ng) {
     return ng + 16 <= 128 ? 128 : nbuf_of(solver, fp) == 3 ? 160 : 256;
@@ -714,12 +714,13 @@ __device__ bool solve_row(const Params &p, const Meta &m, uint32_t tb, int i, in
         if (i < FP) yv[i] = bi;
         if (et == 0) cflag[0] = 0;
         gs.sync();
-        if (!chol_fac<FP>(et, lead_of(g), Ls, Dv, invd, gs)) cflag[0] = 1;
+        if (!chol_fac<FP>(et, lead_of(g), Ls, Dv, invd, yv, sv, gs)) cflag[0] = 1;
         gs.sync();
         good = cflag[0] == 0;
         if (good) {
-            float *xb = vec + 256;  // the triangular solves' per-block results (16 floats)
-            chol_solve_group<FP>(i, Ls, Dv, yv, xb, gs);
+            float *xb = vec + 256;  // the triangular solves' per-block results (32 floats)
+            float acc = i < FP ? sv[i] : 0.f;
+            chol_backward<FP>(i, Ls, Dv, xb, acc, gs);
             if (wg == (g & 3)) {
                 // condition estimate from the Cholesky diagonal: (max L_jj / min L_jj)^2
                 float dmax = 0.f, dmin = 3.0e38f;
@@ -737,7 +738,7 @@ __device__ bool solve_row(const Params &p, const Meta &m, uint32_t tb, int i, in
                     cflag[1] = (dmax / dmin) * (dmax / dmin) > p.cond_threshold ? 1 : 0;
             }
             gs.sync();
-            xi = i < f ? yv[i] : 0.f;
+            xi = i < f ? acc : 0.f;
             const bool wide = cflag[1] != 0;
             for (int s = 0; s < p.refine_steps; ++s) {
                 if (i < FP) sv[i] = xi * di;  // (FP8: sum_j A'_ij d_j x_j, then times d_i)
@@ -749,9 +750,10 @@ __device__ bool solve_row(const Params &p, const Meta &m, uint32_t tb, int i, in
                     ri = (float)((double)bi - ax - (double)reg * (double)xi);
                 else
                     ri = bi - (float)ax - reg * xi;
-                if (i < FP) yv[i] = i < f ? ri : 0.f;  // (the solve reads and writes each
-                chol_solve_group<FP>(i, Ls, Dv, yv, xb, gs);  //  thread's own row)
-                if (i < f) xi += yv[i];
+                acc = i < f ? ri : 0.f;
+                chol_forward<FP>(i, Ls, Dv, xb, acc, gs);
+                chol_backward<FP>(i, Ls, Dv, xb, acc, gs);
+                if (i < f) xi += acc;
             }
             if (wide && et == 0 && p.refine_steps > 0) atomicAdd(&p.flags[1], 1);
         }
