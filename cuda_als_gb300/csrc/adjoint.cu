@@ -532,7 +532,7 @@ cudaError_t group_held(int64_t nkeys, int64_t nh, const int32_t *key, const int3
                        int32_t *ptr, int32_t *oth, float *gval, cudaStream_t st) {
     if (nh > 0) {
         const cudaError_t e = radix_sort_pairs(key, nullptr, skey, perm, nh,
-                                               (int32_t)(nkeys > 0 ? nkeys - 1 : 0), scratch, st);
+                                               key_bits(nkeys), scratch, st);
         if (e != cudaSuccess) return e;
         gather_held_kernel<<<(unsigned)std::min<int64_t>((nh + 255) / 256, 152 * 16), 256, 0, st>>>(
             nh, perm, other, val, oth, gval);
@@ -638,7 +638,7 @@ als_status adjoint_impl(als_handle *h, const als_coo_view *held, const T *d_Y, T
         take(d_part, (size_t)(nchunks * f + 1));
         take(d_parts, (size_t)(2 * m + 2));
         char *sort = nullptr;
-        take(sort, radix_sort_scratch_bytes(nh));
+        take(sort, radix_sort_scratch_bytes(nh, 1));
         d_sort = sort;
         return off;
     };

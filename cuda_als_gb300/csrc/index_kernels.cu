@@ -1,19 +1,20 @@
-// index_kernels.cu — integer work of the sweep, bit-exact: exclusive scan, stable LSD radix sort,
-// stable CSR->CSC transpose and the degree order of rows.
+// index_kernels.cu — integer work of the sweep, bit-exact: stable LSD radix sorts, the stable
+// CSR->CSC transpose and the degree order of rows.
 //
 // The reference transposes offline with scipy (data/netflix/prepare_netflix_data.py:102-109,
 // data/toy_data_2/prepare_toy_data_2.py:195-200: R.tocsr(), R.tocsc()) and loads both layouts
 // from disk (main.cpp:68-71).  Here the CSC is built on the GPU from the CSR: a stable sort of
 // the entries by column index keeps them in row order inside each column, which is exactly the
 // order scipy's csr_tocsc produces.  All of it is HBM-bound integer traffic: coalesced tiles of
-// 4096 keys per CTA, one 256-bin histogram per tile, a device-wide scan of the digit-major
-// histogram matrix, then a stable scatter ranked with warp match-any.
+// 4096 keys per CTA, one 256-bin histogram per tile, a scan of every digit's tile counts, then a
+// stable scatter ranked with warp match-any.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
-#include <utility>
 #include <string>
+#include <utility>
 
 #include "internal.h"
 
@@ -21,254 +22,255 @@ namespace als {
 
 namespace {
 
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;  // 2048
-
 constexpr int RADIX_BITS = 8;
-constexpr int RADIX_BINS = 1 << RADIX_BITS;  // 256 == threads per CTA
-constexpr int RADIX_THREADS = 256;
-constexpr int RADIX_ROUNDS = 16;                                 // keys per lane (histogram)
-constexpr int RADIX_TILE = RADIX_THREADS * RADIX_ROUNDS;          // 4096
-// The scatter is latency-bound (each CTA loads its whole tile, ranks it, then writes it): it
-// runs the same 4,096-key tile with twice the threads and half the keys a lane, so that two
-// CTAs of 16 warps fit an SM within its registers (at 16 keys a lane, 99 registers held it to
-// two CTAs of 8 warps).
+constexpr int RADIX_BINS = 1 << RADIX_BITS;
+constexpr int RADIX_THREADS = 256;  // histogram: a thread a bin
+constexpr int RADIX_ROUNDS = 16;                          // keys a thread (histogram)
+constexpr int RADIX_TILE = RADIX_THREADS * RADIX_ROUNDS;  // 4096
+constexpr int SCAN_THREADS = 512;
+constexpr int SCAN_ITEMS = 8;
+// The scatter is latency-bound (each CTA loads its whole tile, ranks it, then writes it): 512
+// threads of 8 keys each, so that several CTAs of 16 warps fit an SM within its registers.
 constexpr int SCAT_THREADS = 512;
 constexpr int SCAT_WARPS = SCAT_THREADS / 32;                     // 16
 constexpr int SCAT_ROUNDS = RADIX_TILE / SCAT_THREADS;            // 8 keys per lane
 constexpr int SCAT_WARP_SPAN = 32 * SCAT_ROUNDS;                  // 256 contiguous keys / warp
+static_assert(RADIX_TILE == TILE_KEYS, "tiles");
 static_assert(SCAT_THREADS >= RADIX_BINS && RADIX_BINS % 32 == 0, "one thread per digit");
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+inline size_t array_bytes(int64_t n) { return align256(sizeof(int32_t) * (size_t)(n > 0 ? n : 1)); }
+inline int64_t tiles_of(int64_t n) { return ceil_div(n > 0 ? n : 1, RADIX_TILE); }
+inline int passes_of(int bits) { return std::max(1, (bits + RADIX_BITS - 1) / RADIX_BITS); }
 
-// Block-wide exclusive scan of per-thread sums (fixed order); returns this thread's prefix and
-// the block total in *total.
-__device__ int block_exclusive_scan(int v, int *total) {
+// Exclusive scan, in place, of the `len` counts of row blockIdx.x; its total.
+__global__ void __launch_bounds__(SCAN_THREADS)
+scan_rows_kernel(int32_t *__restrict__ counts, int64_t len, int32_t *__restrict__ totals) {
     __shared__ int warp_sums[SCAN_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < SCAN_THREADS / 32 ? warp_sums[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < SCAN_THREADS / 32) warp_sums[lane] = w;  // inclusive
-    }
-    __syncthreads();
-    int warp_prefix = warp > 0 ? warp_sums[warp - 1] : 0;
-    *total = warp_sums[SCAN_THREADS / 32 - 1];
-    __syncthreads();  // warp_sums is reused by the next call
-    return warp_prefix + x - v;
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS)
-scan_reduce_kernel(const int32_t *__restrict__ in, int64_t n, int32_t *__restrict__ bsums) {
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int s = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i)
-        if (base + i < n) s += in[base + i];
-    int total;
-    block_exclusive_scan(s, &total);
-    if (threadIdx.x == 0) bsums[blockIdx.x] = total;
-}
-
-// One CTA scans the block sums in place (exclusive), looping over tiles with a carry.
-__global__ void __launch_bounds__(SCAN_THREADS)
-scan_bsums_kernel(int32_t *__restrict__ bsums, int64_t nb) {
+    int32_t *row = counts + (int64_t)blockIdx.x * len;
     int carry = 0;
-    for (int64_t t0 = 0; t0 < nb; t0 += SCAN_TILE) {
-        int64_t base = t0 + (int64_t)threadIdx.x * SCAN_ITEMS;
+    for (int64_t t0 = 0; t0 < len; t0 += SCAN_THREADS * SCAN_ITEMS) {
+        const int64_t base = t0 + (int64_t)threadIdx.x * SCAN_ITEMS;
         int v[SCAN_ITEMS];
         int s = 0;
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; ++i) {
-            v[i] = base + i < nb ? bsums[base + i] : 0;
+            v[i] = base + i < len ? row[base + i] : 0;
             s += v[i];
         }
-        int total;
-        int pre = block_exclusive_scan(s, &total) + carry;
+        int x = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_sums[warp] = x;
+        __syncthreads();
+        int before = carry;
+        for (int w = 0; w < SCAN_THREADS / 32; ++w) {
+            const int y = warp_sums[w];
+            before += w < warp ? y : 0;
+            carry += y;
+        }
+        int pre = before + x - s;
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; ++i) {
-            if (base + i < nb) bsums[base + i] = pre;
+            if (base + i < len) row[base + i] = pre;
             pre += v[i];
         }
-        carry += total;
+        __syncthreads();  // warp_sums is written again
     }
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS)
-scan_apply_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t n,
-                  const int32_t *__restrict__ bsums, int with_total) {
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int v[SCAN_ITEMS];
-    int s = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        v[i] = base + i < n ? in[base + i] : 0;
-        s += v[i];
-    }
-    int total;
-    int pre = block_exclusive_scan(s, &total) + bsums[blockIdx.x];
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        if (base + i < n) out[base + i] = pre;
-        pre += v[i];
-    }
-    if (with_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == SCAN_THREADS - 1)
-        out[n] = pre;  // last thread's running sum == grand total
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
 // ---- radix sort -----------------------------------------------------------------------------
 
 __global__ void __launch_bounds__(RADIX_THREADS)
-radix_hist_kernel(const int32_t *__restrict__ keys, int64_t n, int shift, int64_t ntiles,
+radix_hist_kernel(const uint32_t *__restrict__ keys, int64_t n, int shift, int64_t ntiles,
                   int32_t *__restrict__ hist) {
     __shared__ int h[RADIX_BINS];
     h[threadIdx.x] = 0;
-    __syncthreads();
-    int64_t base = (int64_t)blockIdx.x * RADIX_TILE;
-#pragma unroll 4
+    const int64_t base = (int64_t)blockIdx.x * RADIX_TILE;
+    const int nvalid = (int)(n - base < RADIX_TILE ? n - base : RADIX_TILE);
+    const uint32_t *k = keys + base;
+    uint32_t d[RADIX_ROUNDS];
+#pragma unroll
     for (int i = 0; i < RADIX_ROUNDS; ++i) {
-        int64_t pos = base + (int64_t)i * RADIX_THREADS + threadIdx.x;
-        if (pos < n) atomicAdd(&h[(keys[pos] >> shift) & (RADIX_BINS - 1)], 1);
+        const int o = i * RADIX_THREADS + threadIdx.x;
+        d[i] = o < nvalid ? k[o] : 0;
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RADIX_ROUNDS; ++i)
+        if (i * RADIX_THREADS + (int)threadIdx.x < nvalid)
+            atomicAdd(&h[(d[i] >> shift) & (RADIX_BINS - 1)], 1);
     __syncthreads();
     hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Payload words moved with the keys: pass 0 reads in[w] at the key's position (or, for word
-// `pos_word`, takes the position itself), later passes read the previous pass's outputs.
-struct Payload {
-    const int32_t *in[3];
-    int32_t *out[3];
-    int pos_word;  // -1: none
+// What a scatter moves.
+//   MOVE_PAIR    words `key` with a value each
+//   MOVE_CSR     a transpose's first pass: the digit is column `key`'s lowest; the word that moves
+//                on is the column's remaining bits above the row's `row_bits`, with a value
+//   MOVE_TRIPLE  words `key` with two values each (`a`, `val`)
+// A null `val` stands for the positions 0 .. n - 1.  Words and `a` are written through `keep`.
+enum { MOVE_PAIR = 0, MOVE_CSR = 1, MOVE_TRIPLE = 2 };
+struct Move {
+    const uint32_t *key, *a, *val;  // a: MOVE_CSR rows, MOVE_TRIPLE the first value
+    uint32_t *key_out, *a_out, *val_out;  // key_out: MOVE_TRIPLE only
+    int shift;                      // the digit's place in the key
+    int row_bits;                   // MOVE_CSR
+    uint32_t high_mask;             // MOVE_CSR: bits of the column past its lowest digit
+    uint32_t keep;
 };
 
 // Stable scatter.  Warp w of tile t owns the contiguous key range [t*4096 + w*256, +256) and
 // walks it in 8 rounds of 32; a key's rank inside its warp is (keys of the same digit in earlier
 // rounds) + (lanes below it with the same digit in this round), found with match.any.  The warp
-// offsets per digit are an exclusive prefix over warps, the tile's digit starts an exclusive
-// scan over digits.  The keys and their W payload words are first placed in shared memory in
-// digit order (the tile sorted by digit), then streamed out: consecutive threads write
-// consecutive addresses of a digit's run, so the global stores coalesce instead of scattering 32
-// ways per instruction.  A key's destination, goff[d] + (warp offset within d) + rank, is the
-// same either way (stable).  Dynamic shared memory: (1 + W) x RADIX_TILE words.
-template <int W>
-__global__ void __launch_bounds__(SCAT_THREADS, 2)
-radix_scatter_kernel(const int32_t *__restrict__ keys_in, int32_t *__restrict__ keys_out,
-                     Payload pl, int64_t n, int shift, int64_t ntiles,
-                     const int32_t *__restrict__ hist_scan) {
-    extern __shared__ int32_t tile_words[];  // skey[RADIX_TILE], then W payload tiles
+// offsets per digit are an exclusive prefix over warps on top of the tile's digit starts (a scan
+// over digits).  The entries are first placed in shared memory in digit order (the tile sorted by
+// digit), then streamed out: consecutive threads write consecutive addresses of a digit's run, so
+// the global stores coalesce instead of scattering 32 ways per instruction.  hist: every digit's
+// tile counts, scanned; totals: every digit's count (its start is scanned here).
+// Shared memory sets the pace (random 8-byte stores, then rows of a digit), so a transpose moves
+// two words a rating where they fit: 98.6M ratings into 17,770 columns 2.41 -> 1.55 ms (three words,
+// sorted column ids kept for the pointers, scans of the whole histogram before).
+template <int MOVE>
+__global__ void __launch_bounds__(SCAT_THREADS, MOVE == MOVE_TRIPLE ? 2 : 3)
+radix_scatter_kernel(const Move mv, int64_t n, int64_t ntiles, const int32_t *__restrict__ hist,
+                     const int32_t *__restrict__ totals) {
+    extern __shared__ uint2 sorted[];  // [RADIX_TILE], then keys (TRIPLE) or digits (CSR)
     __shared__ int wcnt[SCAT_WARPS][RADIX_BINS];
     __shared__ int goff[RADIX_BINS];
-    __shared__ int tstart[RADIX_BINS];
-    __shared__ int wsum[RADIX_BINS / 32];
-    int32_t *skey = tile_words;
-    int32_t *spay = tile_words + RADIX_TILE;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool digit_thread = threadIdx.x < RADIX_BINS;  // whole warps: RADIX_BINS % 32 == 0
-    for (int i = threadIdx.x; i < SCAT_WARPS * RADIX_BINS; i += SCAT_THREADS) (&wcnt[0][0])[i] = 0;
-    if (digit_thread) goff[threadIdx.x] = hist_scan[(int64_t)threadIdx.x * ntiles + blockIdx.x];
-    __syncthreads();
-
+    __shared__ int wsum[2][RADIX_BINS / 32];
+    uint32_t *skey = reinterpret_cast<uint32_t *>(sorted + RADIX_TILE);
+    uint8_t *sdig = reinterpret_cast<uint8_t *>(sorted + RADIX_TILE);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool digit_thread = tid < RADIX_BINS;  // whole warps: RADIX_BINS % 32 == 0
     // tile-local 32-bit offsets (n <= INT32_MAX): one 64-bit base per array
     const int64_t tile0 = (int64_t)blockIdx.x * RADIX_TILE;
     const int nvalid = (int)(n - tile0 < RADIX_TILE ? n - tile0 : RADIX_TILE);
-    const int32_t *kin = keys_in + tile0;
     const int wbase = warp * SCAT_WARP_SPAN;
     const unsigned lt_mask = (1u << lane) - 1u;
-    int32_t key[SCAT_ROUNDS], pay[W][SCAT_ROUNDS];
-    int rank[SCAT_ROUNDS];
+    uint32_t key[SCAT_ROUNDS], x[SCAT_ROUNDS], y[SCAT_ROUNDS];
+    uint32_t at[SCAT_ROUNDS];  // digit << 16 | rank
 #pragma unroll
     for (int q = 0; q < SCAT_ROUNDS; ++q) {
         const int o = wbase + q * 32 + lane;
         const bool valid = o < nvalid;
-        key[q] = valid ? kin[o] : 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-            pay[w][q] = !valid ? 0 : w == pl.pos_word ? (int32_t)(tile0 + o) : pl.in[w][tile0 + o];
+        key[q] = valid ? mv.key[tile0 + o] : 0;
+        x[q] = MOVE == MOVE_PAIR || !valid ? 0 : mv.a[tile0 + o];
+        y[q] = !valid ? 0 : mv.val ? mv.val[tile0 + o] : (uint32_t)(tile0 + o);
     }
+    int first = 0, total = 0;
+    if (digit_thread) {
+        first = hist[(int64_t)tid * ntiles + blockIdx.x];
+        total = totals[tid];
+    }
+    for (int i = tid; i < SCAT_WARPS * RADIX_BINS; i += SCAT_THREADS) (&wcnt[0][0])[i] = 0;
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < SCAT_ROUNDS; ++q) {
         const bool valid = wbase + q * 32 + lane < nvalid;
         // invalid lanes get a private digit so they never match a real one
-        const int d = valid ? ((key[q] >> shift) & (RADIX_BINS - 1)) : (RADIX_BINS + lane);
+        const uint32_t d = valid ? (key[q] >> mv.shift) & (RADIX_BINS - 1) : RADIX_BINS + lane;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const int before = valid ? wcnt[warp][d] : 0;
-        rank[q] = valid ? before + __popc(peers & lt_mask) : -1;
+        at[q] = d << 16 | (uint32_t)(before + __popc(peers & lt_mask));
+        if (MOVE == MOVE_PAIR) x[q] = key[q];
+        if (MOVE == MOVE_CSR) x[q] |= ((key[q] >> RADIX_BITS) & mv.high_mask) << mv.row_bits;
         __syncwarp();
         if (valid && (__ffs(peers) - 1) == lane) wcnt[warp][d] = before + __popc(peers);
         __syncwarp();
     }
     __syncthreads();
-    int cnt = 0, incl = 0;  // keys of digit threadIdx.x in this tile; inclusive scan over digits
+    int cnt = 0, icnt = 0, itot = 0;  // keys of digit tid in this tile; inclusive scans over digits
     if (digit_thread) {
-        for (int w = 0; w < SCAT_WARPS; ++w) {  // exclusive prefix over warps for this digit
-            const int t = wcnt[w][threadIdx.x];
-            wcnt[w][threadIdx.x] = cnt;
-            cnt += t;
-        }
-        incl = cnt;
+#pragma unroll
+        for (int w = 0; w < SCAT_WARPS; ++w) cnt += wcnt[w][tid];
+        icnt = cnt;
+        itot = total;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
+            const int u = __shfl_up_sync(0xffffffffu, icnt, o), v = __shfl_up_sync(0xffffffffu, itot, o);
+            if (lane >= o) {
+                icnt += u;
+                itot += v;
+            }
         }
-        if (lane == 31) wsum[warp] = incl;
+        if (lane == 31) {
+            wsum[0][warp] = icnt;
+            wsum[1][warp] = itot;
+        }
     }
     __syncthreads();
-    if (digit_thread) {  // tstart = exclusive scan of cnt over the 256 digits
-        int add = 0;
-        for (int w = 0; w < warp; ++w) add += wsum[w];
-        const int ts = add + incl - cnt;
-        tstart[threadIdx.x] = ts;
-        goff[threadIdx.x] -= ts;  // a sorted slot j of digit d goes to goff[d] + j
+    if (digit_thread) {
+        int start = icnt - cnt, base = itot - total;
+        for (int w = 0; w < warp; ++w) {
+            start += wsum[0][w];
+            base += wsum[1][w];
+        }
+        goff[tid] = base + first - start;  // a sorted slot j of digit d goes to goff[d] + j
+#pragma unroll
+        for (int w = 0; w < SCAT_WARPS; ++w) {
+            const int t = wcnt[w][tid];
+            wcnt[w][tid] = start;
+            start += t;
+        }
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < SCAT_ROUNDS; ++q) {
-        if (rank[q] < 0) continue;
-        const int d = (key[q] >> shift) & (RADIX_BINS - 1);
-        const int lp = tstart[d] + wcnt[warp][d] + rank[q];
-        skey[lp] = key[q];
-#pragma unroll
-        for (int w = 0; w < W; ++w) spay[w * RADIX_TILE + lp] = pay[w][q];
+        const uint32_t d = at[q] >> 16;
+        if (d >= RADIX_BINS) continue;
+        const int lp = wcnt[warp][d] + (int)(at[q] & 0xffffu);
+        sorted[lp] = make_uint2(x[q], y[q]);
+        if (MOVE == MOVE_TRIPLE) skey[lp] = key[q];
+        if (MOVE == MOVE_CSR) sdig[lp] = (uint8_t)d;
     }
     __syncthreads();
-#pragma unroll 2
-    for (int j = threadIdx.x; j < nvalid; j += SCAT_THREADS) {
-        const int32_t k = skey[j];
-        const int d = (k >> shift) & (RADIX_BINS - 1);
+#pragma unroll 4
+    for (int j = tid; j < nvalid; j += SCAT_THREADS) {
+        const uint2 e = sorted[j];
+        const uint32_t k = MOVE == MOVE_TRIPLE ? skey[j] : MOVE == MOVE_CSR ? sdig[j] : e.x;
+        const uint32_t d = MOVE == MOVE_CSR ? k : (k >> mv.shift) & (RADIX_BINS - 1);
         const int dst = goff[d] + j;
-        keys_out[dst] = k;
-#pragma unroll
-        for (int w = 0; w < W; ++w) pl.out[w][dst] = spay[w * RADIX_TILE + j];
+        if (MOVE == MOVE_TRIPLE) mv.key_out[dst] = k;
+        mv.a_out[dst] = e.x & mv.keep;
+        mv.val_out[dst] = e.y;
     }
 }
 
-// One scatter pass: the launch with its dynamic shared memory ((1 + W) 16 KB tiles; the limit
-// is raised first, as the static counters and the dynamic tiles together pass 48 KB).
-template <int W>
-cudaError_t launch_scatter(const int32_t *keys_in, int32_t *keys_out, const Payload &pl, int64_t n,
-                           int shift, int64_t ntiles, const int32_t *hist, cudaStream_t st) {
-    const size_t dyn = sizeof(int32_t) * (size_t)(1 + W) * RADIX_TILE;
-    cudaError_t e = cudaFuncSetAttribute(radix_scatter_kernel<W>,
+// The counters of a sort of n keys: [RADIX_BINS][tiles] tile counts and the digits' totals, two
+// sets of the latter (a transpose needs those of its first pass after its last).
+struct Counters {
+    int32_t *hist, *totals[2];
+};
+inline size_t counter_bytes(int64_t n) {
+    return align256(sizeof(int32_t) * RADIX_BINS * (size_t)tiles_of(n)) + 2 * sizeof(int32_t) * RADIX_BINS;
+}
+inline Counters counters_at(void *p, int64_t n) {
+    Counters c;
+    c.hist = (int32_t *)p;
+    c.totals[0] = (int32_t *)((char *)p + align256(sizeof(int32_t) * RADIX_BINS * (size_t)tiles_of(n)));
+    c.totals[1] = c.totals[0] + RADIX_BINS;
+    return c;
+}
+
+// One pass: tile histograms, their scans, the scatter.  (The scatter's dynamic shared memory is
+// raised first: static counters and tile together pass 48 KB.)
+template <int MOVE>
+cudaError_t radix_pass(const Move &mv, int64_t n, const Counters &c, int32_t *totals, cudaStream_t st) {
+    const int64_t ntiles = tiles_of(n);
+    const size_t dyn = RADIX_TILE * (sizeof(uint2) + (MOVE == MOVE_TRIPLE ? sizeof(uint32_t) : MOVE == MOVE_CSR ? 1 : 0));
+    cudaError_t e = cudaFuncSetAttribute(radix_scatter_kernel<MOVE>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
-    radix_scatter_kernel<W><<<(unsigned)ntiles, SCAT_THREADS, dyn, st>>>(keys_in, keys_out, pl, n,
-                                                                       shift, ntiles, hist);
+    radix_hist_kernel<<<(unsigned)ntiles, RADIX_THREADS, 0, st>>>(mv.key, n, mv.shift, ntiles, c.hist);
+    scan_rows_kernel<<<RADIX_BINS, SCAN_THREADS, 0, st>>>(c.hist, ntiles, totals);
+    radix_scatter_kernel<MOVE><<<(unsigned)ntiles, SCAT_THREADS, dyn, st>>>(mv, n, ntiles, c.hist, totals);
     return cudaGetLastError();
 }
 
@@ -284,26 +286,6 @@ __global__ void expand_rows_kernel(int64_t rows, int64_t nnz, const int32_t *__r
     }
 }
 
-// (row, value) of each CSR position side by side, so the permutation gather below reads one
-// 8-byte pair (one sector) per rating instead of two 4-byte values from two arrays.
-__global__ void pack_rows_vals_kernel(int64_t nnz, const int32_t *__restrict__ coo_rows,
-                                      const float *__restrict__ val, int2 *__restrict__ pk) {
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
-         p += (int64_t)gridDim.x * blockDim.x)
-        pk[p] = make_int2(coo_rows[p], __float_as_int(val[p]));
-}
-
-__global__ void gather_csc_kernel(int64_t nnz, const int32_t *__restrict__ perm,
-                                  const int2 *__restrict__ pk, int32_t *__restrict__ ridx,
-                                  float *__restrict__ cval) {
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int2 v = pk[perm[p]];
-        ridx[p] = v.x;
-        cval[p] = __int_as_float(v.y);
-    }
-}
-
 // col_ptrs[c] = first position whose sorted key >= c (lower bound), written without atomics.
 __global__ void col_ptrs_from_sorted_kernel(int64_t nnz, int64_t cols,
                                             const int32_t *__restrict__ skeys,
@@ -316,6 +298,55 @@ __global__ void col_ptrs_from_sorted_kernel(int64_t nnz, int64_t cols,
         hi = hi > cols ? cols : hi;
         for (int64_t c = lo; c <= hi; ++c) cptr[c] = (int32_t)p;
     }
+}
+
+// Column pointers of a transpose by one or two passes, from its counters (scanned tile counts of
+// the last pass, both passes' totals): with one, a column is a digit.  With two, the entries of
+// columns (d1, d0) start, before the last pass, where those of the lowest digit d0 start
+// (position s); column (d1, d0) starts where the pass sends the first entry of digit d1 at or
+// after s: behind those of d1 in earlier tiles and in s's tile before s.  Block d0, a thread a d1.
+__global__ void __launch_bounds__(RADIX_BINS)
+col_ptrs_kernel(int passes, int64_t nnz, int64_t cols, int64_t ntiles, const uint32_t *__restrict__ words,
+                int shift, const int32_t *__restrict__ hist, const int32_t *__restrict__ first_totals,
+                const int32_t *__restrict__ last_totals, int32_t *__restrict__ cptr) {
+    __shared__ int cnt[RADIX_BINS];
+    __shared__ int wsum[2][RADIX_BINS / 32];
+    __shared__ int start;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t0 = first_totals[tid], t1 = last_totals[tid];
+    int i0 = t0, i1 = t1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, i0, o), v = __shfl_up_sync(0xffffffffu, i1, o);
+        if (lane >= o) {
+            i0 += u;
+            i1 += v;
+        }
+    }
+    if (lane == 31) {
+        wsum[0][warp] = i0;
+        wsum[1][warp] = i1;
+    }
+    cnt[tid] = 0;
+    __syncthreads();
+    int s0 = i0 - t0, s1 = i1 - t1;  // digit tid's start in the first and the last pass
+    for (int w = 0; w < warp; ++w) {
+        s0 += wsum[0][w];
+        s1 += wsum[1][w];
+    }
+    if (blockIdx.x == 0 && tid == 0) cptr[cols] = (int32_t)nnz;
+    if (passes == 1) {
+        if (tid < cols) cptr[tid] = s0;
+        return;
+    }
+    if (tid == (int)blockIdx.x) start = s0;
+    __syncthreads();
+    const int64_t t = start / RADIX_TILE;
+    for (int64_t p = t * RADIX_TILE + tid; p < start; p += RADIX_BINS)
+        atomicAdd(&cnt[(words[p] >> shift) & (RADIX_BINS - 1)], 1);
+    __syncthreads();
+    const int64_t c = ((int64_t)tid << RADIX_BITS) + blockIdx.x;
+    if (c < cols) cptr[c] = s1 + (t < ntiles ? hist[tid * ntiles + t] + cnt[tid] : t1);
 }
 
 __global__ void degree_keys_kernel(int64_t rows, const int32_t *__restrict__ ptr, int32_t maxd,
@@ -347,94 +378,84 @@ int grid_for(int64_t work, int threads, int cap = 152 * 16) {
 
 // ---------------------------------------------------------------------------------------------
 
-size_t scan_scratch_bytes(int64_t n) {
-    return align256(sizeof(int32_t) * (size_t)(ceil_div(n > 0 ? n : 1, SCAN_TILE) + 1));
-}
+size_t tile_counts_bytes(int64_t n) { return array_bytes(tiles_of(n)); }
 
-cudaError_t exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n, bool with_total,
-                               void *scratch, cudaStream_t st) {
-    if (n <= 0) {
-        if (with_total) return cudaMemsetAsync(out, 0, sizeof(int32_t), st);
-        return cudaSuccess;
-    }
-    int64_t nb = ceil_div(n, SCAN_TILE);
-    int32_t *bsums = (int32_t *)scratch;
-    scan_reduce_kernel<<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, n, bsums);
-    scan_bsums_kernel<<<1, SCAN_THREADS, 0, st>>>(bsums, nb);
-    scan_apply_kernel<<<(unsigned)nb, SCAN_THREADS, 0, st>>>(in, out, n, bsums,
-                                                              with_total ? 1 : 0);
+cudaError_t scan_tile_counts(int32_t *counts, int64_t n, int32_t *total, cudaStream_t st) {
+    scan_rows_kernel<<<1, SCAN_THREADS, 0, st>>>(counts, tiles_of(n), total);
     return cudaGetLastError();
 }
 
-static int radix_passes(int32_t max_key) {
-    int bits = 0;
-    while (bits < 31 && (int64_t(1) << bits) <= (int64_t)max_key) ++bits;
-    int p = (bits + RADIX_BITS - 1) / RADIX_BITS;
-    return p < 1 ? 1 : p;
+size_t radix_sort_scratch_bytes(int64_t n, int values) {
+    return (1 + (size_t)values) * array_bytes(n) + counter_bytes(n);
 }
 
-size_t radix_sort_scratch_bytes(int64_t n) {
-    int64_t ntiles = ceil_div(n > 0 ? n : 1, RADIX_TILE);
-    size_t hist = (size_t)RADIX_BINS * (size_t)ntiles;
-    return 4 * align256(sizeof(int32_t) * (size_t)(n > 0 ? n : 1)) +
-           align256(sizeof(int32_t) * hist) + scan_scratch_bytes((int64_t)hist);
-}
-
+// The passes alternate between the scratch set and the outputs, so that the last one lands there.
 cudaError_t radix_sort_pairs(const int32_t *keys_in, const int32_t *vals_in, int32_t *keys_out,
-                             int32_t *vals_out, int64_t n, int32_t max_key, void *scratch,
+                             int32_t *vals_out, int64_t n, int bits, void *scratch,
                              cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const int64_t ntiles = ceil_div(n, RADIX_TILE);
-    const size_t arr = align256(sizeof(int32_t) * (size_t)n);
-    char *s = (char *)scratch;
-    int32_t *bk[2] = {(int32_t *)s, (int32_t *)(s + 2 * arr)};
-    int32_t *bv[2] = {(int32_t *)(s + arr), (int32_t *)(s + 3 * arr)};
-    s += 4 * arr;
-    int32_t *hist = (int32_t *)s;
-    s += align256(sizeof(int32_t) * (size_t)RADIX_BINS * (size_t)ntiles);
-    void *scan_scratch = s;
-
-    const int passes = radix_passes(max_key);
-    const int32_t *src_k = keys_in, *src_v = vals_in;
+    uint32_t *set[2][2] = {{(uint32_t *)keys_out, (uint32_t *)vals_out},
+                           {(uint32_t *)scratch, (uint32_t *)((char *)scratch + array_bytes(n))}};
+    const Counters c = counters_at((char *)scratch + 2 * array_bytes(n), n);
+    const int passes = passes_of(bits);
+    Move mv{};
+    mv.key = (const uint32_t *)keys_in;
+    mv.val = (const uint32_t *)vals_in;
+    mv.keep = ~0u;
     for (int p = 0; p < passes; ++p) {
-        int32_t *dst_k = p == passes - 1 ? keys_out : bk[p & 1];
-        int32_t *dst_v = p == passes - 1 ? vals_out : bv[p & 1];
-        const int shift = p * RADIX_BITS;
-        radix_hist_kernel<<<(unsigned)ntiles, RADIX_THREADS, 0, st>>>(src_k, n, shift, ntiles,
-                                                                       hist);
-        cudaError_t e = exclusive_scan_i32(hist, hist, (int64_t)RADIX_BINS * ntiles, false,
-                                           scan_scratch, st);
+        uint32_t **dst = set[(passes - 1 - p) & 1];
+        mv.a_out = dst[0];
+        mv.val_out = dst[1];
+        mv.shift = p * RADIX_BITS;
+        const cudaError_t e = radix_pass<MOVE_PAIR>(mv, n, c, c.totals[0], st);
         if (e != cudaSuccess) return e;
-        Payload pl{};
-        pl.in[0] = src_v;
-        pl.out[0] = dst_v;
-        pl.pos_word = src_v ? -1 : 0;  // no values given: the positions themselves
-        e = launch_scatter<1>(src_k, dst_k, pl, n, shift, ntiles, hist, st);
-        if (e != cudaSuccess) return e;
-        src_k = dst_k;
-        src_v = dst_v;
+        mv.key = dst[0];
+        mv.val = dst[1];
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
-// Key + payload sets a payload-carrying sort of `cols` column ids passes through: the first pass
-// reads the inputs and the last writes the outputs, so one pass needs none, two passes one (the
-// 17,770 columns of the Netflix shape), more passes two in turn.
-static int transpose_sets(int64_t cols) {
-    const int passes = radix_passes((int32_t)(cols > 0 ? cols - 1 : 0));
-    return passes >= 3 ? 2 : passes - 1;
+cudaError_t radix_sort_triples(const int32_t *keys_in, const int32_t *a_in, const int32_t *b_in,
+                               int32_t *keys_out, int32_t *a_out, int32_t *b_out, int64_t n,
+                               int bits, void *scratch, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    char *s = (char *)scratch;
+    const size_t arr = array_bytes(n);
+    uint32_t *set[2][3] = {{(uint32_t *)keys_out, (uint32_t *)a_out, (uint32_t *)b_out},
+                           {(uint32_t *)s, (uint32_t *)(s + arr), (uint32_t *)(s + 2 * arr)}};
+    const Counters c = counters_at(s + 3 * arr, n);
+    const int passes = passes_of(bits);
+    Move mv{};
+    mv.key = (const uint32_t *)keys_in;
+    mv.a = (const uint32_t *)a_in;
+    mv.val = (const uint32_t *)b_in;
+    mv.keep = ~0u;
+    for (int p = 0; p < passes; ++p) {
+        uint32_t **dst = set[(passes - 1 - p) & 1];
+        mv.key_out = dst[0];
+        mv.a_out = dst[1];
+        mv.val_out = dst[2];
+        mv.shift = p * RADIX_BITS;
+        const cudaError_t e = radix_pass<MOVE_TRIPLE>(mv, n, c, c.totals[0], st);
+        if (e != cudaSuccess) return e;
+        mv.key = dst[0];
+        mv.a = dst[1];
+        mv.val = dst[2];
+    }
+    return cudaSuccess;
 }
 
-size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool compact) {
-    (void)rows;
-    const size_t arr = align256(sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1));
-    if (compact) return 3 * arr + radix_sort_scratch_bytes(nnz);
-    // rows of the CSR, the sorted keys, the ping-pong sets of key + three payload words, the
-    // per-tile digit histogram and its scan
-    const int64_t ntiles = ceil_div(nnz > 0 ? nnz : 1, RADIX_TILE);
-    const size_t hist = (size_t)RADIX_BINS * (size_t)ntiles;
-    return (2 + 4 * (size_t)transpose_sets(cols)) * arr + align256(sizeof(int32_t) * hist) +
-           scan_scratch_bytes((int64_t)hist);
+// Whether one or two passes over packed words transpose the matrix: a word holds the row and what
+// is left of the column after its lowest digit.
+static bool transpose_packs(int64_t rows, int64_t cols) {
+    const int cb = key_bits(cols);
+    return cb <= 2 * RADIX_BITS && key_bits(rows) + std::max(0, cb - RADIX_BITS) <= 32;
+}
+
+// The rows of the CSR, a set of two words a rating and the counters; the general path's set has
+// three, and it sorts the columns themselves.
+size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz) {
+    return (transpose_packs(rows, cols) ? 3 : 5) * array_bytes(nnz) + counter_bytes(nnz);
 }
 
 cudaError_t expand_rows(int64_t rows, int64_t nnz, const int32_t *ptr, int32_t *coo_rows,
@@ -447,76 +468,71 @@ cudaError_t expand_rows(int64_t rows, int64_t nnz, const int32_t *ptr, int32_t *
 cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int32_t *ptr,
                               const int32_t *idx, const float *val, int32_t *cptr,
                               int32_t *ridx, float *cval, void *scratch, cudaStream_t st,
-                              int32_t *coo_rows_out, int32_t *perm_out, bool compact) {
+                              int32_t *coo_rows_out, int32_t *perm_out, bool rows_ready) {
     if (nnz <= 0) return cudaMemsetAsync(cptr, 0, sizeof(int32_t) * (size_t)(cols + 1), st);
-    const size_t arr = align256(sizeof(int32_t) * (size_t)nnz);
+    const size_t arr = array_bytes(nnz);
     char *s = (char *)scratch;
     int32_t *coo_rows = coo_rows_out ? coo_rows_out : (int32_t *)s;
-    int32_t *skeys = (int32_t *)(s + arr);
-    cudaError_t e = expand_rows(rows, nnz, ptr, coo_rows, st);
-    if (e != cudaSuccess) return e;
-    if (compact) {
-        // sort (column, CSR position), then gather the (row, value) pairs by that permutation
-        int32_t *perm = perm_out ? perm_out : (int32_t *)(s + 2 * arr);
-        void *sort_scratch = s + 3 * arr;
-        e = radix_sort_pairs(idx, nullptr, skeys, perm, nnz, (int32_t)(cols > 0 ? cols - 1 : 0),
-                             sort_scratch, st);
+    cudaError_t e = cudaSuccess;
+    if (!rows_ready) {
+        e = expand_rows(rows, nnz, ptr, coo_rows, st);
         if (e != cudaSuccess) return e;
-        // the sort's four n-int buffers are free again: the packed pairs take two of them
-        int2 *pk = reinterpret_cast<int2 *>(sort_scratch);
-        pack_rows_vals_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(nnz, coo_rows, val, pk);
-        gather_csc_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(nnz, perm, pk, ridx, cval);
-    } else {
-        // sort the columns with the rating's row and value (and its CSR position when the caller
-        // keeps the permutation) as payload: the last pass writes the CSC arrays themselves
-        const int nsets = transpose_sets(cols);
-        int32_t *set[2][4] = {};
-        for (int k = 0; k < nsets; ++k)
-            for (int w = 0; w < 4; ++w) set[k][w] = (int32_t *)(s + (2 + 4 * k + w) * arr);
-        const int64_t ntiles = ceil_div(nnz, RADIX_TILE);
-        char *hs = s + (2 + 4 * (size_t)nsets) * arr;
-        int32_t *hist = (int32_t *)hs;
-        void *scan_scratch = hs + align256(sizeof(int32_t) * (size_t)RADIX_BINS * ntiles);
-        const int passes = radix_passes((int32_t)(cols > 0 ? cols - 1 : 0));
-        for (int pass = 0; pass < passes; ++pass) {
-            const bool last = pass == passes - 1;
-            const int32_t *src_k = pass == 0 ? idx : set[(pass - 1) & 1][0];
-            int32_t *dst_k = last ? skeys : set[pass & 1][0];
-            Payload pl{};
-            pl.pos_word = pass == 0 && perm_out ? 2 : -1;
-            for (int w = 0; w < 3; ++w) {
-                pl.in[w] = pass == 0 ? (w == 0 ? coo_rows : w == 1 ? (const int32_t *)val : nullptr)
-                                     : set[(pass - 1) & 1][1 + w];
-                pl.out[w] = last ? (w == 0 ? ridx : w == 1 ? (int32_t *)cval : perm_out)
-                                 : set[pass & 1][1 + w];
-            }
-            radix_hist_kernel<<<(unsigned)ntiles, RADIX_THREADS, 0, st>>>(src_k, nnz, pass * RADIX_BITS,
-                                                                         ntiles, hist);
-            e = exclusive_scan_i32(hist, hist, (int64_t)RADIX_BINS * ntiles, false, scan_scratch, st);
-            if (e != cudaSuccess) return e;
-            e = perm_out ? launch_scatter<3>(src_k, dst_k, pl, nnz, pass * RADIX_BITS, ntiles, hist, st)
-                         : launch_scatter<2>(src_k, dst_k, pl, nnz, pass * RADIX_BITS, ntiles, hist, st);
+    }
+    // the rating moves with its row, or its CSR position where the caller keeps the permutation
+    const uint32_t *v_in = perm_out ? nullptr : (const uint32_t *)val;
+    uint32_t *v_out = (uint32_t *)(perm_out ? perm_out : (int32_t *)cval);
+    const int cb = key_bits(cols), rb = key_bits(rows), passes = passes_of(cb);
+    if (transpose_packs(rows, cols)) {
+        uint32_t *word = (uint32_t *)(s + arr), *pay = (uint32_t *)(s + 2 * arr);
+        const Counters c = counters_at(s + 3 * arr, nnz);
+        const bool one = passes == 1;
+        Move mv{};
+        mv.key = (const uint32_t *)idx;
+        mv.a = (const uint32_t *)coo_rows;
+        mv.val = v_in;
+        mv.a_out = one ? (uint32_t *)ridx : word;
+        mv.val_out = one ? v_out : pay;
+        mv.row_bits = rb;
+        mv.high_mask = one ? 0u : (1u << (cb - RADIX_BITS)) - 1u;
+        mv.keep = ~0u;
+        e = radix_pass<MOVE_CSR>(mv, nnz, c, c.totals[0], st);
+        if (e != cudaSuccess) return e;
+        if (!one) {
+            mv.key = word;
+            mv.val = pay;
+            mv.a_out = (uint32_t *)ridx;
+            mv.val_out = v_out;
+            mv.shift = rb;
+            mv.keep = (1u << rb) - 1u;
+            e = radix_pass<MOVE_PAIR>(mv, nnz, c, c.totals[1], st);
             if (e != cudaSuccess) return e;
         }
+        col_ptrs_kernel<<<one ? 1 : RADIX_BINS, RADIX_BINS, 0, st>>>(
+            passes, nnz, cols, tiles_of(nnz), word, rb, c.hist, c.totals[0], c.totals[one ? 0 : 1], cptr);
+    } else {
+        int32_t *skeys = (int32_t *)(s + arr);
+        e = radix_sort_triples(idx, coo_rows, (const int32_t *)v_in, skeys, ridx, (int32_t *)v_out,
+                               nnz, cb, s + 2 * arr, st);
+        if (e != cudaSuccess) return e;
+        col_ptrs_from_sorted_kernel<<<grid_for(nnz + 1, 256), 256, 0, st>>>(nnz, cols, skeys, cptr);
     }
-    col_ptrs_from_sorted_kernel<<<grid_for(nnz + 1, 256), 256, 0, st>>>(nnz, cols, skeys, cptr);
+    if (perm_out) return gather_f32(nnz, perm_out, val, cval, st);
     return cudaGetLastError();
 }
 
 size_t degree_order_scratch_bytes(int64_t rows) {
-    return 2 * align256(sizeof(int32_t) * (size_t)(rows > 0 ? rows : 1)) +
-           radix_sort_scratch_bytes(rows);
+    return 2 * array_bytes(rows) + radix_sort_scratch_bytes(rows, 1);
 }
 
 cudaError_t degree_order_device(int64_t rows, const int32_t *ptr, int32_t max_degree,
                                 int32_t *perm, void *scratch, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
-    const size_t arr = align256(sizeof(int32_t) * (size_t)rows);
+    const size_t arr = array_bytes(rows);
     char *s = (char *)scratch;
     int32_t *keys = (int32_t *)s;
     int32_t *skeys = (int32_t *)(s + arr);
     degree_keys_kernel<<<grid_for(rows, 256), 256, 0, st>>>(rows, ptr, max_degree, keys);
-    return radix_sort_pairs(keys, nullptr, skeys, perm, rows, max_degree, s + 2 * arr, st);
+    return radix_sort_pairs(keys, nullptr, skeys, perm, rows, key_bits((int64_t)max_degree + 1), s + 2 * arr, st);
 }
 
 __global__ void gather_f32_kernel(int64_t n, const int32_t *__restrict__ perm,
@@ -554,10 +570,10 @@ cudaError_t count_bad_entries(int64_t nnz, const int32_t *idx, int32_t limit, co
 // plug-ins hosted by an engine that owns all device memory and forbids allocations inside its
 // callbacks, and latency-critical loops that must not synchronise on the allocator.  For them the
 // transpose's scratch lives in one file-scope device array of NOALLOC_SCRATCH_BYTES (16 MiB),
-// which every GPU that loads this library holds until the process exits.  The compact transpose
-// needs 28 bytes per rating plus 1 KiB per 4,096 ratings (its radix histograms), each array
-// rounded up to 256 bytes, which admits at most 593,856 ratings; larger inputs are rejected with
-// ALS_ERR_INVALID_ARG before anything runs.
+// which every GPU that loads this library holds until the process exits.  It admits
+// NOALLOC_MAX_RATINGS (28 bytes a rating and 1 KiB of radix histograms per 4,096 ratings, of which
+// the present transpose needs 20 at most); larger inputs are rejected with ALS_ERR_INVALID_ARG
+// before anything runs.
 //
 // In host code the array's name is only a host-side stand-in, so the device address is looked up
 // with cudaGetSymbolAddress (with the device current) on the first call made in each CUDA
@@ -571,6 +587,7 @@ cudaError_t count_bad_entries(int64_t nnz, const int32_t *idx, int32_t limit, co
 namespace {
 
 constexpr size_t NOALLOC_SCRATCH_BYTES = 16u << 20;
+constexpr int64_t NOALLOC_MAX_RATINGS = 593856;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
@@ -616,13 +633,14 @@ extern "C" als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int
     if (csr->rows < 0 || csr->cols < 0 || csr->nnz < 0 || csr->nnz > INT32_MAX ||
         csr->rows >= INT32_MAX || csr->cols >= INT32_MAX)
         return set_global_error(ALS_ERR_INVALID_ARG, "shape out of range");
-    const size_t need = transpose_scratch_bytes(csr->rows, csr->cols, csr->nnz, true);
-    if (need > NOALLOC_SCRATCH_BYTES)
+    if (csr->nnz > NOALLOC_MAX_RATINGS ||
+        transpose_scratch_bytes(csr->rows, csr->cols, csr->nnz) > NOALLOC_SCRATCH_BYTES)
         return set_global_error(
             ALS_ERR_INVALID_ARG,
-            "als_csr_to_csc_device_noalloc: " + std::to_string(csr->nnz) +
-                " ratings need " + std::to_string(need) + " bytes of scratch, more than its fixed " +
-                std::to_string(NOALLOC_SCRATCH_BYTES) + "-byte array; use als_csr_to_csc_device");
+            "als_csr_to_csc_device_noalloc: " + std::to_string(csr->nnz) + " ratings, more than the " +
+                std::to_string(NOALLOC_MAX_RATINGS) + " of its fixed " +
+                std::to_string(NOALLOC_SCRATCH_BYTES) +
+                "-byte scratch array; use als_csr_to_csc_device");
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess)
@@ -649,7 +667,7 @@ extern "C" als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int
     }
     e = csr_to_csc_device(csr->rows, csr->cols, csr->nnz, csr->row_ptrs, csr->col_idxs,
                           csr->vals, col_ptrs, row_idxs, vals, scratch, (cudaStream_t)stream,
-                          nullptr, nullptr, /*compact=*/true);
+                          nullptr, nullptr);
     if (e != cudaSuccess)
         return set_global_error(ALS_ERR_CUDA, std::string("csr_to_csc: ") + cudaGetErrorString(e));
     return ALS_OK;

@@ -26,30 +26,39 @@ als_status set_global_error(als_status s, const std::string &msg);
 // Index kernels (index_kernels.cu)
 // ---------------------------------------------------------------------------------------------
 
-// Bytes of scratch needed by radix_sort_pairs for n keys.
-size_t radix_sort_scratch_bytes(int64_t n);
-// Stable LSD radix sort of (keys, vals) by key, 8-bit digits, keys in [0, max_key].
-// keys_in/vals_in are read (vals_in may be NULL: vals are then the positions 0..n-1);
-// results land in keys_out/vals_out.  `scratch` holds radix_sort_scratch_bytes(n) bytes and
-// two ping-pong arrays are carved from it.
+// Significant bits of the keys 0 .. count - 1.
+inline int key_bits(int64_t count) {
+    int b = 0;
+    while (b < 31 && (int64_t(1) << b) < count) ++b;
+    return b;
+}
+
+// Bytes of scratch needed by a sort of n keys with `values` values each.
+size_t radix_sort_scratch_bytes(int64_t n, int values);
+// Stable LSD radix sorts of keys with one or two values each by the keys' lowest `bits` bits (at
+// most 32; keys are unsigned).  A null last value stands for the positions 0..n-1.  Outputs may
+// not be inputs; `scratch` holds radix_sort_scratch_bytes(n, values) bytes.
 cudaError_t radix_sort_pairs(const int32_t *keys_in, const int32_t *vals_in, int32_t *keys_out,
-                             int32_t *vals_out, int64_t n, int32_t max_key, void *scratch,
+                             int32_t *vals_out, int64_t n, int bits, void *scratch,
                              cudaStream_t st);
+cudaError_t radix_sort_triples(const int32_t *keys_in, const int32_t *a_in, const int32_t *b_in,
+                               int32_t *keys_out, int32_t *a_out, int32_t *b_out, int64_t n,
+                               int bits, void *scratch, cudaStream_t st);
 
-// Exclusive scan of int32 in[0..n) into out[0..n); out[n] receives the total when with_total.
-size_t scan_scratch_bytes(int64_t n);
-cudaError_t exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n, bool with_total,
-                               void *scratch, cudaStream_t st);
+// Counts per tile of TILE_KEYS keys: bytes for n keys, and their exclusive scan in place with the
+// total in *total.
+constexpr int TILE_KEYS = 4096;
+size_t tile_counts_bytes(int64_t n);
+cudaError_t scan_tile_counts(int32_t *counts, int64_t n, int32_t *total, cudaStream_t st);
 
-// CSR -> CSC on the device, stable.  Scratch: transpose_scratch_bytes (compact: the smaller
-// sort-then-gather variant, for the fixed-scratch entry point).
-size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool compact = false);
+// CSR -> CSC on the device, stable.  Scratch: transpose_scratch_bytes.
+size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz);
 cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int32_t *ptr,
                               const int32_t *idx, const float *val, int32_t *cptr,
                               int32_t *ridx, float *cval, void *scratch, cudaStream_t st,
                               int32_t *coo_rows_out /* optional, nnz */,
                               int32_t *perm_out /* optional, nnz: CSC position -> CSR position */,
-                              bool compact = false);
+                              bool rows_ready = false /* coo_rows_out holds the rows already */);
 
 // ptr[k] = first position of the ascending keys skeys[0..n) that is >= k, for k in [0, nkeys]
 // (the pointer array of sorted row or column indices).
