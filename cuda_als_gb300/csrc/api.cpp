@@ -574,13 +574,21 @@ extern "C" als_status als_update_values(als_handle *h, const float *vals) {
     return refresh_csc_values(h);
 }
 
-extern "C" als_status als_init_factors(als_handle *h) {
-    if (!h) return set_global_error(ALS_ERR_INVALID_ARG, "null handle");
+// On the handle's stream, not waited for.
+static als_status init_factors(als_handle *h) {
     cudaSetDevice(h->cfg.device);
     if (h->cfg.autotune) reset_tuning(h);  // a new run re-tunes the ALS_SOLVE_AUTO plan
     // als_model.cu:1772-1777: srand(0), VT[k] = 0.2*((float)rand()/(float)RAND_MAX), UT = 0,
     // generated on the GPU bit for bit (init.cu: glibc's rand() sequence by jump-ahead)
     H_CUDA(h, init_factors_device(h->m, h->n, h->f, h->d_U, h->d_V, h->stream));
+    return ALS_OK;
+}
+
+extern "C" als_status als_init_factors(als_handle *h) {
+    if (!h) return set_global_error(ALS_ERR_INVALID_ARG, "null handle");
+    const als_status s = init_factors(h);
+    if (s != ALS_OK) return s;
+    H_CUDA(h, cudaStreamSynchronize(h->stream));
     return ALS_OK;
 }
 
@@ -658,7 +666,8 @@ extern "C" als_status als_iterate(als_handle *h, int32_t iters) {
 extern "C" als_status als_train(als_handle *h) {
     if (!h) return set_global_error(ALS_ERR_INVALID_ARG, "null handle");
     if (h->log) als::log_text(h->log, "als model training started", h->log_cout);  // :1768-1770
-    als_status s = als_init_factors(h);
+    als_status s = init_factors(h);
+    if (s == ALS_OK && h->log) H_CUDA(h, cudaStreamSynchronize(h->stream));  // the line says "done"
     if (s != ALS_OK) return s;
     if (h->log) als::log_text(h->log, "factors initialization done", h->log_cout);  // :1786-1788
     s = als_iterate(h, h->cfg.iters);
