@@ -373,7 +373,7 @@ cudaError_t launch_rows(const AdjArgs<float> &a, int64_t m, cudaStream_t st) {
             adjoint_tile_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    adjoint_tile_kernel<P><<<(unsigned)m, tile::up32(tile::tiles_of(nb)), smem, st>>>(a, nb);
+    adjoint_tile_kernel<P><<<(unsigned)m, tile::gram_threads(a.f, tile::patched<P>()), smem, st>>>(a, nb);
     return cudaGetLastError();
 }
 

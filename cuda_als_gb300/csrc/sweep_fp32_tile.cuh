@@ -7,6 +7,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "internal.h"
 #include "solvers.cuh"
 #include "tilesolve.cuh"
@@ -66,11 +68,16 @@ inline int tile_mode_of(int solve) {
            : solve == ALS_SOLVE_CG_FP32 || solve == ALS_SOLVE_CG_FP16 ? TILE_CG
                                                                       : TILE_LDLT;
 }
-// Threads: one a tile.  CG keeps the thread count of the 4 x 8 tiling, which its sums' order
-// depends on.
+// Threads: one a tile, or enough for the Gram's patches.  CG keeps the thread count of the 4 x 8
+// tiling, which its sums' order depends on, and whole tiles.
+template <int P>
+__host__ __device__ constexpr bool patch_mode(int mode) { return mode != TILE_CG && tile::patched<P>(); }
+template <int P>
 inline int tile_threads(int f, int mode) {
     const int nb = tile::nb_of(f);
-    return mode == TILE_CG ? nt_of(fp_of(f)) : tile::up32(mode == TILE_LU ? nb * nb : tile::tiles_of(nb));
+    return mode == TILE_CG ? nt_of(fp_of(f))
+                           : std::max(tile::up32(mode == TILE_LU ? nb * nb : 0),
+                                      tile::gram_threads(f, patch_mode<P>(mode)));
 }
 // CG: the Gram (stride 8 nb + 1) over the ring, then the ratings, its five vectors and the
 // reduction scratch.
@@ -156,8 +163,8 @@ __global__ void __launch_bounds__(512) sweep_tile_kernel(const SweepArgs a, cons
     tile::clear(acc);
     float2 bsum = make_float2(0.f, 0.f), bcomp = bsum;
     float *rv = smem + (MODE == TILE_CG ? cg_big_floats<P>(nb) : tile::big_floats<P>(nb, true));
-    tile::accumulate<P>(a.idx, a.val, a.Y, a.f, nb, beg, end, t, t.on && t.bi >= t.bj, acc, bsum,
-                        bcomp, smem, rv);
+    tile::accumulate<P, patch_mode<P>(MODE)>(a.idx, a.val, a.Y, a.f, nb, beg, end, t,
+                                             t.on && t.bi >= t.bj, acc, bsum, bcomp, smem, rv);
     tile_solve<MODE, P>(a, nb, row, nu, acc, t, make_float2(bsum.x - bcomp.x, bsum.y - bcomp.y), smem);
 }
 
@@ -244,7 +251,8 @@ __global__ void __launch_bounds__(512)
 
 template <int MODE, int P>
 cudaError_t launch_tiles(const SweepArgs &a, const Fp32Split *sp, cudaStream_t st, int *launches) {
-    const int nb = tile::nb_of(a.f), nt = tile_threads(a.f, MODE), ntp = tile::up32(tile::tiles_of(nb));
+    const int nb = tile::nb_of(a.f), nt = tile_threads<P>(a.f, MODE);
+    const int ntp = tile::gram_threads(a.f, tile::patched<P>());
     const size_t smem = tile_smem<P>(a.f, MODE);
     if (smem > 48 * 1024) {  // (a part's ring stays below)
         cudaError_t e = cudaFuncSetAttribute(sweep_tile_kernel<MODE, P>,
