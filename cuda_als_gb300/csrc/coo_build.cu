@@ -19,7 +19,7 @@
 //      is not stable, so no fixed order would do better).  The heads write the row pointers too;
 //   4. the CSC by the library's stable transpose (rows ascending within a column: scipy's tocsc
 //      order).
-// 10.0M triples, 69,878 x 10,677: 2.80 -> 1.44 ms (positions sorted by column, then by row, with
+// 10.0M triples, 69,878 x 10,677: 2.80 -> 1.05 ms (positions sorted by column, then by row, with
 // random gathers of rows, columns and values between, before).
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -40,16 +40,26 @@ inline int grid_of(int64_t work, int threads) {
 }
 
 // Counts the triples with an index out of range; writes row << col_bits | column where `word` is
-// given (rows and columns in range then fit 32 bits).
+// given (rows and columns in range then fit 32 bits).  Four triples a step: their loads overlap.
 __global__ void check_pack_kernel(int64_t nnz, const int32_t *__restrict__ r,
                                   const int32_t *__restrict__ c, int32_t rows, int32_t cols,
                                   int col_bits, uint32_t *__restrict__ word, int32_t *bad) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
     int local = 0;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t i = r[p], j = c[p];
-        if (i < 0 || i >= rows || j < 0 || j >= cols) ++local;
-        if (word) word[p] = (uint32_t)i << col_bits | (uint32_t)j;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += 4 * step) {
+        int32_t i[4], j[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool on = p + q * step < nnz;
+            i[q] = on ? r[p + q * step] : 0;
+            j[q] = on ? c[p + q * step] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (p + q * step >= nnz) break;
+            if (i[q] < 0 || i[q] >= rows || j[q] < 0 || j[q] >= cols) ++local;
+            if (word) word[p + q * step] = (uint32_t)i[q] << col_bits | (uint32_t)j[q];
+        }
     }
     local = __reduce_add_sync(0xffffffffu, local);
     if ((threadIdx.x & 31) == 0 && local) atomicAdd(bad, local);
@@ -142,17 +152,19 @@ emit_kernel(const Cells c, int64_t n, int64_t rows, const int32_t *__restrict__ 
 // Whether row and column share a 32-bit key.
 static bool coo_packs(int64_t rows, int64_t cols) { return key_bits(rows) + key_bits(cols) <= 32; }
 
-// Flags, heads per tile; then the sorted entries and the sort's scratch, of which the transpose
-// takes the place.
-size_t coo_build_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz) {
+// Flags and heads per tile; then the sort's entries and counters, of which the transpose takes the
+// place.  Packed, the entries pass between one set of two words here and the arrays of the CSC
+// (scratch has to be mapped on every call: 0.34 ms of 1.44 for five arrays of 10.0M entries).
+size_t coo_build_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool csc) {
     const size_t arr = a256(sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1));
-    const size_t sort = coo_packs(rows, cols) ? 3 * arr + radix_sort_scratch_bytes(nnz, 1)
+    const size_t sort = coo_packs(rows, cols) ? (csc ? 2 : 4) * arr + radix_counter_bytes(nnz)
                                               : 6 * arr + radix_sort_scratch_bytes(nnz, 2);
-    return 256 + a256(tile_counts_bytes(nnz)) + std::max(sort, transpose_scratch_bytes(rows, cols, nnz));
+    return 256 + a256(tile_counts_bytes(nnz)) +
+           std::max(sort, csc ? transpose_scratch_bytes(rows, cols, nnz) : 0);
 }
 
 // Device core.  `*nnz_out` (host) receives the cell count; the stream is synchronised to read the
-// validation count and the cell count (every later launch depends on them) and at the end.
+// validation count, to read the cell count (every later launch depends on them) and at the end.
 // *bad_out receives the number of triples with an index outside [0, rows) x [0, cols); then
 // nothing is built.
 cudaError_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int32_t *ridx,
@@ -182,16 +194,29 @@ cudaError_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int
 
     cudaError_t e = cudaMemsetAsync(flags, 0, 2 * sizeof(int32_t), st);
     if (e != cudaSuccess) return e;
-    check_pack_kernel<<<grid_of(nnz, 256), 256, 0, st>>>(nnz, ridx, cidx, (int32_t)rows, (int32_t)cols,
-                                                         cb, packed ? (uint32_t *)array(0) : nullptr,
-                                                         flags);
+    check_pack_kernel<<<grid_of(nnz, 4 * 256), 256, 0, st>>>(nnz, ridx, cidx, (int32_t)rows,
+                                                             (int32_t)cols, cb,
+                                                             packed ? (uint32_t *)array(0) : nullptr,
+                                                             flags);
+    int32_t got = 0;
+    e = cudaMemcpyAsync(&got, flags, sizeof(got), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    if (got) {
+        *bad_out = got;
+        return cudaSuccess;
+    }
     // 1. by row and column
     Cells c{};
     c.col_bits = cb;
     if (packed) {
-        e = radix_sort_pairs(array(0), (const int32_t *)val, array(1), array(2), nnz, rb + cb, array(3), st);
-        c.word = (const uint32_t *)array(1);
-        c.val = (const float *)array(2);
+        int32_t *const set[2][2] = {{col_ptrs ? csc_rows : array(2), col_ptrs ? (int32_t *)csc_vals : array(3)},
+                                    {array(0), array(1)}};
+        int last = 0;
+        e = radix_sort_between(array(0), (const int32_t *)val, set, nnz, rb + cb,
+                               array(col_ptrs ? 2 : 4), st, &last);
+        c.word = (const uint32_t *)set[last][0];
+        c.val = (const float *)set[last][1];
     } else {
         e = radix_sort_triples(cidx, ridx, (const int32_t *)val, array(0), array(1), array(2), nnz, cb,
                                array(6), st);
@@ -208,15 +233,10 @@ cudaError_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int
     count_heads_kernel<<<ntiles, CELL_THREADS, 0, st>>>(c, nnz, counts);
     e = scan_tile_counts(counts, nnz, flags + 1, st);
     if (e != cudaSuccess) return e;
-    int32_t got[2] = {0, 0};
-    e = cudaMemcpyAsync(got, flags, sizeof(got), cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(&got, flags + 1, sizeof(got), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
-    if (got[0]) {
-        *bad_out = got[0];
-        return cudaSuccess;
-    }
-    const int64_t cells = got[1];
+    const int64_t cells = got;
     // 3. one entry per cell, duplicates summed
     emit_kernel<<<ntiles, CELL_THREADS, 0, st>>>(c, nnz, rows, counts, flags + 1, row_ptrs, coo_rows,
                                                  col_idxs, vals);
@@ -270,8 +290,8 @@ extern "C" als_status als_coo_to_csr_device(const als_coo_view *coo, int32_t *ro
     if (s != ALS_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     void *scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(&scratch, coo_build_scratch_bytes(coo->rows, coo->cols,
-                                                                      coo->nnz), st);
+    cudaError_t e = cudaMallocAsync(&scratch, coo_build_scratch_bytes(coo->rows, coo->cols, coo->nnz,
+                                                                      col_ptrs != nullptr), st);
     if (e != cudaSuccess) return cuda_fail("cudaMallocAsync", e);
     int bad = 0;
     e = coo_to_csr_device(coo->rows, coo->cols, coo->nnz, coo->row_idxs, coo->col_idxs,
@@ -303,7 +323,7 @@ extern "C" als_status als_coo_to_csr(const als_coo_view *coo, int32_t *row_ptrs,
     // inputs (3 nnz), CSR (rows + 1, 2 nnz), COO rows (nnz), CSC (cols + 1, 2 nnz), scratch
     const size_t a_in = 3 * a256(n4), a_csr = a256(sizeof(int32_t) * (rows + 1)) + 2 * a256(n4);
     const size_t a_rows = a256(n4), a_csc = a256(sizeof(int32_t) * (cols + 1)) + 2 * a256(n4);
-    const size_t a_scr = coo_build_scratch_bytes(rows, cols, nnz);
+    const size_t a_scr = coo_build_scratch_bytes(rows, cols, nnz, col_ptrs != nullptr);
     e = cudaMalloc(&buf, a_in + a_csr + a_rows + a_csc + a_scr);
     if (e != cudaSuccess) {
         cudaStreamDestroy(st);

@@ -7,7 +7,7 @@
 // the entries by column index keeps them in row order inside each column, which is exactly the
 // order scipy's csr_tocsc produces.  All of it is HBM-bound integer traffic: coalesced tiles of
 // 4096 keys per CTA, one 256-bin histogram per tile, a scan of every digit's tile counts, then a
-// stable scatter ranked with warp match-any.
+// stable scatter ranked with warp ballots.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -35,7 +35,7 @@ constexpr int SCAT_THREADS = 512;
 constexpr int SCAT_WARPS = SCAT_THREADS / 32;                     // 16
 constexpr int SCAT_ROUNDS = RADIX_TILE / SCAT_THREADS;            // 8 keys per lane
 constexpr int SCAT_WARP_SPAN = 32 * SCAT_ROUNDS;                  // 256 contiguous keys / warp
-static_assert(RADIX_TILE == TILE_KEYS, "tiles");
+static_assert(RADIX_TILE == TILE_KEYS && SCAT_WARP_SPAN <= 256 && SCAT_ROUNDS % 4 == 0, "tiles");
 static_assert(SCAT_THREADS >= RADIX_BINS && RADIX_BINS % 32 == 0, "one thread per digit");
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -128,7 +128,7 @@ struct Move {
 
 // Stable scatter.  Warp w of tile t owns the contiguous key range [t*4096 + w*256, +256) and
 // walks it in 8 rounds of 32; a key's rank inside its warp is (keys of the same digit in earlier
-// rounds) + (lanes below it with the same digit in this round), found with match.any.  The warp
+// rounds) + (lanes below it with the same digit in this round), found with a ballot a digit bit.  The warp
 // offsets per digit are an exclusive prefix over warps on top of the tile's digit starts (a scan
 // over digits).  The entries are first placed in shared memory in digit order (the tile sorted by
 // digit), then streamed out: consecutive threads write consecutive addresses of a digit's run, so
@@ -136,9 +136,12 @@ struct Move {
 // tile counts, scanned; totals: every digit's count (its start is scanned here).
 // Shared memory sets the pace (random 8-byte stores, then rows of a digit), so a transpose moves
 // two words a rating where they fit: 98.6M ratings into 17,770 columns 2.41 -> 1.55 ms (three words,
-// sorted column ids kept for the pointers, scans of the whole histogram before).
+// sorted column ids kept for the pointers, scans of the whole histogram before), then 1.38 with
+// ballots instead of match.any, values loaded behind the ranking and two CTAs an SM without spills
+// instead of three (uniform columns: match.any 1.71, ballots 1.46, with three CTAs 1.58, with 1,024
+// threads of four keys 1.61).
 template <int MOVE>
-__global__ void __launch_bounds__(SCAT_THREADS, MOVE == MOVE_TRIPLE ? 2 : 3)
+__global__ void __launch_bounds__(SCAT_THREADS, 2)
 radix_scatter_kernel(const Move mv, int64_t n, int64_t ntiles, const int32_t *__restrict__ hist,
                      const int32_t *__restrict__ totals) {
     extern __shared__ uint2 sorted[];  // [RADIX_TILE], then keys (TRIPLE) or digits (CSR)
@@ -152,17 +155,13 @@ radix_scatter_kernel(const Move mv, int64_t n, int64_t ntiles, const int32_t *__
     // tile-local 32-bit offsets (n <= INT32_MAX): one 64-bit base per array
     const int64_t tile0 = (int64_t)blockIdx.x * RADIX_TILE;
     const int nvalid = (int)(n - tile0 < RADIX_TILE ? n - tile0 : RADIX_TILE);
-    const int wbase = warp * SCAT_WARP_SPAN;
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const int mine = warp * SCAT_WARP_SPAN + lane;  // this thread's first entry, then every 32nd
+    const int left = nvalid - mine;
     uint32_t key[SCAT_ROUNDS], x[SCAT_ROUNDS], y[SCAT_ROUNDS];
-    uint32_t at[SCAT_ROUNDS];  // digit << 16 | rank
+    uint32_t rank[SCAT_ROUNDS / 4] = {};  // below SCAT_WARP_SPAN: four to a register
 #pragma unroll
     for (int q = 0; q < SCAT_ROUNDS; ++q) {
-        const int o = wbase + q * 32 + lane;
-        const bool valid = o < nvalid;
-        key[q] = valid ? mv.key[tile0 + o] : 0;
-        x[q] = MOVE == MOVE_PAIR || !valid ? 0 : mv.a[tile0 + o];
-        y[q] = !valid ? 0 : mv.val ? mv.val[tile0 + o] : (uint32_t)(tile0 + o);
+        key[q] = 32 * q < left ? mv.key[tile0 + mine + 32 * q] : 0;
     }
     int first = 0, total = 0;
     if (digit_thread) {
@@ -173,22 +172,32 @@ radix_scatter_kernel(const Move mv, int64_t n, int64_t ntiles, const int32_t *__
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < SCAT_ROUNDS; ++q) {
-        const bool valid = wbase + q * 32 + lane < nvalid;
-        // invalid lanes get a private digit so they never match a real one
-        const uint32_t d = valid ? (key[q] >> mv.shift) & (RADIX_BINS - 1) : RADIX_BINS + lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const bool valid = 32 * q < left;
+        const uint32_t d = (key[q] >> mv.shift) & (RADIX_BINS - 1);
+        unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int b = 0; b < RADIX_BITS; ++b) {
+            const bool one = (d >> b) & 1;
+            const unsigned m = __ballot_sync(0xffffffffu, one);
+            peers &= one ? m : ~m;
+        }
         const int before = valid ? wcnt[warp][d] : 0;
-        at[q] = d << 16 | (uint32_t)(before + __popc(peers & lt_mask));
-        if (MOVE == MOVE_PAIR) x[q] = key[q];
-        if (MOVE == MOVE_CSR) x[q] |= ((key[q] >> RADIX_BITS) & mv.high_mask) << mv.row_bits;
+        rank[q / 4] |= (uint32_t)(before + __popc(peers & ((1u << lane) - 1u))) << 8 * (q % 4);
         __syncwarp();
         if (valid && (__ffs(peers) - 1) == lane) wcnt[warp][d] = before + __popc(peers);
         __syncwarp();
     }
+    // the rest of the entries is under way during the scans
+#pragma unroll
+    for (int q = 0; q < SCAT_ROUNDS; ++q) {
+        const bool valid = 32 * q < left;
+        x[q] = MOVE == MOVE_PAIR ? key[q] : valid ? mv.a[tile0 + mine + 32 * q] : 0;
+        y[q] = !valid ? 0 : mv.val ? mv.val[tile0 + mine + 32 * q] : (uint32_t)(tile0 + mine + 32 * q);
+    }
     __syncthreads();
     int cnt = 0, icnt = 0, itot = 0;  // keys of digit tid in this tile; inclusive scans over digits
     if (digit_thread) {
-#pragma unroll
+#pragma unroll 4
         for (int w = 0; w < SCAT_WARPS; ++w) cnt += wcnt[w][tid];
         icnt = cnt;
         itot = total;
@@ -213,7 +222,7 @@ radix_scatter_kernel(const Move mv, int64_t n, int64_t ntiles, const int32_t *__
             base += wsum[1][w];
         }
         goff[tid] = base + first - start;  // a sorted slot j of digit d goes to goff[d] + j
-#pragma unroll
+#pragma unroll 4
         for (int w = 0; w < SCAT_WARPS; ++w) {
             const int t = wcnt[w][tid];
             wcnt[w][tid] = start;
@@ -223,9 +232,10 @@ radix_scatter_kernel(const Move mv, int64_t n, int64_t ntiles, const int32_t *__
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < SCAT_ROUNDS; ++q) {
-        const uint32_t d = at[q] >> 16;
-        if (d >= RADIX_BINS) continue;
-        const int lp = wcnt[warp][d] + (int)(at[q] & 0xffffu);
+        if (32 * q >= left) continue;
+        const uint32_t d = (key[q] >> mv.shift) & (RADIX_BINS - 1);
+        const int lp = wcnt[warp][d] + (int)(rank[q / 4] >> 8 * (q % 4) & 0xffu);
+        if (MOVE == MOVE_CSR) x[q] |= ((key[q] >> RADIX_BITS) & mv.high_mask) << mv.row_bits;
         sorted[lp] = make_uint2(x[q], y[q]);
         if (MOVE == MOVE_TRIPLE) skey[lp] = key[q];
         if (MOVE == MOVE_CSR) sdig[lp] = (uint8_t)d;
@@ -356,14 +366,23 @@ __global__ void degree_keys_kernel(int64_t rows, const int32_t *__restrict__ ptr
         keys[r] = maxd - (ptr[r + 1] - ptr[r]);
 }
 
+// Four entries a step, so that their loads overlap: 9.0M ratings 36.9 -> 16.0 us.
 __global__ void count_bad_kernel(int64_t nnz, const int32_t *__restrict__ idx, int32_t limit,
                                  const float *__restrict__ val, int32_t *bad) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
     int local = 0;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        int32_t c = idx[p];
-        float v = val ? val[p] : 0.0f;
-        if (c < 0 || c >= limit || !isfinite(v)) ++local;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += 4 * step) {
+        int32_t c[4];
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool on = p + q * step < nnz;
+            c[q] = on ? idx[p + q * step] : 0;
+            v[q] = on && val ? val[p + q * step] : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (p + q * step < nnz && (c[q] < 0 || c[q] >= limit || !isfinite(v[q]))) ++local;
     }
     local = __reduce_add_sync(0xffffffffu, local);
     if ((threadIdx.x & 31) == 0 && local) atomicAdd(bad, local);
@@ -389,30 +408,42 @@ size_t radix_sort_scratch_bytes(int64_t n, int values) {
     return (1 + (size_t)values) * array_bytes(n) + counter_bytes(n);
 }
 
-// The passes alternate between the scratch set and the outputs, so that the last one lands there.
-cudaError_t radix_sort_pairs(const int32_t *keys_in, const int32_t *vals_in, int32_t *keys_out,
-                             int32_t *vals_out, int64_t n, int bits, void *scratch,
-                             cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    uint32_t *set[2][2] = {{(uint32_t *)keys_out, (uint32_t *)vals_out},
-                           {(uint32_t *)scratch, (uint32_t *)((char *)scratch + array_bytes(n))}};
-    const Counters c = counters_at((char *)scratch + 2 * array_bytes(n), n);
+size_t radix_counter_bytes(int64_t n) { return counter_bytes(n); }
+
+cudaError_t radix_sort_between(const int32_t *keys_in, const int32_t *vals_in,
+                               int32_t *const (&set)[2][2], int64_t n, int bits, void *counters,
+                               cudaStream_t st, int *last) {
+    const Counters c = counters_at(counters, n);
     const int passes = passes_of(bits);
+    *last = (passes - 1) & 1;
+    if (n <= 0) return cudaSuccess;
     Move mv{};
     mv.key = (const uint32_t *)keys_in;
     mv.val = (const uint32_t *)vals_in;
     mv.keep = ~0u;
     for (int p = 0; p < passes; ++p) {
-        uint32_t **dst = set[(passes - 1 - p) & 1];
-        mv.a_out = dst[0];
-        mv.val_out = dst[1];
+        mv.a_out = (uint32_t *)set[p & 1][0];
+        mv.val_out = (uint32_t *)set[p & 1][1];
         mv.shift = p * RADIX_BITS;
         const cudaError_t e = radix_pass<MOVE_PAIR>(mv, n, c, c.totals[0], st);
         if (e != cudaSuccess) return e;
-        mv.key = dst[0];
-        mv.val = dst[1];
+        mv.key = mv.a_out;
+        mv.val = mv.val_out;
     }
     return cudaSuccess;
+}
+
+// The passes alternate between the scratch set and the outputs, so that the last one lands there.
+cudaError_t radix_sort_pairs(const int32_t *keys_in, const int32_t *vals_in, int32_t *keys_out,
+                             int32_t *vals_out, int64_t n, int bits, void *scratch,
+                             cudaStream_t st) {
+    int32_t *k2 = (int32_t *)scratch, *v2 = (int32_t *)((char *)scratch + array_bytes(n));
+    void *counters = (char *)scratch + 2 * array_bytes(n);
+    const bool odd = passes_of(bits) & 1;
+    int32_t *const set[2][2] = {{odd ? keys_out : k2, odd ? vals_out : v2},
+                                {odd ? k2 : keys_out, odd ? v2 : vals_out}};
+    int last = 0;
+    return radix_sort_between(keys_in, vals_in, set, n, bits, counters, st, &last);
 }
 
 cudaError_t radix_sort_triples(const int32_t *keys_in, const int32_t *a_in, const int32_t *b_in,
@@ -452,10 +483,11 @@ static bool transpose_packs(int64_t rows, int64_t cols) {
     return cb <= 2 * RADIX_BITS && key_bits(rows) + std::max(0, cb - RADIX_BITS) <= 32;
 }
 
-// The rows of the CSR, a set of two words a rating and the counters; the general path's set has
-// three, and it sorts the columns themselves.
+// Two passes: a set of two words a rating (the rows of the CSR wait in the output's); one pass: the
+// rows; the general path: the rows, a set of three words and the sorted columns.  And the counters.
 size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz) {
-    return (transpose_packs(rows, cols) ? 3 : 5) * array_bytes(nnz) + counter_bytes(nnz);
+    const int arrays = !transpose_packs(rows, cols) ? 5 : passes_of(key_bits(cols)) == 2 ? 2 : 1;
+    return arrays * array_bytes(nnz) + counter_bytes(nnz);
 }
 
 cudaError_t expand_rows(int64_t rows, int64_t nnz, const int32_t *ptr, int32_t *coo_rows,
@@ -472,7 +504,9 @@ cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int
     if (nnz <= 0) return cudaMemsetAsync(cptr, 0, sizeof(int32_t) * (size_t)(cols + 1), st);
     const size_t arr = array_bytes(nnz);
     char *s = (char *)scratch;
-    int32_t *coo_rows = coo_rows_out ? coo_rows_out : (int32_t *)s;
+    const int cb = key_bits(cols), rb = key_bits(rows), passes = passes_of(cb);
+    const bool packs = transpose_packs(rows, cols), one = passes == 1;
+    int32_t *coo_rows = coo_rows_out ? coo_rows_out : packs && !one ? ridx : (int32_t *)s;
     cudaError_t e = cudaSuccess;
     if (!rows_ready) {
         e = expand_rows(rows, nnz, ptr, coo_rows, st);
@@ -481,11 +515,9 @@ cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int
     // the rating moves with its row, or its CSR position where the caller keeps the permutation
     const uint32_t *v_in = perm_out ? nullptr : (const uint32_t *)val;
     uint32_t *v_out = (uint32_t *)(perm_out ? perm_out : (int32_t *)cval);
-    const int cb = key_bits(cols), rb = key_bits(rows), passes = passes_of(cb);
-    if (transpose_packs(rows, cols)) {
-        uint32_t *word = (uint32_t *)(s + arr), *pay = (uint32_t *)(s + 2 * arr);
-        const Counters c = counters_at(s + 3 * arr, nnz);
-        const bool one = passes == 1;
+    if (packs) {
+        uint32_t *word = (uint32_t *)s, *pay = (uint32_t *)(s + arr);  // (two passes only)
+        const Counters c = counters_at(s + (one ? 1 : 2) * arr, nnz);
         Move mv{};
         mv.key = (const uint32_t *)idx;
         mv.a = (const uint32_t *)coo_rows;
@@ -559,7 +591,7 @@ cudaError_t gather_f32(int64_t n, const int32_t *perm, const float *src, float *
 cudaError_t count_bad_entries(int64_t nnz, const int32_t *idx, int32_t limit, const float *val,
                               int32_t *bad, cudaStream_t st) {
     if (nnz <= 0) return cudaSuccess;
-    count_bad_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(nnz, idx, limit, val, bad);
+    count_bad_kernel<<<grid_for(nnz, 4 * 256), 256, 0, st>>>(nnz, idx, limit, val, bad);
     return cudaGetLastError();
 }
 

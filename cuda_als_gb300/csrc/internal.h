@@ -41,6 +41,13 @@ size_t radix_sort_scratch_bytes(int64_t n, int values);
 cudaError_t radix_sort_pairs(const int32_t *keys_in, const int32_t *vals_in, int32_t *keys_out,
                              int32_t *vals_out, int64_t n, int bits, void *scratch,
                              cudaStream_t st);
+// The pairs' passes between two sets of (keys, values) of the caller's, the first into set[0];
+// *last is the one that holds the result.  keys_in may be set[1]'s.  `counters` holds
+// radix_counter_bytes(n) bytes.
+size_t radix_counter_bytes(int64_t n);
+cudaError_t radix_sort_between(const int32_t *keys_in, const int32_t *vals_in,
+                               int32_t *const (&set)[2][2], int64_t n, int bits, void *counters,
+                               cudaStream_t st, int *last);
 cudaError_t radix_sort_triples(const int32_t *keys_in, const int32_t *a_in, const int32_t *b_in,
                                int32_t *keys_out, int32_t *a_out, int32_t *b_out, int64_t n,
                                int bits, void *scratch, cudaStream_t st);
