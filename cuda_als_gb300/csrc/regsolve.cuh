@@ -204,21 +204,23 @@ struct TriLayout {
 // Cholesky A = L L^T of the padded FP x FP matrix held in Ls (packed, tri_off rows; entry (i, j)
 // for j <= i must be set, the rest of each row's blocks is scratch), and the forward solve L y = b
 // beside it: `bv` holds b on entry (FP floats, scratch afterwards), `yv` receives y.  On exit entry
-// (i, j <= i) holds L[i][j], Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for r >= c (the inverse of each
-// 8 x 8 diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128 threads of a group (et =
-// 0..127); warp `lead` / 32 works on the diagonal blocks.
+// (i, j) left of the diagonal blocks holds L[i][j], Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for
+// r >= c (the inverse of each 8 x 8 diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128
+// threads of a group (et = 0..127); warp `lead` / 32 works on the diagonal blocks.
 //
 // Left-looking in blocks of 8 columns, three barriers per block:
 //  (a) the block's entries lose L[r][0:k0] . L[k0+4h+kk][0:k0], a (row, column half) item a thread;
-//  (b) thread `lead` factors the 8 x 8 diagonal block in registers (rsqrt pivots) and eight lanes
-//      of its warp invert it, a column each;
+//  (b) the lead warp factors the 8 x 8 diagonal block in registers (rsqrt pivots), every lane alike,
+//      so that eight of them have it at hand to invert it, a column each;
 //  (c) every row below takes its block columns as s L_KK^-T; each thread also forms the block's
 //      y = L_KK^-1 b and folds it into its own row's b.
-// Work is dealt from the lead warp on, so that the groups' few busy warps sit on different
-// schedulers.  Half-sweep over 480,189 rows and 98.6M ratings, ms at f = 64 / 100 / 128: 24.0 / 50.9
-// / 91.5 with separate solves and work dealt from warp 0 (and one buffer less at 128), now 18.0 /
-// 36.1 / 51.8.  Two rows an item: 18.8 / 38.5 / 53.8; (a) for the next block by the warps that idle
-// in (b): 19.1 / 38.2 / 50.5.
+// The groups' serial steps, (b) above all, set the time.  Work is dealt from the lead warp on, so
+// that the groups' few busy warps sit on different schedulers.  Half-sweep over 480,189 rows and
+// 98.6M ratings, ms at f = 64 / 100 / 128: 24.0 / 50.9 / 91.5 with separate solves and work dealt
+// from warp 0 (and one buffer less at 128), then 18.0 / 36.1 / 51.8; with (b)'s factor no longer
+// passed from one lane to the inverting ones through shared memory f = 64 15.8, and 100,000 rows of
+// 9.0M ratings at f = 100 / 128 7.39 / 10.61 -> 6.69 / 9.50.  Two rows an item in (a): 18.8 / 38.5 /
+// 53.8; (a) for the next block by the warps that idle in (b): 19.1 / 38.2 / 50.5.
 // Returns false (on thread lead) if a pivot was not positive and finite.
 template <int FP>
 __device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, float *bv, float *yv,
@@ -262,68 +264,46 @@ __device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, fl
         }
         float *dv = Dv + K * B * B;
         if (ev < 32) {
-            if (et == lead) {
-                // (b) factor: right-looking inside the block, everything in registers
-                float m[B][B];
+            // (b) right-looking in registers, on every lane alike (a pivot that is not positive
+            // leaves the rest undefined: the caller drops the row)
+            float m[B][B], iv[B];
 #pragma unroll
-                for (int r = 0; r < B; ++r) {
-                    const float *lr = Ls + tri_off(k0 + r) + k0;
-                    const float4 x = *reinterpret_cast<const float4 *>(lr);
+            for (int r = 0; r < B; ++r) {
+                const float *lr = Ls + tri_off(k0 + r) + k0;
+                const float4 x = *reinterpret_cast<const float4 *>(lr);
+                m[r][0] = x.x; m[r][1] = x.y; m[r][2] = x.z; m[r][3] = x.w;
+                if (r >= 4) {
                     const float4 y = *reinterpret_cast<const float4 *>(lr + 4);
-                    m[r][0] = x.x; m[r][1] = x.y; m[r][2] = x.z; m[r][3] = x.w;
                     m[r][4] = y.x; m[r][5] = y.y; m[r][6] = y.z; m[r][7] = y.w;
                 }
-                float iv[B];
+            }
 #pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const float dk2 = m[k][k];
-                    const bool good = dk2 > 0.f && isfinite(dk2);
-                    ok = ok && good;
-                    const float inv = good ? rsqrtf(dk2) : 1.f;
-                    m[k][k] = good ? dk2 * inv : 1.f;
-                    iv[k] = inv;
+            for (int k = 0; k < B; ++k) {
+                const float dk2 = m[k][k];
+                ok = ok && dk2 > 0.f && isfinite(dk2);
+                iv[k] = rsqrtf(dk2);
 #pragma unroll
-                    for (int r = k + 1; r < B; ++r) m[r][k] *= inv;
+                for (int r = k + 1; r < B; ++r) m[r][k] *= iv[k];
 #pragma unroll
-                    for (int r = k + 1; r < B; ++r)
+                for (int r = k + 1; r < B; ++r)
 #pragma unroll
-                        for (int j = k + 1; j <= r; ++j) m[r][j] = fmaf(-m[r][k], m[j][k], m[r][j]);
-                }
-#pragma unroll
-                for (int r = 0; r < B; ++r) {  // L rows (entries right of the diagonal: zero)
-                    float *lr = Ls + tri_off(k0 + r) + k0;
-                    *reinterpret_cast<float4 *>(lr) =
-                        make_float4(m[r][0], r >= 1 ? m[r][1] : 0.f, r >= 2 ? m[r][2] : 0.f,
-                                    r >= 3 ? m[r][3] : 0.f);
-                    *reinterpret_cast<float4 *>(lr + 4) =
-                        make_float4(r >= 4 ? m[r][4] : 0.f, r >= 5 ? m[r][5] : 0.f,
-                                    r >= 6 ? m[r][6] : 0.f, r >= 7 ? m[r][7] : 0.f);
-                }
+                    for (int j = k + 1; j <= r; ++j) m[r][j] = fmaf(-m[r][k], m[j][k], m[r][j]);
+            }
+            if (et == lead) {
                 *reinterpret_cast<float4 *>(invd + k0) = make_float4(iv[0], iv[1], iv[2], iv[3]);
                 *reinterpret_cast<float4 *>(invd + k0 + 4) = make_float4(iv[4], iv[5], iv[6], iv[7]);
             }
-            __syncwarp();
+            // its inverse, lane c column c: D[c][c] = 1 / L_cc,
+            // D[r][c] = -(sum_{c <= t < r} L[r][t] D[t][c]) / L[r][r]
             const int c = et & 31;
-            if (c < B) {
-                // inverse, lane c its column: D[c][c] = 1 / L_cc,
-                // D[r][c] = -(sum_{c <= t < r} L[r][t] D[t][c]) / L[r][r]
-                float iv[B], d[B];
-                const float4 i0 = *reinterpret_cast<const float4 *>(invd + k0);
-                const float4 i1 = *reinterpret_cast<const float4 *>(invd + k0 + 4);
-                iv[0] = i0.x; iv[1] = i0.y; iv[2] = i0.z; iv[3] = i0.w;
-                iv[4] = i1.x; iv[5] = i1.y; iv[6] = i1.z; iv[7] = i1.w;
+            float d[B];
 #pragma unroll
-                for (int r = 0; r < B; ++r) {
-                    const float *lr = Ls + tri_off(k0 + r) + k0;
-                    const float4 x = *reinterpret_cast<const float4 *>(lr);
-                    const float4 y = *reinterpret_cast<const float4 *>(lr + 4);
-                    const float m[B] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-                    float acc = 0.f;
+            for (int r = 0; r < B; ++r) {
+                float acc = 0.f;
 #pragma unroll
-                    for (int t = 0; t < r; ++t) acc = fmaf(m[t], d[t], acc);  // (d[t < c] is zero)
-                    d[r] = r < c ? 0.f : r == c ? iv[r] : -acc * iv[r];
-                    if (r >= c) dv[r * B + c] = d[r];
-                }
+                for (int t = 0; t < r; ++t) acc = fmaf(m[r][t], d[t], acc);  // (d[t < c] is zero)
+                d[r] = r < c ? 0.f : r == c ? iv[r] : -acc * iv[r];
+                if (c < B && r >= c) dv[r * B + c] = d[r];
             }
         }
         gs.sync();
@@ -342,12 +322,15 @@ __device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, fl
             sb[4] = x1.x; sb[5] = x1.y; sb[6] = x1.z; sb[7] = x1.w;
 #pragma unroll
             for (int kk = 0; kk < B; ++kk) {
-                float acc = 0.f, accy = 0.f;
+                float acc = 0.f, accy = 0.f, dr[B];
+                const float4 d0 = *reinterpret_cast<const float4 *>(dv + kk * B);
+                const float4 d1 = *reinterpret_cast<const float4 *>(dv + kk * B + (kk >= 4 ? 4 : 0));
+                dr[0] = d0.x; dr[1] = d0.y; dr[2] = d0.z; dr[3] = d0.w;
+                dr[4] = d1.x; dr[5] = d1.y; dr[6] = d1.z; dr[7] = d1.w;
 #pragma unroll
                 for (int q = 0; q <= kk; ++q) {
-                    const float dq = dv[kk * B + q];
-                    acc = fmaf(sb[q], dq, acc);
-                    accy = fmaf(dq, rb[q], accy);
+                    acc = fmaf(sb[q], dr[q], acc);
+                    accy = fmaf(dr[q], rb[q], accy);
                 }
                 o[kk] = acc;
                 y[kk] = accy;
