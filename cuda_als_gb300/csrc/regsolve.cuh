@@ -201,9 +201,9 @@ struct TriLayout {
     static constexpr int floats = 32 * (FP / 8) * (FP / 8 + 1) + 4 * FP;
 };
 
-// Cholesky A = L L^T of the padded FP x FP matrix held in Ls (packed, tri_off rows; entry (i, j)
+// Cholesky A = L L^T of the leading n x n matrix (n a multiple of 16) held in Ls (packed, tri_off rows; entry (i, j)
 // for j <= i must be set, the rest of each row's blocks is scratch), and the forward solve L y = b
-// beside it: `bv` holds b on entry (FP floats, scratch afterwards), `yv` receives y.  On exit entry
+// beside it: `bv` holds b on entry (n floats, scratch afterwards), `yv` receives y.  On exit entry
 // (i, j) left of the diagonal blocks holds L[i][j], Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for
 // r >= c (the inverse of each 8 x 8 diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128
 // threads of a group (et = 0..127); warp `lead` / 32 works on the diagonal blocks.
@@ -222,17 +222,16 @@ struct TriLayout {
 // 9.0M ratings at f = 100 / 128 7.39 / 10.61 -> 6.69 / 9.50.  Two rows an item in (a): 18.8 / 38.5 /
 // 53.8; (a) for the next block by the warps that idle in (b): 19.1 / 38.2 / 50.5.
 // Returns false (on thread lead) if a pivot was not positive and finite.
-template <int FP>
-__device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, float *bv, float *yv,
+__device__ __forceinline__ bool chol_fac(int et, int n, int lead, float *Ls, float *Dv, float *invd, float *bv, float *yv,
                          const GroupSync &gs) {
     constexpr int B = 8;
     bool ok = true;
     const int ev = (et + 128 - lead) & 127;
 #pragma unroll 1
-    for (int K = 0; K < FP / B; ++K) {
+    for (int K = 0; K < n / B; ++K) {
         const int k0 = K * B;
         if (k0 > 0) {
-            const int nitems = 2 * (FP - k0);
+            const int nitems = 2 * (n - k0);
             for (int t = ev; t < nitems; t += 128) {
                 const int r = k0 + (t >> 1), c0 = k0 + 4 * (t & 1);
                 float *lr = Ls + tri_off(r);
@@ -309,13 +308,13 @@ __device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, fl
         gs.sync();
         // (c) rows below the block; b's block by every thread, the first keeps it
         const int row = k0 + B + ev;
-        if (row < FP || ev == 0) {
+        if (row < n || ev == 0) {
             float rb[B], y[B], sb[B], o[B];
             const float4 b0 = *reinterpret_cast<const float4 *>(bv + k0);
             const float4 b1 = *reinterpret_cast<const float4 *>(bv + k0 + 4);
             rb[0] = b0.x; rb[1] = b0.y; rb[2] = b0.z; rb[3] = b0.w;
             rb[4] = b1.x; rb[5] = b1.y; rb[6] = b1.z; rb[7] = b1.w;
-            float *lr = Ls + tri_off(row < FP ? row : k0) + k0;
+            float *lr = Ls + tri_off(row < n ? row : k0) + k0;
             const float4 x0 = *reinterpret_cast<const float4 *>(lr);
             const float4 x1 = *reinterpret_cast<const float4 *>(lr + 4);
             sb[0] = x0.x; sb[1] = x0.y; sb[2] = x0.z; sb[3] = x0.w;
@@ -335,7 +334,7 @@ __device__ bool chol_fac(int et, int lead, float *Ls, float *Dv, float *invd, fl
                 o[kk] = acc;
                 y[kk] = accy;
             }
-            if (row < FP) {
+            if (row < n) {
                 *reinterpret_cast<float4 *>(lr) = make_float4(o[0], o[1], o[2], o[3]);
                 *reinterpret_cast<float4 *>(lr + 4) = make_float4(o[4], o[5], o[6], o[7]);
                 float t = bv[row];
@@ -369,15 +368,14 @@ __device__ __forceinline__ void read8(const float *p, float (&y)[8]) {
     y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
     y[4] = b.x; y[5] = b.y; y[6] = b.z; y[7] = b.w;
 }
-// `acc` <- the row's y with L y = acc (et >= FP: no row).
-template <int FP>
-__device__ __forceinline__ void chol_forward(int et, const float *Ls, const float *Dv, float *xb,
+// `acc` <- the row's y with L y = acc (et >= n: no row).
+__device__ __forceinline__ void chol_forward(int et, int n, const float *Ls, const float *Dv, float *xb,
                                              float &acc, const GroupSync &gs) {
     const int lane = et & 31, w = et >> 5;
-    const bool live = et < FP;
+    const bool live = et < n;
     const float *own = Ls + tri_off(live ? et : 0);
 #pragma unroll 1
-    for (int b = 0; b < FP / 16; ++b) {
+    for (int b = 0; b < n / 16; ++b) {
         const int k0 = 16 * b;
         float *xk = xb + (b & 1) * 16;
         float y[8], l[8];
@@ -421,8 +419,7 @@ __device__ __forceinline__ void chol_forward(int et, const float *Ls, const floa
     }
 }
 // `acc` <- the row's x with L^T x = acc.
-template <int FP>
-__device__ __forceinline__ void chol_backward(int et, const float *Ls, const float *Dv, float *xb,
+__device__ __forceinline__ void chol_backward(int et, int n, const float *Ls, const float *Dv, float *xb,
                                               float &acc, const GroupSync &gs) {
     const int lane = et & 31, w = et >> 5;
     auto fold = [&](int r0, const float (&x)[8]) {  // the results of rows r0..r0+7
@@ -430,7 +427,7 @@ __device__ __forceinline__ void chol_backward(int et, const float *Ls, const flo
         for (int q = 0; q < 8; ++q) acc = fmaf(-Ls[tri_off(r0 + q) + et], x[q], acc);
     };
 #pragma unroll 1
-    for (int b = FP / 16 - 1; b >= 0; --b) {
+    for (int b = n / 16 - 1; b >= 0; --b) {
         const int k0 = 16 * b;
         float *xk = xb + ((b + 1) & 1) * 16;
         float x[8];
