@@ -105,7 +105,7 @@ als_status prepare_precision_path(als_handle *h);
 void release_precision_path(als_handle *h);
 void invalidate_graphs(als_handle *h);
 als_status refresh_csc_values(als_handle *h);
-als_status run_half_sweep(als_handle *h, int side);
+als_status run_half_sweep(als_handle *h, int side, bool timed = true);
 als_status run_epochs(als_handle *h, int32_t iters);
 void data_changed(als_handle *h);
 void reset_tuning(als_handle *h);

@@ -149,7 +149,6 @@ struct TcState {
     unsigned int *d_cmax = nullptr;               // column maxima (bit patterns) [MAXF]
     int32_t *d_work = nullptr;                     // one row counter per bucket
     int num_sms = 0;
-    cudaEvent_t ev_q[2] = {nullptr, nullptr};
 };
 
 bool tc_path_supported(int f) { return f >= 1 && f <= tcg::MAXF; }
@@ -204,7 +203,6 @@ als_status tc_prepare(als_handle *h, std::string *why) {
         *why = "out of memory";
         return ALS_ERR_OUT_OF_MEMORY;
     }
-    for (auto &e : t->ev_q) cudaEventCreate(&e);
     // sets every solver variant's shared-memory limit, which also loads them now, so no launch
     // inside a timed region (the autotuner's) loads a module
     cudaError_t e;
@@ -233,8 +231,6 @@ void tc_release(als_handle *h) {
         if (p) cudaFree(p);
     if (t->d_cmax) cudaFree(t->d_cmax);
     if (t->d_work) cudaFree(t->d_work);
-    for (auto e : t->ev_q)
-        if (e) cudaEventDestroy(e);
     delete t;
     h->tc = nullptr;
 }
@@ -249,7 +245,6 @@ als_status tc_quantise(als_handle *h, int side, int *launches, std::string *why)
     TcState *t = h->tc;
     const int64_t opp = side == 0 ? h->n : h->m;
     const float *Y = side == 0 ? h->d_V : h->d_U;
-    record_event(t->ev_q[0], h->stream);
     if (t->f8) {
         const int grid = (int)std::max<int64_t>(
             1, std::min<int64_t>((opp * h->f + 255) / 256, (int64_t)t->num_sms * 8));
@@ -263,7 +258,6 @@ als_status tc_quantise(als_handle *h, int side, int *launches, std::string *why)
             *launches += 2;
             e = cudaGetLastError();
         }
-        record_event(t->ev_q[1], h->stream);
         if (e != cudaSuccess) {
             *why = std::string("FP8 quantise: ") + cudaGetErrorString(e);
             return ALS_ERR_CUDA;
@@ -276,7 +270,6 @@ als_status tc_quantise(als_handle *h, int side, int *launches, std::string *why)
     tcg::quantise_bf16_kernel<<<grid, 256, 0, h->stream>>>(Y, opp, h->f, t->geo[0].fst,
                                                            t->d_bf[side]);
     ++*launches;
-    record_event(t->ev_q[1], h->stream);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         *why = std::string("quantise_bf16_kernel: ") + cudaGetErrorString(e);
