@@ -309,7 +309,8 @@ __global__ void __launch_bounds__(512) adjoint_tile_kernel(const AdjArgs<float> 
     float2 bsum = make_float2(0.f, 0.f), bcomp = bsum;
     tile::accumulate<P>(a.idx, a.val, a.Y, f, nb, beg, end, t, t.on, acc, bsum, bcomp, s.big, s.rv);
     tile::add_diagonal(acc, t, f, (float)nu * a.lambda);
-    if (2 * tid < f) *reinterpret_cast<float2 *>(s.vb + 2 * tid) = bsum;
+    const int rt = tile::rhs_thread(tile::patched<P>(), nb);
+    if (tile::rhs_columns(rt, f)) *reinterpret_cast<float2 *>(s.vb + 2 * rt) = bsum;
     for (int i = f + (f & 1) + tid; i < 8 * nb; i += nt) s.vb[i] = 0.f;
     __syncthreads();
     const bool ok = tile::factor<false, P>(acc, t, f, nb, s);

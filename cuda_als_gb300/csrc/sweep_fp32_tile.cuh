@@ -101,13 +101,15 @@ inline size_t tile_part_floats(int f) {
     return 64 * (size_t)tile::tiles_of(nb) + 16 * (size_t)nb;
 }
 
-// From the finished Gram tiles and the right-hand side's two columns of thread tid: regularise,
+// From the finished Gram tiles and the rhs_threads' two columns of the right-hand side: regularise,
 // solve, write x (or x = 0 and a flag).
 template <int MODE, int P>
 __device__ __forceinline__ void tile_solve(const SweepArgs &a, int nb, int row, int nu,
                                            tile::Acc &acc, const tile::Tile &t, float2 b,
                                            float *smem) {
     const int f = a.f, tid = threadIdx.x;
+    const int rt = tile::rhs_thread(patch_mode<P>(MODE), nb);
+    const bool rhs = tile::rhs_columns(rt, f);
     float *xo = a.X + (int64_t)row * f;
     tile::add_diagonal(acc, t, f, (float)nu * a.lambda);  // items_cnt * lambda (als_model.cu:157-159)
     if constexpr (MODE == TILE_CG) {
@@ -123,9 +125,9 @@ __device__ __forceinline__ void tile_solve(const SweepArgs &a, int nb, int row, 
 #pragma unroll
                 for (int c = 0; c < 8; ++c) G[(8 * t.bi + r) * GS + 8 * t.bj + c] = m[r][c];
         }
-        if (2 * tid < f) {
-            vb[2 * tid] = b.x;
-            vb[2 * tid + 1] = b.y;
+        if (rhs) {
+            vb[2 * rt] = b.x;
+            vb[2 * rt + 1] = b.y;
         }
         for (int i = tid; i < f; i += blockDim.x) vx[i] = xo[i];
         __syncthreads();
@@ -133,7 +135,7 @@ __device__ __forceinline__ void tile_solve(const SweepArgs &a, int nb, int row, 
     } else {
         const tile::Shared s = tile::carve<P>(smem, nb, MODE == TILE_LU);
         if (tid == 0) *s.bad = 0;
-        if (2 * tid < f) *reinterpret_cast<float2 *>(s.vb + 2 * tid) = b;
+        if (rhs) *reinterpret_cast<float2 *>(s.vb + 2 * rt) = b;
         for (int i = f + (f & 1) + tid; i < 8 * nb; i += blockDim.x) s.vb[i] = 0.f;
         if (MODE == TILE_LU) tile::mirror(acc, t, nb, s);
         __syncthreads();
@@ -191,9 +193,10 @@ __global__ void __launch_bounds__(512)
                 reinterpret_cast<ulonglong2 *>(out)[(4 * q + h) * T + tid] =
                     make_ulonglong2(acc[q][2 * h], acc[q][2 * h + 1]);
     }
-    if (2 * tid < a.f) {
-        *reinterpret_cast<float2 *>(out + 64 * (int64_t)T + 2 * tid) = bsum;
-        *reinterpret_cast<float2 *>(out + 64 * (int64_t)T + 8 * nb + 2 * tid) = bcomp;
+    const int rt = tile::rhs_thread(tile::patched<P>(), nb);
+    if (tile::rhs_columns(rt, a.f)) {
+        *reinterpret_cast<float2 *>(out + 64 * (int64_t)T + 2 * rt) = bsum;
+        *reinterpret_cast<float2 *>(out + 64 * (int64_t)T + 8 * nb + 2 * rt) = bcomp;
     }
 }
 
@@ -215,6 +218,7 @@ __global__ void __launch_bounds__(512)
         for (int c = 0; c < 16; ++c) sum[q][c] = 0.f;
     float2 bsum = make_float2(0.f, 0.f), bcomp = bsum, blost = bsum;
     const int64_t stride = 64 * (int64_t)T + 16 * nb;
+    const int rt = tile::rhs_thread(patch_mode<P>(MODE), nb);
     for (int32_t p = first[h]; p < first[h + 1]; ++p) {
         const float *in = part + (int64_t)p * stride;
         if (tid < T) {
@@ -229,9 +233,9 @@ __global__ void __launch_bounds__(512)
                     sum[q][4 * g + 3] += v.w;
                 }
         }
-        if (2 * tid < a.f) {
-            const float2 b = *reinterpret_cast<const float2 *>(in + 64 * (int64_t)T + 2 * tid);
-            const float2 c = *reinterpret_cast<const float2 *>(in + 64 * (int64_t)T + 8 * nb + 2 * tid);
+        if (tile::rhs_columns(rt, a.f)) {
+            const float2 b = *reinterpret_cast<const float2 *>(in + 64 * (int64_t)T + 2 * rt);
+            const float2 c = *reinterpret_cast<const float2 *>(in + 64 * (int64_t)T + 8 * nb + 2 * rt);
             const float y0 = b.x - bcomp.x, y1 = b.y - bcomp.y;
             const float t0 = bsum.x + y0, t1 = bsum.y + y1;
             bcomp = make_float2((t0 - bsum.x) - y0, (t1 - bsum.y) - y1);
@@ -274,7 +278,11 @@ cudaError_t launch_tiles(const SweepArgs &a, const Fp32Split *sp, cudaStream_t s
     }
     const int n = b.row_end - b.row_begin;
     if (n > 0) {
-        sweep_tile_kernel<MODE, P><<<(unsigned)n, nt, smem, st>>>(b, nb);
+        // Up to eight rows an SM are a matter of latency: another warp shares the copies and, at
+        // f <= 16, takes the right-hand side over.  With more rows it would take CTAs' places.
+        // 1,000 x 500, f = 10, ten epochs: 0.57 -> 0.48 ms a training call; f = 24, 1,000 rows 53 -> 47 us.
+        const int more = patch_mode<P>(MODE) && n <= 8 * 152 ? 32 : 0;
+        sweep_tile_kernel<MODE, P><<<(unsigned)n, nt + more, smem, st>>>(b, nb);
         if (launches) ++*launches;
     }
     return cudaGetLastError();
