@@ -300,9 +300,8 @@ als_status als_csr_to_csc_device(const als_csr_view *csr, int32_t *col_ptrs, int
 /* The same stable transpose without allocating anything: for callers that may not allocate
  * device memory (a plug-in inside an engine that owns all device memory, an allocation-free
  * latency-critical loop).  No counterpart in the reference.  Scratch is a fixed 16 MiB device
- * array inside this library; the transpose needs 28 bytes per rating plus 1 KiB per 4,096
- * ratings, each array rounded up to 256 bytes, so at most 593,856 ratings are accepted and larger
- * inputs are rejected with ALS_ERR_INVALID_ARG.  The first call in each CUDA context looks the
+ * array inside this library; at most 593,856 ratings are accepted (28 bytes each plus 1 KiB per
+ * 4,096) and larger inputs are rejected with ALS_ERR_INVALID_ARG.  The first call in each CUDA context looks the
  * array up (again after a device reset); all calls share the array, so calls that overlap on the
  * GPU race and must be serialised by the caller.  DEVICE pointers, enqueued on `stream`. */
 als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int32_t *col_ptrs,
@@ -325,7 +324,8 @@ als_status als_coo_to_csr(const als_coo_view *coo, int32_t *row_ptrs, int32_t *c
 
 /* Same, DEVICE pointers, enqueued on `stream` (cudaStream_t as void*), scratch allocated with
  * cudaMallocAsync on it; synchronous (the count after summing duplicates sizes the later
- * launches and is returned in *nnz_out, host memory). */
+ * launches and is returned in *nnz_out, host memory).  The CSC's arrays also serve as scratch:
+ * their entries past the count are undefined. */
 als_status als_coo_to_csr_device(const als_coo_view *coo, int32_t *row_ptrs, int32_t *col_idxs,
                                  float *vals, int32_t *coo_rows, int32_t *col_ptrs,
                                  int32_t *row_idxs, float *csc_vals, int64_t *nnz_out,
