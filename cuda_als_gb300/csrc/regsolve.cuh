@@ -208,8 +208,9 @@ struct TriLayout {
 // r >= c (the inverse of each 8 x 8 diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128
 // threads of a group (et = 0..127); warp `lead` / 32 works on the diagonal blocks.
 //
-// Left-looking in blocks of 8 columns, three barriers per block:
-//  (a) the block's entries lose L[r][0:k0] . L[k0+4h+kk][0:k0], a (row, column half) item a thread;
+// Left-looking in blocks of 8 columns, two barriers per block:
+//  (a) the block's entries lose L[r][0:k0] . L[k0+4h+kk][0:k0], a (row, column half) item a thread,
+//      the diagonal block's among the lead warp's, which goes on to (b) without waiting;
 //  (b) the lead warp factors the 8 x 8 diagonal block in registers (rsqrt pivots), every lane alike,
 //      so that eight of them have it at hand to invert it, a column each;
 //  (c) every row below takes its block columns as s L_KK^-T; each thread also forms the block's
@@ -219,7 +220,8 @@ struct TriLayout {
 // 98.6M ratings, ms at f = 64 / 100 / 128: 24.0 / 50.9 / 91.5 with separate solves and work dealt
 // from warp 0 (and one buffer less at 128), then 18.0 / 36.1 / 51.8; with (b)'s factor no longer
 // passed from one lane to the inverting ones through shared memory f = 64 15.8, and 100,000 rows of
-// 9.0M ratings at f = 100 / 128 7.39 / 10.61 -> 6.69 / 9.50.  Two rows an item in (a): 18.8 / 38.5 /
+// 9.0M ratings at f = 100 / 128 7.39 / 10.61 -> 6.69 / 9.50; with (b) beside the other warps' (a) f = 64
+// 15.4, 100,000 rows 6.59 / 8.98.  Two rows an item in (a): 18.8 / 38.5 /
 // 53.8; (a) for the next block by the warps that idle in (b): 19.1 / 38.2 / 50.5.
 // Returns false (on thread lead) if a pivot was not positive and finite.
 __device__ __forceinline__ bool chol_fac(int et, int n, int lead, float *Ls, float *Dv, float *invd, float *bv, float *yv,
@@ -232,7 +234,7 @@ __device__ __forceinline__ bool chol_fac(int et, int n, int lead, float *Ls, flo
         const int k0 = K * B;
         if (k0 > 0) {
             const int nitems = 2 * (n - k0);
-            for (int t = ev; t < nitems; t += 128) {
+            for (int t = ev; t < nitems; t += ev < 32 ? nitems : 96) {
                 const int r = k0 + (t >> 1), c0 = k0 + 4 * (t & 1);
                 float *lr = Ls + tri_off(r);
                 const float *l0 = Ls + tri_off(c0), *l1 = Ls + tri_off(c0 + 1);
@@ -259,7 +261,7 @@ __device__ __forceinline__ bool chol_fac(int et, int n, int lead, float *Ls, flo
                 v.x -= s0; v.y -= s1; v.z -= s2; v.w -= s3;
                 *d = v;
             }
-            gs.sync();
+            __syncwarp();
         }
         float *dv = Dv + K * B * B;
         if (ev < 32) {
