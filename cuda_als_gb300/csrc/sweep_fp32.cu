@@ -11,11 +11,12 @@
 // The reference writes every f x f Gram to HBM (d_xtxs) and reads it back in the solver; here
 // the Gram lives in shared memory only.
 //
-// Two layouts.  f <= 175: the matrix in registers, one 8 x 8 tile a thread (tilesolve.cuh), the
-// direct solvers in place there, CG on the Gram stored to shared memory.  Larger f (the "wide"
-// kernels; a tile a thread would take more than 512 threads of 128 registers): 4 x 8 register
-// tiles for the Gram, which is stored to shared memory (stride FP + 1, conflict-free column
-// walks) and solved there.  Both do the same arithmetic in the same order: each Gram entry is one
+// Two layouts.  The direct solvers at f <= 175: the matrix in registers, one 8 x 8 tile a thread
+// (tilesolve.cuh).  Larger f (a tile a thread would take more than 512 threads of 128 registers) and
+// CG at every f: the "wide" kernels, 4 x 8 register tiles for the Gram, which is stored to shared
+// memory (stride FP + 1, conflict-free column walks) and solved there.  CG reads its matrix from
+// shared memory in every product, so it gains nothing from tiles in registers and lost CTAs to
+// them (17,504 rows of 48,369 ratings at f = 120: 1.13 ms here, 2.55 on 8 x 8 tiles).  Both do the same arithmetic in the same order: each Gram entry is one
 // sequential FMA chain over the row's ratings, in rating order (the order of the reference's
 // calculate_vtvs, als_model.cu:137-155).  The right-hand side is summed apart, more accurately:
 // thread j sums r_k y_kj over each 32 ratings and adds those sums with compensated (Kahan)
@@ -33,6 +34,51 @@
 namespace als {
 
 namespace {
+
+// The 4 x 8 tiling: padded size (a column for the rating) and threads.
+__host__ __device__ inline int fp_of(int f) { return ((f + 1 + 7) / 8) * 8; }
+__host__ __device__ inline int nt_of(int fp) {
+    int nb = fp / 8;
+    int t = nb * (nb + 1);
+    t = (t + 31) / 32 * 32;
+    return t < 64 ? 64 : t;
+}
+
+// From the regularised Gram's lower triangle in G (stride GS), b in vb and the warm start in vx:
+// solve with the selected solver and write x (or x = 0 and a flag for a non-SPD / non-finite row).
+__device__ void solve_shared(const SweepArgs &a, float *G, int GS, float *vb, float *vx, float *vr,
+                             float *vp, float *vap, float *red, float *xo) {
+    const int f = a.f;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    bool ok = true;
+    const int nt = blockDim.x;
+    if (a.solve == ALS_SOLVE_CG_FP32 || a.solve == ALS_SOLVE_CG_FP16) {
+        if (a.solve == ALS_SOLVE_CG_FP16) {  // the Gram rounded to binary16 (cg.cu:236-430)
+            for (int i = warp; i < f; i += nwarps)
+                for (int j = lane; j <= i; j += 32)
+                    G[i * GS + j] = __half2float(__float2half_rn(G[i * GS + j]));
+            __syncthreads();
+        }
+        cg_solve<CtaSync>(G, GS, f, vb, vx, vr, vp, vap, red, a.cg_iters, a.cg_tol, tid, nt);
+    } else if (a.solve == ALS_SOLVE_LU) {
+        ok = lu_nopivot_solve<CtaSync>(G, GS, f, vb, tid, nt);
+        for (int i = tid; i < f; i += blockDim.x) vx[i] = vb[i];
+    } else {
+        ok = ldlt_factor<CtaSync>(G, GS, f, tid, nt);
+        if (ok) ldlt_solve<CtaSync>(G, GS, f, vb, tid);
+        for (int i = tid; i < f; i += blockDim.x) vx[i] = vb[i];
+    }
+    __syncthreads();
+    float bad = 0.f;
+    for (int i = tid; i < f; i += blockDim.x) bad += isfinite(vx[i]) ? 0.f : 1.f;
+    bad = group_sum<CtaSync>(bad, red, tid, nt);
+    if (!ok || bad > 0.f) {
+        for (int i = tid; i < f; i += blockDim.x) xo[i] = 0.f;
+        if (tid == 0 && a.flags) atomicAdd(&a.flags[0], 1);
+        return;
+    }
+    for (int i = tid; i < f; i += blockDim.x) xo[i] = vx[i];
+}
 
 constexpr int KC = 32;      // ratings gathered per chunk
 constexpr int MAX_FP = 232; // shared-memory bound of the Gram (FP x (FP+1) floats)
@@ -241,7 +287,8 @@ bool fp32_supported(int f) { return f >= 1 && fp_of(f) <= MAX_FP; }
 
 cudaError_t launch_sweep_fp32(const SweepArgs &a, const Fp32Split *sp, cudaStream_t st,
                               int *launches) {
-    if (tile::fits(a.f)) {
+    const bool cg = a.solve == ALS_SOLVE_CG_FP32 || a.solve == ALS_SOLVE_CG_FP16;
+    if (tile::fits(a.f) && !cg) {
         switch (tile::pitch_of(a.f)) {
         case 32: return launch_tiles_32(a, sp, st, launches);
         case 64: return launch_tiles_64(a, sp, st, launches);
@@ -283,9 +330,9 @@ cudaError_t launch_sweep_fp32(const SweepArgs &a, const Fp32Split *sp, cudaStrea
 }
 
 size_t fp32_part_floats(int f) {
-    if (tile::fits(f)) return tile_part_floats(f);
-    const int FP = fp_of(f);
-    return (size_t)FP * (FP + 1) + 2 * (size_t)FP;
+    const int FP = fp_of(f);  // (a handle's buckets may run either layout)
+    const size_t wide = (size_t)FP * (FP + 1) + 2 * (size_t)FP;
+    return tile::fits(f) ? std::max(wide, tile_part_floats(f)) : wide;
 }
 
 }  // namespace als

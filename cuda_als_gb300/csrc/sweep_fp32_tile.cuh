@@ -15,82 +15,17 @@
 
 namespace als {
 
-// The 4 x 8 tiling of the wide kernels: padded size (a column for the rating) and threads.
-__host__ __device__ inline int fp_of(int f) { return ((f + 1 + 7) / 8) * 8; }
-__host__ __device__ inline int nt_of(int fp) {
-    int nb = fp / 8;
-    int t = nb * (nb + 1);
-    t = (t + 31) / 32 * 32;
-    return t < 64 ? 64 : t;
-}
+enum { TILE_LDLT = 0, TILE_LU = 1 };
 
-// From the regularised Gram's lower triangle in G (stride GS), b in vb and the warm start in vx:
-// solve with the selected solver and write x (or x = 0 and a flag for a non-SPD / non-finite row).
-static __device__ void solve_shared(const SweepArgs &a, float *G, int GS, float *vb, float *vx, float *vr,
-                             float *vp, float *vap, float *red, float *xo) {
-    const int f = a.f;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    bool ok = true;
-    const int nt = blockDim.x;
-    if (a.solve == ALS_SOLVE_CG_FP32 || a.solve == ALS_SOLVE_CG_FP16) {
-        if (a.solve == ALS_SOLVE_CG_FP16) {  // the Gram rounded to binary16 (cg.cu:236-430)
-            for (int i = warp; i < f; i += nwarps)
-                for (int j = lane; j <= i; j += 32)
-                    G[i * GS + j] = __half2float(__float2half_rn(G[i * GS + j]));
-            __syncthreads();
-        }
-        cg_solve<CtaSync>(G, GS, f, vb, vx, vr, vp, vap, red, a.cg_iters, a.cg_tol, tid, nt);
-    } else if (a.solve == ALS_SOLVE_LU) {
-        ok = lu_nopivot_solve<CtaSync>(G, GS, f, vb, tid, nt);
-        for (int i = tid; i < f; i += blockDim.x) vx[i] = vb[i];
-    } else {
-        ok = ldlt_factor<CtaSync>(G, GS, f, tid, nt);
-        if (ok) ldlt_solve<CtaSync>(G, GS, f, vb, tid);
-        for (int i = tid; i < f; i += blockDim.x) vx[i] = vb[i];
-    }
-    __syncthreads();
-    float bad = 0.f;
-    for (int i = tid; i < f; i += blockDim.x) bad += isfinite(vx[i]) ? 0.f : 1.f;
-    bad = group_sum<CtaSync>(bad, red, tid, nt);
-    if (!ok || bad > 0.f) {
-        for (int i = tid; i < f; i += blockDim.x) xo[i] = 0.f;
-        if (tid == 0 && a.flags) atomicAdd(&a.flags[0], 1);
-        return;
-    }
-    for (int i = tid; i < f; i += blockDim.x) xo[i] = vx[i];
-}
-
-
-enum { TILE_LDLT = 0, TILE_LU = 1, TILE_CG = 2 };
-
-inline int tile_mode_of(int solve) {
-    return solve == ALS_SOLVE_LU                                   ? TILE_LU
-           : solve == ALS_SOLVE_CG_FP32 || solve == ALS_SOLVE_CG_FP16 ? TILE_CG
-                                                                      : TILE_LDLT;
-}
-// Threads: one a tile, or enough for the Gram's patches.  CG keeps the thread count of the 4 x 8
-// tiling, which its sums' order depends on, and whole tiles.
-template <int P>
-__host__ __device__ constexpr bool patch_mode(int mode) { return mode != TILE_CG && tile::patched<P>(); }
+// Threads: one a tile, or enough for the Gram's patches.
 template <int P>
 inline int tile_threads(int f, int mode) {
     const int nb = tile::nb_of(f);
-    return mode == TILE_CG ? nt_of(fp_of(f))
-                           : std::max(tile::up32(mode == TILE_LU ? nb * nb : 0),
-                                      tile::gram_threads(f, patch_mode<P>(mode)));
-}
-// CG: the Gram (stride 8 nb + 1) over the ring, then the ratings, its five vectors and the
-// reduction scratch.
-template <int P>
-__host__ __device__ inline size_t cg_big_floats(int nb) {
-    const size_t g = (size_t)(8 * nb) * (8 * nb + 1), r = (size_t)tile::RING * tile::KCH * P;
-    return ((g > r ? g : r) + 3) / 4 * 4;
+    return std::max(tile::up32(mode == TILE_LU ? nb * nb : 0), tile::gram_threads(f, tile::patched<P>()));
 }
 template <int P>
 inline size_t tile_smem(int f, int mode) {
-    const int nb = tile::nb_of(f);
-    return sizeof(float) * (mode == TILE_CG ? cg_big_floats<P>(nb) + tile::RING * tile::KCH + 40 * (size_t)nb + 64
-                                            : tile::shared_floats<P>(nb, mode == TILE_LU));
+    return sizeof(float) * tile::shared_floats<P>(tile::nb_of(f), mode == TILE_LU);
 }
 template <int P>
 inline size_t part_smem() {
@@ -108,45 +43,23 @@ __device__ __forceinline__ void tile_solve(const SweepArgs &a, int nb, int row, 
                                            tile::Acc &acc, const tile::Tile &t, float2 b,
                                            float *smem) {
     const int f = a.f, tid = threadIdx.x;
-    const int rt = tile::rhs_thread(patch_mode<P>(MODE), nb);
+    const int rt = tile::rhs_thread(tile::patched<P>(), nb);
     const bool rhs = tile::rhs_columns(rt, f);
     float *xo = a.X + (int64_t)row * f;
     tile::add_diagonal(acc, t, f, (float)nu * a.lambda);  // items_cnt * lambda (als_model.cu:157-159)
-    if constexpr (MODE == TILE_CG) {
-        const int GS = 8 * nb + 1;
-        float *G = smem;
-        float *vb = smem + cg_big_floats<P>(nb) + tile::RING * tile::KCH, *vx = vb + 8 * nb;
-        float *vr = vx + 8 * nb, *vp = vr + 8 * nb, *vap = vp + 8 * nb, *red = vap + 8 * nb;
-        if (t.on) {
-            float m[8][8];
-            tile::unpack(acc, m);
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-#pragma unroll
-                for (int c = 0; c < 8; ++c) G[(8 * t.bi + r) * GS + 8 * t.bj + c] = m[r][c];
-        }
-        if (rhs) {
-            vb[2 * rt] = b.x;
-            vb[2 * rt + 1] = b.y;
-        }
-        for (int i = tid; i < f; i += blockDim.x) vx[i] = xo[i];
-        __syncthreads();
-        solve_shared(a, G, GS, vb, vx, vr, vp, vap, red, xo);
-    } else {
-        const tile::Shared s = tile::carve<P>(smem, nb, MODE == TILE_LU);
-        if (tid == 0) *s.bad = 0;
-        if (rhs) *reinterpret_cast<float2 *>(s.vb + 2 * rt) = b;
-        for (int i = f + (f & 1) + tid; i < 8 * nb; i += blockDim.x) s.vb[i] = 0.f;
-        if (MODE == TILE_LU) tile::mirror(acc, t, nb, s);
-        __syncthreads();
-        bool ok = tile::factor<MODE == TILE_LU, P>(acc, t, f, nb, s);
-        if (ok) tile::backward<MODE == TILE_LU>(s.vb, s.vx, f, nb, s);
-        int bad = 0;
-        for (int i = tid; ok && i < f; i += blockDim.x) bad |= isfinite(s.vx[i]) ? 0 : 1;
-        if (__syncthreads_or(bad)) ok = false;
-        for (int i = tid; i < f; i += blockDim.x) xo[i] = ok ? s.vx[i] : 0.f;
-        if (!ok && tid == 0 && a.flags) atomicAdd(&a.flags[0], 1);
-    }
+    const tile::Shared s = tile::carve<P>(smem, nb, MODE == TILE_LU);
+    if (tid == 0) *s.bad = 0;
+    if (rhs) *reinterpret_cast<float2 *>(s.vb + 2 * rt) = b;
+    for (int i = f + (f & 1) + tid; i < 8 * nb; i += blockDim.x) s.vb[i] = 0.f;
+    if (MODE == TILE_LU) tile::mirror(acc, t, nb, s);
+    __syncthreads();
+    bool ok = tile::factor<MODE == TILE_LU, P>(acc, t, f, nb, s);
+    if (ok) tile::backward<MODE == TILE_LU>(s.vb, s.vx, f, nb, s);
+    int bad = 0;
+    for (int i = tid; ok && i < f; i += blockDim.x) bad |= isfinite(s.vx[i]) ? 0 : 1;
+    if (__syncthreads_or(bad)) ok = false;
+    for (int i = tid; i < f; i += blockDim.x) xo[i] = ok ? s.vx[i] : 0.f;
+    if (!ok && tid == 0 && a.flags) atomicAdd(&a.flags[0], 1);
 }
 
 template <int MODE, int P>
@@ -164,9 +77,8 @@ __global__ void __launch_bounds__(512) sweep_tile_kernel(const SweepArgs a, cons
     tile::Acc acc;
     tile::clear(acc);
     float2 bsum = make_float2(0.f, 0.f), bcomp = bsum;
-    float *rv = smem + (MODE == TILE_CG ? cg_big_floats<P>(nb) : tile::big_floats<P>(nb, true));
-    tile::accumulate<P, patch_mode<P>(MODE)>(a.idx, a.val, a.Y, a.f, nb, beg, end, t,
-                                             t.on && t.bi >= t.bj, acc, bsum, bcomp, smem, rv);
+    tile::accumulate<P>(a.idx, a.val, a.Y, a.f, nb, beg, end, t, t.on && t.bi >= t.bj, acc, bsum, bcomp,
+                        smem, smem + tile::big_floats<P>(nb, true));
     tile_solve<MODE, P>(a, nb, row, nu, acc, t, make_float2(bsum.x - bcomp.x, bsum.y - bcomp.y), smem);
 }
 
@@ -218,7 +130,7 @@ __global__ void __launch_bounds__(512)
         for (int c = 0; c < 16; ++c) sum[q][c] = 0.f;
     float2 bsum = make_float2(0.f, 0.f), bcomp = bsum, blost = bsum;
     const int64_t stride = 64 * (int64_t)T + 16 * nb;
-    const int rt = tile::rhs_thread(patch_mode<P>(MODE), nb);
+    const int rt = tile::rhs_thread(tile::patched<P>(), nb);
     for (int32_t p = first[h]; p < first[h + 1]; ++p) {
         const float *in = part + (int64_t)p * stride;
         if (tid < T) {
@@ -281,7 +193,7 @@ cudaError_t launch_tiles(const SweepArgs &a, const Fp32Split *sp, cudaStream_t s
         // Up to eight rows an SM are a matter of latency: another warp shares the copies and, at
         // f <= 16, takes the right-hand side over.  With more rows it would take CTAs' places.
         // 1,000 x 500, f = 10, ten epochs: 0.57 -> 0.48 ms a training call; f = 24, 1,000 rows 53 -> 47 us.
-        const int more = patch_mode<P>(MODE) && n <= 8 * 152 ? 32 : 0;
+        const int more = tile::patched<P>() && n <= 8 * 152 ? 32 : 0;
         sweep_tile_kernel<MODE, P><<<(unsigned)n, nt + more, smem, st>>>(b, nb);
         if (launches) ++*launches;
     }
@@ -290,11 +202,8 @@ cudaError_t launch_tiles(const SweepArgs &a, const Fp32Split *sp, cudaStream_t s
 
 template <int P>
 cudaError_t launch_tiles_of(const SweepArgs &a, const Fp32Split *sp, cudaStream_t st, int *launches) {
-    switch (tile_mode_of(a.solve)) {
-    case TILE_LU: return launch_tiles<TILE_LU, P>(a, sp, st, launches);
-    case TILE_CG: return launch_tiles<TILE_CG, P>(a, sp, st, launches);
-    default: return launch_tiles<TILE_LDLT, P>(a, sp, st, launches);
-    }
+    return a.solve == ALS_SOLVE_LU ? launch_tiles<TILE_LU, P>(a, sp, st, launches)
+                                   : launch_tiles<TILE_LDLT, P>(a, sp, st, launches);
 }
 
 #define ALS_FP32_TILES(P)                                                                        \
