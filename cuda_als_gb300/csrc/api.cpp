@@ -789,10 +789,11 @@ extern "C" als_status als_csr_to_csc_device(const als_csr_view *csr, int32_t *co
         return set_global_error(ALS_ERR_INVALID_ARG, "shape out of range");
     cudaStream_t st = (cudaStream_t)stream;
     void *scratch = nullptr;
-    G_CUDA(cudaMallocAsync(&scratch, transpose_scratch_bytes(csr->rows, csr->cols, csr->nnz), st));
+    const bool in_place = transposes_in_place(*csr, row_idxs, vals);
+    G_CUDA(cudaMallocAsync(&scratch, transpose_scratch_bytes(csr->rows, csr->cols, csr->nnz, in_place), st));
     cudaError_t e = csr_to_csc_device(csr->rows, csr->cols, csr->nnz, csr->row_ptrs,
                                       csr->col_idxs, csr->vals, col_ptrs, row_idxs, vals, scratch,
-                                      st, nullptr, nullptr);
+                                      st, nullptr, nullptr, false, in_place);
     cudaFreeAsync(scratch, st);
     if (e != cudaSuccess)
         return set_global_error(ALS_ERR_CUDA, std::string("csr_to_csc: ") + cudaGetErrorString(e));

@@ -485,9 +485,22 @@ static bool transpose_packs(int64_t rows, int64_t cols) {
 
 // Two passes: a set of two words a rating (the rows of the CSR wait in the output's); one pass: the
 // rows; the general path: the rows, a set of three words and the sorted columns.  And the counters.
-size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz) {
-    const int arrays = !transpose_packs(rows, cols) ? 5 : passes_of(key_bits(cols)) == 2 ? 2 : 1;
-    return arrays * array_bytes(nnz) + counter_bytes(nnz);
+// In place, the outputs are written in the last pass only: two passes keep the rows in scratch too,
+// one pass takes copies of the columns and values.
+static int transpose_arrays(int64_t rows, int64_t cols, bool in_place) {
+    if (!transpose_packs(rows, cols)) return 5;
+    return in_place ? 3 : passes_of(key_bits(cols)) == 2 ? 2 : 1;
+}
+size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool in_place) {
+    return transpose_arrays(rows, cols, in_place) * array_bytes(nnz) + counter_bytes(nnz);
+}
+
+bool transposes_in_place(const als_csr_view &csr, const int32_t *ridx, const float *cval) {
+    auto shares = [&](const void *out) {
+        return share_words(out, csr.nnz, csr.col_idxs, csr.nnz) || share_words(out, csr.nnz, csr.vals, csr.nnz) ||
+               share_words(out, csr.nnz, csr.row_ptrs, csr.rows + 1);
+    };
+    return csr.nnz > 0 && (shares(ridx) || shares(cval));
 }
 
 cudaError_t expand_rows(int64_t rows, int64_t nnz, const int32_t *ptr, int32_t *coo_rows,
@@ -500,14 +513,26 @@ cudaError_t expand_rows(int64_t rows, int64_t nnz, const int32_t *ptr, int32_t *
 cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int32_t *ptr,
                               const int32_t *idx, const float *val, int32_t *cptr,
                               int32_t *ridx, float *cval, void *scratch, cudaStream_t st,
-                              int32_t *coo_rows_out, int32_t *perm_out, bool rows_ready) {
+                              int32_t *coo_rows_out, int32_t *perm_out, bool rows_ready,
+                              bool in_place) {
     if (nnz <= 0) return cudaMemsetAsync(cptr, 0, sizeof(int32_t) * (size_t)(cols + 1), st);
     const size_t arr = array_bytes(nnz);
     char *s = (char *)scratch;
     const int cb = key_bits(cols), rb = key_bits(rows), passes = passes_of(cb);
     const bool packs = transpose_packs(rows, cols), one = passes == 1;
-    int32_t *coo_rows = coo_rows_out ? coo_rows_out : packs && !one ? ridx : (int32_t *)s;
+    int32_t *coo_rows = coo_rows_out          ? coo_rows_out
+                        : !packs || one       ? (int32_t *)s
+                        : in_place            ? (int32_t *)(s + 2 * arr)
+                                              : ridx;
     cudaError_t e = cudaSuccess;
+    if (in_place && packs && one) {
+        e = cudaMemcpyAsync(s + arr, idx, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s + 2 * arr, val, sizeof(float) * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return e;
+        idx = (const int32_t *)(s + arr);
+        val = (const float *)(s + 2 * arr);
+    }
     if (!rows_ready) {
         e = expand_rows(rows, nnz, ptr, coo_rows, st);
         if (e != cudaSuccess) return e;
@@ -517,7 +542,7 @@ cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int
     uint32_t *v_out = (uint32_t *)(perm_out ? perm_out : (int32_t *)cval);
     if (packs) {
         uint32_t *word = (uint32_t *)s, *pay = (uint32_t *)(s + arr);  // (two passes only)
-        const Counters c = counters_at(s + (one ? 1 : 2) * arr, nnz);
+        const Counters c = counters_at(s + transpose_arrays(rows, cols, in_place) * arr, nnz);
         Move mv{};
         mv.key = (const uint32_t *)idx;
         mv.a = (const uint32_t *)coo_rows;
@@ -543,8 +568,10 @@ cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int
             passes, nnz, cols, tiles_of(nnz), word, rb, c.hist, c.totals[0], c.totals[one ? 0 : 1], cptr);
     } else {
         int32_t *skeys = (int32_t *)(s + arr);
+        // (an odd number of passes starts in the outputs: in place, one more over zero digits)
+        const int bits = in_place && passes % 2 ? passes * RADIX_BITS + 1 : cb;
         e = radix_sort_triples(idx, coo_rows, (const int32_t *)v_in, skeys, ridx, (int32_t *)v_out,
-                               nnz, cb, s + 2 * arr, st);
+                               nnz, bits, s + 2 * arr, st);
         if (e != cudaSuccess) return e;
         col_ptrs_from_sorted_kernel<<<grid_for(nnz + 1, 256), 256, 0, st>>>(nnz, cols, skeys, cptr);
     }
@@ -665,8 +692,9 @@ extern "C" als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int
     if (csr->rows < 0 || csr->cols < 0 || csr->nnz < 0 || csr->nnz > INT32_MAX ||
         csr->rows >= INT32_MAX || csr->cols >= INT32_MAX)
         return set_global_error(ALS_ERR_INVALID_ARG, "shape out of range");
+    const bool in_place = transposes_in_place(*csr, row_idxs, vals);
     if (csr->nnz > NOALLOC_MAX_RATINGS ||
-        transpose_scratch_bytes(csr->rows, csr->cols, csr->nnz) > NOALLOC_SCRATCH_BYTES)
+        transpose_scratch_bytes(csr->rows, csr->cols, csr->nnz, in_place) > NOALLOC_SCRATCH_BYTES)
         return set_global_error(
             ALS_ERR_INVALID_ARG,
             "als_csr_to_csc_device_noalloc: " + std::to_string(csr->nnz) + " ratings, more than the " +
@@ -699,7 +727,7 @@ extern "C" als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int
     }
     e = csr_to_csc_device(csr->rows, csr->cols, csr->nnz, csr->row_ptrs, csr->col_idxs,
                           csr->vals, col_ptrs, row_idxs, vals, scratch, (cudaStream_t)stream,
-                          nullptr, nullptr);
+                          nullptr, nullptr, false, in_place);
     if (e != cudaSuccess)
         return set_global_error(ALS_ERR_CUDA, std::string("csr_to_csc: ") + cudaGetErrorString(e));
     return ALS_OK;

@@ -58,14 +58,22 @@ constexpr int TILE_KEYS = 4096;
 size_t tile_counts_bytes(int64_t n);
 cudaError_t scan_tile_counts(int32_t *counts, int64_t n, int32_t *total, cudaStream_t st);
 
-// CSR -> CSC on the device, stable.  Scratch: transpose_scratch_bytes.
-size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz);
+// CSR -> CSC on the device, stable.  Scratch: transpose_scratch_bytes.  in_place: ridx or cval may
+// share memory with the inputs (transposes_in_place).
+size_t transpose_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool in_place = false);
+bool transposes_in_place(const als_csr_view &csr, const int32_t *ridx, const float *cval);
 cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int32_t *ptr,
                               const int32_t *idx, const float *val, int32_t *cptr,
                               int32_t *ridx, float *cval, void *scratch, cudaStream_t st,
                               int32_t *coo_rows_out /* optional, nnz */,
                               int32_t *perm_out /* optional, nnz: CSC position -> CSR position */,
-                              bool rows_ready = false /* coo_rows_out holds the rows already */);
+                              bool rows_ready = false /* coo_rows_out holds the rows already */,
+                              bool in_place = false /* no coo_rows_out, no perm_out */);
+// Whether n 32-bit words at a and k at b share memory.
+inline bool share_words(const void *a, int64_t n, const void *b, int64_t k) {
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + 4 * (uintptr_t)k && y < x + 4 * (uintptr_t)n;
+}
 
 // ptr[k] = first position of the ascending keys skeys[0..n) that is >= k, for k in [0, nkeys]
 // (the pointer array of sorted row or column indices).

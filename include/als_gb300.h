@@ -288,7 +288,8 @@ als_status als_user_halfsweep_adjoint_f64(als_handle *h, const als_coo_view *hel
 /* Stable CSR -> CSC transpose (rows inside each column ascending, i.e. the order scipy's
  * tocsc() produces).  The reference does this offline in scipy
  * (data/netflix/prepare_netflix_data.py:102-109, data/toy_data_2/prepare_toy_data_2.py:195-200).
- * HOST pointers; output arrays must hold cols+1 / nnz / nnz elements. */
+ * HOST pointers; output arrays must hold cols+1 / nnz / nnz elements.  In all three forms row_idxs and
+ * vals may be the CSR's own arrays. */
 als_status als_csr_to_csc(const als_csr_view *csr, int32_t *col_ptrs, int32_t *row_idxs,
                           float *vals);
 
