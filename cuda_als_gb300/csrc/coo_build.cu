@@ -152,12 +152,19 @@ emit_kernel(const Cells c, int64_t n, int64_t rows, const int32_t *__restrict__ 
 // Whether row and column share a 32-bit key.
 static bool coo_packs(int64_t rows, int64_t cols) { return key_bits(rows) + key_bits(cols) <= 32; }
 
+// Whether the CSC's arrays can hold entries between passes: not where they share memory with the
+// values, which the first pass reads (rows and columns are packed before it).
+static bool sorts_in_csc(int64_t nnz, const float *val, const int32_t *csc_rows, const float *csc_vals) {
+    return csc_rows && !share_words(csc_rows, nnz, val, nnz) && !share_words(csc_vals, nnz, val, nnz);
+}
+
 // Flags and heads per tile; then the sort's entries and counters, of which the transpose takes the
 // place.  Packed, the entries pass between one set of two words here and the arrays of the CSC
-// (scratch has to be mapped on every call: 0.34 ms of 1.44 for five arrays of 10.0M entries).
-size_t coo_build_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool csc) {
+// (scratch has to be mapped on every call: 0.34 ms of 1.44 for five arrays of 10.0M entries), or a
+// second set here.
+size_t coo_build_scratch_bytes(int64_t rows, int64_t cols, int64_t nnz, bool csc, bool in_csc) {
     const size_t arr = a256(sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1));
-    const size_t sort = coo_packs(rows, cols) ? (csc ? 2 : 4) * arr + radix_counter_bytes(nnz)
+    const size_t sort = coo_packs(rows, cols) ? (in_csc ? 2 : 4) * arr + radix_counter_bytes(nnz)
                                               : 6 * arr + radix_sort_scratch_bytes(nnz, 2);
     return 256 + a256(tile_counts_bytes(nnz)) +
            std::max(sort, csc ? transpose_scratch_bytes(rows, cols, nnz) : 0);
@@ -210,11 +217,12 @@ cudaError_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int
     Cells c{};
     c.col_bits = cb;
     if (packed) {
-        int32_t *const set[2][2] = {{col_ptrs ? csc_rows : array(2), col_ptrs ? (int32_t *)csc_vals : array(3)},
+        const bool in_csc = sorts_in_csc(nnz, val, csc_rows, csc_vals);
+        int32_t *const set[2][2] = {{in_csc ? csc_rows : array(2), in_csc ? (int32_t *)csc_vals : array(3)},
                                     {array(0), array(1)}};
         int last = 0;
-        e = radix_sort_between(array(0), (const int32_t *)val, set, nnz, rb + cb,
-                               array(col_ptrs ? 2 : 4), st, &last);
+        e = radix_sort_between(array(0), (const int32_t *)val, set, nnz, rb + cb, array(in_csc ? 2 : 4), st,
+                               &last);
         c.word = (const uint32_t *)set[last][0];
         c.val = (const float *)set[last][1];
     } else {
@@ -290,8 +298,9 @@ extern "C" als_status als_coo_to_csr_device(const als_coo_view *coo, int32_t *ro
     if (s != ALS_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     void *scratch = nullptr;
+    const bool in_csc = sorts_in_csc(coo->nnz, coo->vals, row_idxs, csc_vals);
     cudaError_t e = cudaMallocAsync(&scratch, coo_build_scratch_bytes(coo->rows, coo->cols, coo->nnz,
-                                                                      col_ptrs != nullptr), st);
+                                                                      col_ptrs != nullptr, in_csc), st);
     if (e != cudaSuccess) return cuda_fail("cudaMallocAsync", e);
     int bad = 0;
     e = coo_to_csr_device(coo->rows, coo->cols, coo->nnz, coo->row_idxs, coo->col_idxs,
@@ -323,7 +332,7 @@ extern "C" als_status als_coo_to_csr(const als_coo_view *coo, int32_t *row_ptrs,
     // inputs (3 nnz), CSR (rows + 1, 2 nnz), COO rows (nnz), CSC (cols + 1, 2 nnz), scratch
     const size_t a_in = 3 * a256(n4), a_csr = a256(sizeof(int32_t) * (rows + 1)) + 2 * a256(n4);
     const size_t a_rows = a256(n4), a_csc = a256(sizeof(int32_t) * (cols + 1)) + 2 * a256(n4);
-    const size_t a_scr = coo_build_scratch_bytes(rows, cols, nnz, col_ptrs != nullptr);
+    const size_t a_scr = coo_build_scratch_bytes(rows, cols, nnz, col_ptrs != nullptr, col_ptrs != nullptr);
     e = cudaMalloc(&buf, a_in + a_csr + a_rows + a_csc + a_scr);
     if (e != cudaSuccess) {
         cudaStreamDestroy(st);

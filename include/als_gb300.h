@@ -326,7 +326,7 @@ als_status als_coo_to_csr(const als_coo_view *coo, int32_t *row_ptrs, int32_t *c
 /* Same, DEVICE pointers, enqueued on `stream` (cudaStream_t as void*), scratch allocated with
  * cudaMallocAsync on it; synchronous (the count after summing duplicates sizes the later
  * launches and is returned in *nnz_out, host memory).  The CSC's arrays also serve as scratch:
- * their entries past the count are undefined. */
+ * their entries past the count are undefined.  They may be the triples' own arrays. */
 als_status als_coo_to_csr_device(const als_coo_view *coo, int32_t *row_ptrs, int32_t *col_idxs,
                                  float *vals, int32_t *coo_rows, int32_t *col_ptrs,
                                  int32_t *row_idxs, float *csc_vals, int64_t *nnz_out,
