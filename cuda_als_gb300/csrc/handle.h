@@ -56,10 +56,12 @@ struct als_handle {
     uint64_t wait_ns = 0;  // bound of the sweep kernels' device waits (0: the default, 10 s)
     std::vector<cudaEvent_t> events;
     cudaEvent_t ev_half[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    // one ALS epoch (U then V half-sweep) captured once the kernel plan is final, replayed by
+    // the U half-sweep, the V half-sweep and both, captured once the kernel plan is final, replayed by
     // als_iterate; dropped whenever a pointer, the data or the plan changes
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
+    struct Replay {
+        cudaGraphExec_t exec = nullptr;
+        int64_t launches = 0;  // its kernels
+    } replay[3];
     int64_t eager_epochs = 0;  // epochs run without a graph since the last invalidation
                                // (capture waits for the first one)
     // kernel plan per side: buckets (rebuilt when the ratings change), half-sweeps since the

@@ -46,6 +46,7 @@ als_status prepare_precision_path(als_handle *h) {
 void release_split(als_handle *h);
 
 void release_precision_path(als_handle *h) {
+    invalidate_graphs(h);
     release_split(h);
     release_adjoint(h, true);
     for (int s = 0; s < 2; ++s)
@@ -55,10 +56,10 @@ void release_precision_path(als_handle *h) {
 }
 
 void invalidate_graphs(als_handle *h) {
-    if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
-    if (h->graph) cudaGraphDestroy(h->graph);
-    h->graph_exec = nullptr;
-    h->graph = nullptr;
+    for (auto &r : h->replay) {
+        if (r.exec) cudaGraphExecDestroy(r.exec);
+        r = als_handle::Replay();
+    }
     // the next capture waits for one eager epoch on the new state, so a reload followed by a
     // single epoch (the e2e pattern) pays for no capture and instantiation
     h->eager_epochs = 0;
@@ -139,7 +140,7 @@ static void build_plan(als_handle *h, int side) {
     }
 }
 
-// The ratings changed (creation, reload): drop the graph and the buckets; an autotuned side keeps
+// The ratings changed (creation, reload): drop the graphs and the buckets; an autotuned side keeps
 // its per-class solver choice and applies it to the new buckets.
 void data_changed(als_handle *h) {
     invalidate_graphs(h);
@@ -405,45 +406,60 @@ als_status read_stage_ms(als_handle *h, int side) {
     return ALS_OK;
 }
 
+// Capture the U half-sweep (0), the V half-sweep (1) or an epoch (2), without timing events, unless
+// it is captured already.
+static als_status capture(als_handle *h, int what) {
+    cudaStream_t st = h->stream;
+    als_handle::Replay &r = h->replay[what];
+    if (r.exec) return ALS_OK;
+    S_CUDA(h, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    als_status s = ALS_OK;
+    r.launches = 0;
+    for (int side = what == 1 ? 1 : 0; side < (what == 0 ? 1 : 2) && s == ALS_OK; ++side) {
+        s = run_half_sweep(h, side, false);
+        r.launches += h->counters[0];
+    }
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(st, &g);
+    if (s == ALS_OK && e == cudaSuccess) e = cudaGraphInstantiate(&r.exec, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (s != ALS_OK) return s;
+    S_CUDA(h, e);
+    return ALS_OK;
+}
+
 // `iters` epochs.  Once the kernel plan is final (first epoch run; under ALS_SOLVE_AUTO the
-// tuning sweeps done) and use_graph is set, an epoch is captured into a CUDA graph once and
-// replayed: one launch call per epoch instead of one per kernel and memset.  The last epoch is
-// launched eagerly, between the events that time its half-sweeps: as nodes of the graph they cost
-// every epoch about 6 us a half-sweep (1,000 x 500, f = 10, ten epochs:
-// 0.65 -> 0.55 ms a training call).
+// tuning sweeps done) and use_graph is set, epochs are replayed from CUDA graphs: one launch call
+// per epoch instead of one per kernel and memset.  The last epoch is replayed by halves, between
+// the events that time them: as nodes of the epoch's graph they cost every epoch about 6 us a
+// half-sweep (1,000 x 500, f = 10, ten epochs: 0.65 -> 0.55 ms a training call), and by halves
+// throughout an epoch costs 2 us more.
 als_status run_epochs(als_handle *h, int32_t iters) {
     cudaStream_t st = h->stream;
-    int epoch_launches = 0;
     for (int32_t it = 0; it < iters; ++it) {
-        const bool graphable = h->cfg.use_graph && h->eager_epochs > 0 && plan_final(h) &&
-                               it + 1 < iters;
-        if (graphable && !h->graph_exec) {
-            S_CUDA(h, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            als_status s = run_half_sweep(h, 0, false);
-            epoch_launches = (int)h->counters[0];
-            if (s == ALS_OK) s = run_half_sweep(h, 1, false);
-            epoch_launches += (int)h->counters[0];
-            cudaGraph_t g = nullptr;
-            const cudaError_t e = cudaStreamEndCapture(st, &g);
-            if (s != ALS_OK) {
-                if (g) cudaGraphDestroy(g);
-                return s;
-            }
-            S_CUDA(h, e);
-            h->graph = g;
-            S_CUDA(h, cudaGraphInstantiate(&h->graph_exec, g, 0));
-            h->counters[0] = epoch_launches;
-        }
-        if (graphable) {
-            S_CUDA(h, cudaGraphLaunch(h->graph_exec, st));
-        } else {
+        if (!(h->cfg.use_graph && h->eager_epochs > 0 && plan_final(h))) {
             als_status s = run_half_sweep(h, 0);
             if (s != ALS_OK) return s;
-            int launches = (int)h->counters[0];
+            const int64_t launches = h->counters[0];
             s = run_half_sweep(h, 1);
             if (s != ALS_OK) return s;
             h->counters[0] += launches;
             ++h->eager_epochs;
+        } else if (it + 1 < iters) {
+            const als_status s = capture(h, 2);
+            if (s != ALS_OK) return s;
+            S_CUDA(h, cudaGraphLaunch(h->replay[2].exec, st));
+        } else {
+            for (int side = 0; side < 2; ++side) {
+                const als_status s = capture(h, side);
+                if (s != ALS_OK) return s;
+            }
+            for (int side = 0; side < 2; ++side) {
+                S_CUDA(h, record_event(h->ev_half[side][0], st));
+                S_CUDA(h, cudaGraphLaunch(h->replay[side].exec, st));
+                S_CUDA(h, record_event(h->ev_half[side][1], st));
+            }
+            h->counters[0] = h->replay[0].launches + h->replay[1].launches;
         }
     }
     return ALS_OK;
@@ -462,7 +478,7 @@ als_status check_sweep_flags(als_handle *h) {
 extern "C" als_status als_set_wait_limit_ns(als_handle *h, uint64_t ns) {
     if (!h) return set_global_error(ALS_ERR_INVALID_ARG, "null handle");
     h->wait_ns = ns;
-    invalidate_graphs(h);  // the limit is a kernel argument captured in the epoch graph
+    invalidate_graphs(h);  // the limit is a kernel argument captured in the graphs
     return ALS_OK;
 }
 
