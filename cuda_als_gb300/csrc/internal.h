@@ -107,15 +107,6 @@ cudaError_t count_bad_entries(int64_t nnz, const int32_t *idx, int32_t limit, co
 // Sweep kernels
 // ---------------------------------------------------------------------------------------------
 
-// Record `ev` on `st`; while `st` is being captured into a graph the record becomes an
-// event-record node of the graph (cudaEventRecordExternal), so replays time themselves.
-inline cudaError_t record_event(cudaEvent_t ev, cudaStream_t st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &cs);
-    return cs == cudaStreamCaptureStatusActive ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal)
-                                               : cudaEventRecord(ev, st);
-}
-
 struct SweepArgs {
     const int32_t *ptr;     // rows + 1 (this side's CSR)
     const int32_t *idx;     // nnz, indices into the opposite table

@@ -364,7 +364,7 @@ static als_status tune_side(als_handle *h, int side, int *launches) {
 als_status run_half_sweep(als_handle *h, int side, bool timed) {
     cudaStream_t st = h->stream;
     if (h->plan[side].empty()) build_plan(h, side);
-    if (timed) S_CUDA(h, record_event(h->ev_half[side][0], st));
+    if (timed) S_CUDA(h, cudaEventRecord(h->ev_half[side][0], st));
     int launches = 0;
     if (h->precision != ALS_PREC_FP32) {
         std::string why;
@@ -389,7 +389,7 @@ als_status run_half_sweep(als_handle *h, int side, bool timed) {
             k = last + 1;
         }
     }
-    if (timed) S_CUDA(h, record_event(h->ev_half[side][1], st));
+    if (timed) S_CUDA(h, cudaEventRecord(h->ev_half[side][1], st));
     h->counters[0] = launches;
     return ALS_OK;
 }
@@ -455,9 +455,9 @@ als_status run_epochs(als_handle *h, int32_t iters) {
                 if (s != ALS_OK) return s;
             }
             for (int side = 0; side < 2; ++side) {
-                S_CUDA(h, record_event(h->ev_half[side][0], st));
+                S_CUDA(h, cudaEventRecord(h->ev_half[side][0], st));
                 S_CUDA(h, cudaGraphLaunch(h->replay[side].exec, st));
-                S_CUDA(h, record_event(h->ev_half[side][1], st));
+                S_CUDA(h, cudaEventRecord(h->ev_half[side][1], st));
             }
             h->counters[0] = h->replay[0].launches + h->replay[1].launches;
         }
