@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(512) adjoint_tile_kernel(const AdjArgs<float> 
         no_gradient();
         return;
     }
-    if (tid == 0) *s.bad = *s.wide = 0;
+    if (tid == 0) *s.bad = 0;
     const tile::Tile t = tile::tile_of<P>(tid, nb, false);
     tile::Acc acc;
     tile::clear(acc);

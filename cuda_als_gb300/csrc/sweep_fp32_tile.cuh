@@ -48,7 +48,7 @@ __device__ __forceinline__ void tile_solve(const SweepArgs &a, int nb, int row, 
     float *xo = a.X + (int64_t)row * f;
     tile::add_diagonal(acc, t, f, (float)nu * a.lambda);  // items_cnt * lambda (als_model.cu:157-159)
     const tile::Shared s = tile::carve<P>(smem, nb, MODE == TILE_LU);
-    if (tid == 0) *s.bad = *s.wide = 0;
+    if (tid == 0) *s.bad = 0;
     if (rhs) *reinterpret_cast<float2 *>(s.vb + 2 * rt) = b;
     for (int i = f + (f & 1) + tid; i < 8 * nb; i += blockDim.x) s.vb[i] = 0.f;
     if (MODE == TILE_LU) tile::mirror(acc, t, nb, s);

@@ -1,5 +1,6 @@
 """The reciprocals and quotients of the register-tile solvers against CUDA's division, and the solvers
-against the column-at-a-time ones, bit for bit over the exponent range (tests/cpp/tile_check.cu)."""
+against the column-at-a-time ones: bit for bit over their range of pivots, and by their errors against
+FP64 beyond (tests/cpp/tile_check.cu)."""
 from __future__ import annotations
 
 import subprocess
