@@ -29,6 +29,7 @@
 
 #include "handle.h"
 #include "internal.h"
+#include "ratings.h"
 #include "solvers.cuh"
 #include "tc.h"
 #include "tilesolve.cuh"
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 512 : 1024)
             xr[i] = T(0);
             gr[i] = T(0);
         }
-        for (int e = hbeg + tid; e < hend; e += nt) loss += (double)a.hval[e] * a.hval[e];
+        for (uint32_t e = hbeg + tid; e < (uint32_t)hend; e += nt) loss += (double)a.hval[e] * a.hval[e];
         const double s = block_sum_d(loss, dsh);
         if (tid == 0) {
             a.loss_part[row] = s;
@@ -146,8 +147,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 512 : 1024)
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[p][c] = T(0);
     T bsum = T(0), bcomp = T(0);  // b_tid: compensated sum of 32-rating chunk sums
-    for (int base = beg; base < end; base += KC) {
-        const int cnt = min(KC, end - base);
+    for (int left = nu; left > 0; left -= KC) {
+        const int cnt = min(KC, left), base = end - left;
         if (tid < KC) {
             scol[tid] = tid < cnt ? a.idx[base + tid] : -1;
             sval[tid] = tid < cnt ? (T)a.val[base + tid] : T(0);
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(512) adjoint_tile_kernel(const AdjArgs<float> 
             xr[i] = 0.f;
             gr[i] = 0.f;
         }
-        for (int e = hbeg + tid; e < hend; e += nt) loss += (double)a.hval[e] * a.hval[e];
+        for (uint32_t e = hbeg + tid; e < (uint32_t)hend; e += nt) loss += (double)a.hval[e] * a.hval[e];
         const double l = block_sum_d(loss, dsh);
         if (tid == 0) {
             a.loss_part[row] = l;
@@ -423,22 +424,24 @@ __global__ void __launch_bounds__(32 * ITEM_WARPS)
             }
         };
         // AHEAD entries' rows in flight, then their contributions in order
-        const int end = cend[ch];
-        for (int e0 = cbeg[ch] + warp; e0 < end; e0 += AHEAD * ITEM_WARPS) {
+        const int len = cend[ch] - cbeg[ch];  // (at most ITEM_CHUNK)
+        const int32_t *usr = cusr + cbeg[ch];
+        const float *val = cval + cbeg[ch];
+        for (int e0 = warp; e0 < len; e0 += AHEAD * ITEM_WARPS) {
             T xu[AHEAD][ITEM_Q], gu[AHEAD][ITEM_Q], c[AHEAD];
 #pragma unroll
             for (int k = 0; k < AHEAD; ++k) {
                 const int e = e0 + k * ITEM_WARPS;
-                if (e < end) {  // (warp-uniform)
-                    const int64_t u = cusr[e];
-                    c[k] = (T)cval[e];
+                if (e < len) {  // (warp-uniform)
+                    const int64_t u = usr[e];
+                    c[k] = (T)val[e];
                     load(X + u * f, xu[k]);
                     load(G + u * f, gu[k]);
                 }
             }
 #pragma unroll
             for (int k = 0; k < AHEAD; ++k) {
-                if (e0 + k * ITEM_WARPS >= end) continue;
+                if (e0 + k * ITEM_WARPS >= len) continue;
                 const T yx = dot(xu[k]), gy = dot(gu[k]);
                 const T ck = c[k] - yx;
 #pragma unroll
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(32 * ITEM_WARPS)
             }
         }
         if (first) {
-            for (int e = hptr[it] + warp; e < hptr[it + 1]; e += ITEM_WARPS) {
+            for (uint32_t e = hptr[it] + warp; e < (uint32_t)hptr[it + 1]; e += ITEM_WARPS) {
                 T xu[ITEM_Q];
                 load(X + (int64_t)husr[e] * f, xu);
                 const T res = (T)hval[e] - dot(xu);
@@ -550,19 +553,20 @@ cudaError_t build_chunks(als_handle *h) {
     const int64_t n = h->n;
     int64_t nchunks = 0;
     for (int64_t i = 0; i < n; ++i)
-        nchunks += std::max<int64_t>(1, ((int64_t)cp[i + 1] - cp[i] + ITEM_CHUNK - 1) / ITEM_CHUNK);
+        nchunks += std::max<int64_t>(1, parts_of(cp[i], cp[i + 1], ITEM_CHUNK));
     std::vector<int32_t> tab((size_t)(3 * nchunks + n + 1));
     int32_t *citem = tab.data(), *cbeg = citem + nchunks, *cend = cbeg + nchunks, *cfirst = cend + nchunks;
     int64_t c = 0;
     for (int64_t i = 0; i < n; ++i) {
         cfirst[i] = (int32_t)c;
-        int32_t s = cp[i];
+        uint32_t s = cp[i];
+        const uint32_t end = cp[i + 1];
         do {
             citem[c] = (int32_t)i;
-            cbeg[c] = s;
-            cend[c++] = std::min(cp[i + 1], s + ITEM_CHUNK);
+            cbeg[c] = (int32_t)s;
+            cend[c++] = (int32_t)(s + part_ratings(s, end, ITEM_CHUNK));
             s += ITEM_CHUNK;
-        } while (s < cp[i + 1]);
+        } while (s < end);
     }
     cfirst[n] = (int32_t)c;
     cudaError_t e = cudaMalloc(&ad.d_chunks, sizeof(int32_t) * tab.size());
@@ -698,7 +702,7 @@ als_status adjoint_impl(als_handle *h, const als_coo_view *held, const T *d_Y, T
         a.lambda = lambda;
         bool tiles = false;
         if constexpr (sizeof(T) == 4) {
-            tiles = tile::fits(f);
+            tiles = tile::fits(f) && h->nnz <= tile::MAX_RATINGS;
             if (tiles && e == cudaSuccess && m > 0) {
                 switch (tile::pitch_of(f)) {
                 case 32: step(launch_rows<32>(a, m, st)); break;

@@ -291,8 +291,8 @@ __global__ void expand_rows_kernel(int64_t rows, int64_t nnz, const int32_t *__r
     int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = warp; r < rows; r += nwarps) {
-        int32_t b = max(0, min((int32_t)nnz, ptr[r])), e = max(b, min((int32_t)nnz, ptr[r + 1]));
-        for (int32_t k = b + lane; k < e; k += 32) coo_rows[k] = (int32_t)r;
+        const int32_t b = max(0, min((int32_t)nnz, ptr[r])), e = max(b, min((int32_t)nnz, ptr[r + 1]));
+        for (uint32_t k = b + lane; k < (uint32_t)e; k += 32) coo_rows[k] = (int32_t)r;
     }
 }
 

@@ -114,6 +114,7 @@ struct SweepArgs {
     const float *Y;         // opposite factors, FP32, row-contiguous (f per row)
     float *X;               // this side's factors (in: CG warm start, out: solution)
     const int32_t *order;   // row processing order (NULL = identity)
+    int64_t nnz;            // ratings of the matrix
     int32_t row_begin;      // slice [row_begin, row_end) of the order
     int32_t row_end;
     int32_t f;

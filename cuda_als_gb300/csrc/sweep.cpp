@@ -14,6 +14,7 @@
 
 #include "handle.h"
 #include "internal.h"
+#include "ratings.h"
 #include "tc.h"
 
 using namespace als;
@@ -191,9 +192,10 @@ static cudaError_t build_split(als_handle *h, int side) {
     std::vector<int32_t> pbeg, pend;
     sp.first.assign(1, 0);
     for (int32_t r : heavy) {
-        for (int32_t b = ptr[r]; b < ptr[r + 1]; b += FP32_SPLIT_RATINGS) {
-            pbeg.push_back(b);
-            pend.push_back(std::min(ptr[r + 1], b + FP32_SPLIT_RATINGS));
+        const uint32_t end = ptr[r + 1];
+        for (uint32_t b = ptr[r]; b < end; b += FP32_SPLIT_RATINGS) {
+            pbeg.push_back((int32_t)b);
+            pend.push_back((int32_t)(b + part_ratings(b, end, FP32_SPLIT_RATINGS)));
         }
         sp.first.push_back((int32_t)pbeg.size());
     }
@@ -230,6 +232,7 @@ static cudaError_t launch_bucket(als_handle *h, int side, const SweepBucket &b, 
     a.Y = side == 0 ? h->d_V : h->d_U;
     a.X = side == 0 ? h->d_U : h->d_V;
     a.order = h->d_order[side];
+    a.nnz = h->nnz;
     a.row_begin = b.lo;
     a.row_end = b.hi;
     a.f = h->f;

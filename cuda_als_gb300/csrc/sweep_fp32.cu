@@ -12,11 +12,13 @@
 // the Gram lives in shared memory only.
 //
 // Two layouts.  The direct solvers at f <= 175: the matrix in registers, one 8 x 8 tile a thread
-// (tilesolve.cuh).  Larger f (a tile a thread would take more than 512 threads of 128 registers) and
-// CG at every f: the "wide" kernels, 4 x 8 register tiles for the Gram, which is stored to shared
-// memory (stride FP + 1, conflict-free column walks) and solved there.  CG reads its matrix from
-// shared memory in every product, so it gains nothing from tiles in registers and lost CTAs to
-// them (17,504 rows of 48,369 ratings at f = 120: 1.13 ms here, 2.55 on 8 x 8 tiles).  Both do the same arithmetic in the same order: each Gram entry is one
+// (tilesolve.cuh).  Larger f (a tile a thread would take more than 512 threads of 128 registers),
+// matrices within 128 ratings of 2^31 (the tiles' index loads look ahead in 32 bits) and CG at every
+// f: the "wide" kernels, 4 x 8 register tiles for the Gram, which is stored to shared memory (stride
+// FP + 1, conflict-free column walks) and solved there.  CG reads its matrix from shared memory in
+// every product, so it gains nothing from tiles in registers and lost CTAs to them (17,504 rows of
+// 48,369 ratings at f = 120: 1.13 ms here, 2.55 on 8 x 8 tiles).  Both do the same arithmetic in the
+// same order: each Gram entry is one
 // sequential FMA chain over the row's ratings, in rating order (the order of the reference's
 // calculate_vtvs, als_model.cu:137-155).  The right-hand side is summed apart, more accurately:
 // thread j sums r_k y_kj over each 32 ratings and adds those sums with compensated (Kahan)
@@ -118,8 +120,8 @@ __device__ void accumulate(const SweepArgs &a, int FP, int beg, int end, const T
                            int32_t *scol, float *sval) {
     const int f = a.f;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    for (int base = beg; base < end; base += KC) {
-        const int cnt = min(KC, end - base);
+    for (int left = end - beg; left > 0; left -= KC) {
+        const int cnt = min(KC, left), base = end - left;
         if (tid < KC) {
             scol[tid] = tid < cnt ? a.idx[base + tid] : -1;
             sval[tid] = tid < cnt ? a.val[base + tid] : 0.f;
@@ -288,7 +290,7 @@ bool fp32_supported(int f) { return f >= 1 && fp_of(f) <= MAX_FP; }
 cudaError_t launch_sweep_fp32(const SweepArgs &a, const Fp32Split *sp, cudaStream_t st,
                               int *launches) {
     const bool cg = a.solve == ALS_SOLVE_CG_FP32 || a.solve == ALS_SOLVE_CG_FP16;
-    if (tile::fits(a.f) && !cg) {
+    if (tile::fits(a.f) && !cg && a.nnz <= tile::MAX_RATINGS) {
         switch (tile::pitch_of(a.f)) {
         case 32: return launch_tiles_32(a, sp, st, launches);
         case 64: return launch_tiles_64(a, sp, st, launches);

@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "ratings.h"
 #include "regsolve.cuh"
 #include "solvers.cuh"
 
@@ -1159,18 +1160,18 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
             while (ok && ccnt > 0) {
                 for (int j = 0; j < ccnt && ok; ++j) {
                     const int row = __shfl_sync(0xffffffffu, crow, j);
-                    const int beg = __shfl_sync(0xffffffffu, cbeg, j);
-                    const int end = __shfl_sync(0xffffffffu, cend, j);
-                    int base = beg;
+                    const uint32_t beg = __shfl_sync(0xffffffffu, cbeg, j);
+                    const uint32_t end = __shfl_sync(0xffffffffu, cend, j);
+                    uint32_t base = beg;
                     do {  // (a row without ratings is one empty stage)
                         const int room = space();
                         if (room <= 0) { ok = false; break; }
-                        const int n = min(max(1, (end - base + KC - 1) / KC), min(room, 32));
+                        const int n = min(max(1, (int)parts_of(base, end, KC)), min(room, 32));
                         if (lane < n) {
-                            const int b = base + lane * KC;
-                            const int flags = (b == beg ? 1 : 0) | (b + KC >= end ? 2 : 0);
+                            const uint32_t b = base + lane * KC;
+                            const int flags = (b == beg ? 1 : 0) | (part_is_last(b, end, KC) ? 2 : 0);
                             desc[(gen + lane) % MR] =
-                                make_int4(row, b, end - beg, min(KC, end - b) | flags << 16);
+                                make_int4(row, (int)b, (int)(end - beg), (int)part_ratings(b, end, KC) | flags << 16);
                         }
                         __threadfence_block();
                         __syncwarp();
