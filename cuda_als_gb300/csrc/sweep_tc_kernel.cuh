@@ -1153,7 +1153,8 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                         if (__shfl_sync(0xffffffffu, stop, 0)) return 0;
                     }
                 }
-                __threadfence_block();
+                __threadfence_block();  // the slots' reads, then this warp's writes
+                __syncwarp();
                 return limit - gen;
             };
             bool ok = true;
@@ -1348,9 +1349,14 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                         }
                     }
                 }
+                // lane 0's acquire, and its count, hold for every lane from here: all read one descriptor
+                __syncwarp();
                 d = desc[t % MR];
                 __syncwarp();
-                if (lane == 0) done[h] = (int)(t + NGATHER);  // the slot may be refilled
+                if (lane == 0) {  // read by every lane: the slot may be refilled
+                    __threadfence_block();
+                    done[h] = (int)(t + NGATHER);
+                }
                 const int cnt = d.w & 0xffff;  // the ragged tail gathers the all-zero row
                 const int32_t *ip = p.idx + d.y + lane;
                 const float *vp = p.val + d.y + lane;
