@@ -570,9 +570,11 @@ cudaError_t build_chunks(als_handle *h) {
     }
     cfirst[n] = (int32_t)c;
     cudaError_t e = cudaMalloc(&ad.d_chunks, sizeof(int32_t) * tab.size());
-    if (e == cudaSuccess)
-        e = cudaMemcpy(ad.d_chunks, tab.data(), sizeof(int32_t) * tab.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return e;
+    if (e == cudaSuccess) e = upload(h->stream, ad.d_chunks, tab.data(), tab.size());
+    if (e != cudaSuccess) {
+        release_adjoint(h, false);
+        return e;
+    }
     ad.nchunks = nchunks;
     ad.built = true;
     return cudaSuccess;

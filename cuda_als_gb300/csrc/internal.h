@@ -69,6 +69,13 @@ cudaError_t csr_to_csc_device(int64_t rows, int64_t cols, int64_t nnz, const int
                               int32_t *perm_out /* optional, nnz: CSC position -> CSR position */,
                               bool rows_ready = false /* coo_rows_out holds the rows already */,
                               bool in_place = false /* no coo_rows_out, no perm_out */);
+// Host words to the device, there for whatever `st` runs next, `src` free to go.  (cudaMemcpy from
+// pageable memory may return before the data has arrived, and a stream created non-blocking does
+// not wait for it.)
+inline cudaError_t upload(cudaStream_t st, int32_t *dst, const int32_t *src, size_t n) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
 // Whether n 32-bit words at a and k at b share memory.
 inline bool share_words(const void *a, int64_t n, const void *b, int64_t k) {
     const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;

@@ -167,12 +167,13 @@ static bool plan_final(const als_handle *h) {
     return true;
 }
 
+static void release(als_handle::Split &sp) {
+    if (sp.d_tab) cudaFree(sp.d_tab);
+    if (sp.d_part) cudaFree(sp.d_part);
+    sp = als_handle::Split();
+}
 void release_split(als_handle *h) {
-    for (auto &sp : h->split) {
-        if (sp.d_tab) cudaFree(sp.d_tab);
-        if (sp.d_part) cudaFree(sp.d_part);
-        sp = als_handle::Split();
-    }
+    for (auto &sp : h->split) release(sp);
 }
 
 // The FP32 path's heavy rows of a side (degree > FP32_SPLIT_RATINGS): the first positions of the
@@ -206,14 +207,13 @@ static cudaError_t build_split(als_handle *h, int side) {
         cudaError_t e = cudaMalloc(&sp.d_tab, sizeof(int32_t) * (2 * np + sp.first.size()));
         if (e == cudaSuccess)
             e = cudaMalloc(&sp.d_part, sizeof(float) * np * fp32_part_floats(h->f));
-        if (e == cudaSuccess)
-            e = cudaMemcpy(sp.d_tab, pbeg.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(sp.d_tab + np, pend.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(sp.d_tab + 2 * np, sp.first.data(), sizeof(int32_t) * sp.first.size(),
-                           cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return e;
+        if (e == cudaSuccess) e = upload(h->stream, sp.d_tab, pbeg.data(), np);
+        if (e == cudaSuccess) e = upload(h->stream, sp.d_tab + np, pend.data(), np);
+        if (e == cudaSuccess) e = upload(h->stream, sp.d_tab + 2 * np, sp.first.data(), sp.first.size());
+        if (e != cudaSuccess) {
+            release(sp);
+            return e;
+        }
     }
     sp.built = true;
     return cudaSuccess;

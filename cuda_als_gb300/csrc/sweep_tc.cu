@@ -181,7 +181,7 @@ als_status tc_prepare(als_handle *h, std::string *why) {
     for (int s = 0; s < 2 && t->f8; ++s) {
         const size_t bytes = (size_t)tcg::F8_ROW_BYTES * (size_t)(opp[s] + 1);
         if (cudaMalloc(&t->d_f8[s], bytes) != cudaSuccess ||
-            cudaMemset(t->d_f8[s], 0, bytes) != cudaSuccess ||
+            cudaMemsetAsync(t->d_f8[s], 0, bytes, h->stream) != cudaSuccess ||
             cudaMalloc(&t->d_scale[s], sizeof(float) * tcg::MAXF) != cudaSuccess) {
             *why = "out of memory for the FP8 factor tables";
             return ALS_ERR_OUT_OF_MEMORY;
@@ -194,7 +194,7 @@ als_status tc_prepare(als_handle *h, std::string *why) {
     for (int s = 0; s < 2 && !t->f8; ++s) {
         const size_t bytes = sizeof(__nv_bfloat16) * (size_t)(opp[s] + 1) * t->geo[0].fst;
         if (cudaMalloc(&t->d_bf[s], bytes) != cudaSuccess ||
-            cudaMemset(t->d_bf[s], 0, bytes) != cudaSuccess) {
+            cudaMemsetAsync(t->d_bf[s], 0, bytes, h->stream) != cudaSuccess) {
             *why = "out of memory for the BF16 factor tables";
             return ALS_ERR_OUT_OF_MEMORY;
         }
