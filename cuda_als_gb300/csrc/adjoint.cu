@@ -594,8 +594,15 @@ als_status bad_heldout(const als_handle *h, const als_coo_view *held) {
                                                      std::to_string(first_bad_heldout(h, held)));
 }
 
-// Writes a byte of every page back as it is.
+// Writes a byte of every page back as it is, where p is pageable host memory (page-locked memory is
+// mapped already, and what CUDA allocated elsewhere is not the host's to write).
 void touch_pages(void *p, size_t bytes) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (a.type != cudaMemoryTypeUnregistered) return;
     volatile char *c = static_cast<volatile char *>(p);
     for (size_t i = 0; i < bytes; i += 4096) c[i] = c[i];
     if (bytes) c[bytes - 1] = c[bytes - 1];
