@@ -161,6 +161,15 @@ def load_traffic(args, side, prec_name):
     return None
 
 
+def traffic_source(solve):
+    """What load_traffic's figure was measured on.  The captures of the autotuned plan's workload are
+    of one solver each, not of the plan's launches."""
+    of = ("one launch over the whole side with the solver that takes most of it in the autotuned plan, "
+          "a stand-in for the plan's launches" if solve == "auto" else "this workload's half-sweep launches")
+    return ("recorded: profiles/dram_traffic.txt (ncu dram__bytes_read.sum + dram__bytes_write.sum of "
+            f"{of}), not measured in this run")
+
+
 def measure_rows(model, make, time_epochs, tr, te, info, peak_hbm):
     """Times of the path's other rows on this workload, through the public API (host wall time
     around synchronous calls, after a warm call; median of 5 where a call is short):
@@ -592,9 +601,7 @@ def run_ours(args):
     roofline = {"bound": "tensor", "achieved": round(achieved, 3), "peak": peak_bf16,
                 "unit": "TFLOP/s", "frac": round(achieved / peak_bf16, 4),
                 "traffic": traffic,
-                "traffic_source": "recorded: profiles/dram_traffic.txt (ncu dram__bytes_read.sum + "
-                                  "dram__bytes_write.sum of this workload's half-sweep launches), "
-                                  "not measured in this run" if traffic is not None else None,
+                "traffic_source": traffic_source(args.solve) if traffic is not None else None,
                 "kernel": f"fused half-sweep ({dom_side} side: BF16 quantise + one sweep_tc_kernel "
                           f"launch per nnz bucket), Gram+RHS flops nnz*f*(f+1)+2*nnz*f over its "
                           f"CUDA-event time averaged over the {iters} epochs of a configured run",
