@@ -13,7 +13,8 @@
 //     L D L^T factor, the forward solve, the row's held-out terms (in order: h_u and the loss),
 //     the second solve with the same factor; writes x_u and g_u, the loss and dL/dlambda parts.
 //     The tile kernel keeps the matrix in registers (tilesolve.cuh), the row kernel factors it in
-//     shared memory a column at a time; FP32 results are the same to the bit.
+//     shared memory a column at a time; FP32 results are the same to the bit (for pivots in
+//     tilesolve.cuh's range of quotients).  Matrices within 128 ratings of 2^31 take the row kernel.
 //   adjoint_chunk_kernel + adjoint_combine_kernel: dL/dy_i from the item's training column (the
 //     CSC) in chunks of 2,048 ratings (one CTA each: heavy items spread over many) and its
 //     held-out ratings; every sum in a fixed order (warps, then chunks): deterministic, no

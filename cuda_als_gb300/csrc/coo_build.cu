@@ -154,7 +154,8 @@ static bool coo_packs(int64_t rows, int64_t cols) { return key_bits(rows) + key_
 
 // Whether the CSC's arrays can hold entries between passes: not where they share memory with the
 // values, which the first pass reads (rows and columns are packed before it).
-static bool sorts_in_csc(int64_t nnz, const float *val, const int32_t *csc_rows, const float *csc_vals) {
+static bool sorts_in_csc(int64_t nnz, const float *val, const int32_t *csc_rows,
+                         const float *csc_vals) {
     return csc_rows && !share_words(csc_rows, nnz, val, nnz) && !share_words(csc_vals, nnz, val, nnz);
 }
 

@@ -86,7 +86,8 @@ struct als_handle {
     } split[2];
 
     // adjoint: chunk table of the item side (built from the ratings, dropped when they change) and
-    // device workspace (grown to the largest call, kept until als_destroy)
+    // device workspace (grown to the largest call, kept until als_destroy: about 8 (m + n) f bytes,
+    // twice that for FP64 calls)
     struct Adjoint {
         bool built = false;
         int64_t nchunks = 0;

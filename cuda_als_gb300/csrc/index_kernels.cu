@@ -128,10 +128,10 @@ struct Move {
 
 // Stable scatter.  Warp w of tile t owns the contiguous key range [t*4096 + w*256, +256) and
 // walks it in 8 rounds of 32; a key's rank inside its warp is (keys of the same digit in earlier
-// rounds) + (lanes below it with the same digit in this round), found with a ballot a digit bit.  The warp
-// offsets per digit are an exclusive prefix over warps on top of the tile's digit starts (a scan
-// over digits).  The entries are first placed in shared memory in digit order (the tile sorted by
-// digit), then streamed out: consecutive threads write consecutive addresses of a digit's run, so
+// rounds) + (lanes below it with the same digit in this round), found with a ballot a digit bit.
+// The warp offsets per digit are an exclusive prefix over warps on top of the tile's digit starts (a
+// scan over digits).  The entries are first placed in shared memory in digit order (the tile sorted
+// by digit), then streamed out: consecutive threads write consecutive addresses of a digit's run, so
 // the global stores coalesce instead of scattering 32 ways per instruction.  hist: every digit's
 // tile counts, scanned; totals: every digit's count (its start is scanned here).
 // Shared memory sets the pace (random 8-byte stores, then rows of a digit), so a transpose moves

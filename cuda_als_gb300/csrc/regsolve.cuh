@@ -13,8 +13,8 @@
 //   chol_fac      Cholesky A = L L^T of the Gram copied to a packed lower triangle in shared
 //                 memory, left-looking in blocks of 8 columns, with the forward solve beside it:
 //                 the dot products are spread over the threads as (row, column half) items,
-//                 one thread factors each 8 x 8 diagonal block in registers and eight lanes invert
-//                 it, three barriers per block.
+//                 every lane of one warp factors each 8 x 8 diagonal block in registers and eight
+//                 of them invert it, two barriers per block.
 //   chol_forward, chol_backward  L y = b and L^T x = y by the group, one barrier per 16 rows.
 // Sums over threads are combined in a fixed order (deterministic).
 #pragma once
@@ -132,7 +132,7 @@ __device__ float cg_reg(const float (&a)[FP], float bi, float xi, int i, float *
     return cg_single_reduction(mul, bi, xi, red, iters, tol, gs);
 }
 
-// CG as cg_reg with the rows quad-blocked (FP = 112).  The four lanes 4a..4a+3 of a warp share
+// CG as cg_reg with the rows quad-blocked (FP = 64, 112, 128).  The four lanes 4a..4a+3 of a warp share
 // rows 4a..4a+3: lane 4a+c holds columns 16k+4c..16k+4c+3 (k < NK = FP/16) of all four, rows 4a
 // and 4a+1 in registers (ar[0], ar[1]), rows 4a+2 and 4a+3 in shared memory (slots 2k and 2k+1
 // of `sa`, the thread's own float4 in each).  A product reads FP/4 floats of p a thread, one
@@ -201,12 +201,13 @@ struct TriLayout {
     static constexpr int floats = 32 * (FP / 8) * (FP / 8 + 1) + 4 * FP;
 };
 
-// Cholesky A = L L^T of the leading n x n matrix (n a multiple of 16) held in Ls (packed, tri_off rows; entry (i, j)
-// for j <= i must be set, the rest of each row's blocks is scratch), and the forward solve L y = b
-// beside it: `bv` holds b on entry (n floats, scratch afterwards), `yv` receives y.  On exit entry
-// (i, j) left of the diagonal blocks holds L[i][j], Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for
-// r >= c (the inverse of each 8 x 8 diagonal block) and invd[j] = 1 / L[j][j].  Called by the 128
-// threads of a group (et = 0..127); warp `lead` / 32 works on the diagonal blocks.
+// Cholesky A = L L^T of the leading n x n matrix (n a multiple of 16) held in Ls (packed, tri_off
+// rows; entry (i, j) for j <= i must be set, the rest of each row's blocks is scratch), and the
+// forward solve L y = b beside it: `bv` holds b on entry (n floats, scratch afterwards), `yv`
+// receives y.  On exit entry (i, j) left of the diagonal blocks holds L[i][j],
+// Dv[K * 64 + r * 8 + c] = (L_KK^-1)[r][c] for r >= c (the inverse of each 8 x 8 diagonal block) and
+// invd[j] = 1 / L[j][j].  Called by the 128 threads of a group (et = 0..127); warp `lead` / 32 works
+// on the diagonal blocks.
 //
 // Left-looking in blocks of 8 columns, two barriers per block:
 //  (a) the block's entries lose L[r][0:k0] . L[k0+4h+kk][0:k0], a (row, column half) item a thread,
@@ -220,12 +221,12 @@ struct TriLayout {
 // 98.6M ratings, ms at f = 64 / 100 / 128: 24.0 / 50.9 / 91.5 with separate solves and work dealt
 // from warp 0 (and one buffer less at 128), then 18.0 / 36.1 / 51.8; with (b)'s factor no longer
 // passed from one lane to the inverting ones through shared memory f = 64 15.8, and 100,000 rows of
-// 9.0M ratings at f = 100 / 128 7.39 / 10.61 -> 6.69 / 9.50; with (b) beside the other warps' (a) f = 64
-// 15.4, 100,000 rows 6.59 / 8.98.  Two rows an item in (a): 18.8 / 38.5 /
-// 53.8; (a) for the next block by the warps that idle in (b): 19.1 / 38.2 / 50.5.
-// Returns false (on thread lead) if a pivot was not positive and finite.
-__device__ __forceinline__ bool chol_fac(int et, int n, int lead, float *Ls, float *Dv, float *invd, float *bv, float *yv,
-                         const GroupSync &gs) {
+// 9.0M ratings at f = 100 / 128 7.39 / 10.61 -> 6.69 / 9.50; with (b) beside the other warps' (a)
+// f = 64 15.4, 100,000 rows 6.59 / 8.98.  Two rows an item in (a): 18.8 / 38.5 / 53.8; (a) for the
+// next block by the warps that idle in (b): 19.1 / 38.2 / 50.5.
+// Returns false (on the lead warp's lanes) if a pivot was not positive and finite.
+__device__ __forceinline__ bool chol_fac(int et, int n, int lead, float *Ls, float *Dv, float *invd,
+                                         float *bv, float *yv, const GroupSync &gs) {
     constexpr int B = 8;
     bool ok = true;
     const int ev = (et + 128 - lead) & 127;

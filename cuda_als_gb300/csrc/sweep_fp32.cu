@@ -18,11 +18,11 @@
 // FP + 1, conflict-free column walks) and solved there.  CG reads its matrix from shared memory in
 // every product, so it gains nothing from tiles in registers and lost CTAs to them (17,504 rows of
 // 48,369 ratings at f = 120: 1.13 ms here, 2.55 on 8 x 8 tiles).  Both do the same arithmetic in the
-// same order: each Gram entry is one
-// sequential FMA chain over the row's ratings, in rating order (the order of the reference's
-// calculate_vtvs, als_model.cu:137-155).  The right-hand side is summed apart, more accurately:
-// thread j sums r_k y_kj over each 32 ratings and adds those sums with compensated (Kahan)
-// addition, so b_u carries about one rounding instead of the n_u of a sequential sum.
+// same order: each Gram entry is one sequential FMA chain over the row's ratings, in rating order
+// (the order of the reference's calculate_vtvs, als_model.cu:137-155).  The right-hand side is summed
+// apart, more accurately: thread j sums r_k y_kj over each 32 ratings and adds those sums with
+// compensated (Kahan) addition, so b_u carries about one rounding instead of the n_u of a sequential
+// sum.
 // (An FP32 sequential right-hand side costs ALS up to 4x in accuracy against FP64 after ten
 // iterations at f = 100-128: its error meets the Gram's condition number in every solve.)
 #include <cuda_runtime.h>
@@ -163,8 +163,8 @@ __device__ void accumulate(const SweepArgs &a, int FP, int beg, int end, const T
     }
 }
 
-// The wide kernels: from the finished Gram tiles and b: regularise, solve with the selected solver (CG warm-started
-// from the current x), write x (or x = 0 and a flag for a non-SPD / non-finite row).
+// The wide kernels: from the finished Gram tiles and b: regularise, solve with the selected solver
+// (CG warm-started from the current x), write x (or x = 0 and a flag for a non-SPD / non-finite row).
 __device__ void solve_and_write(const SweepArgs &a, int FP, int row, int nu, const Tile &t,
                                 const float (&acc)[4][8], float b_tid, float *smem) {
     const int f = a.f, GS = FP + 1, tid = threadIdx.x;

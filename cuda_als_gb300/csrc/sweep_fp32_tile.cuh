@@ -192,7 +192,8 @@ cudaError_t launch_tiles(const SweepArgs &a, const Fp32Split *sp, cudaStream_t s
     if (n > 0) {
         // Up to eight rows an SM are a matter of latency: another warp shares the copies and, at
         // f <= 16, takes the right-hand side over.  With more rows it would take CTAs' places.
-        // 1,000 x 500, f = 10, ten epochs: 0.57 -> 0.48 ms a training call; f = 24, 1,000 rows 53 -> 47 us.
+        // 1,000 x 500, f = 10, ten epochs: 0.57 -> 0.48 ms a training call; f = 24, 1,000 rows 53 ->
+        // 47 us.
         const int more = tile::patched<P>() && n <= 8 * 152 ? 32 : 0;
         sweep_tile_kernel<MODE, P><<<(unsigned)n, nt + more, smem, st>>>(b, nb);
         if (launches) ++*launches;

@@ -95,11 +95,11 @@ __host__ __device__ constexpr int nepi_of(int solver, int fp) {
 // Gather warps: six take a stage in the time of its MMAs (two: V half of 98.6M ratings at f = 100
 // with the FP32 CG 5.69 ms, six 3.57).  A launch's registers are shared out per four warps, so
 // above 640 threads a thread keeps 80 and at 640 it keeps 96.  The tensor-core CG (80 a thread)
-// takes five, as many as its ring has stages; the Cholesky factor and LU (96 and more) two.  The quad-blocked CG
-// splits its registers (setmaxnreg): launched with six gather warps at 80 a thread (FP = 128, three
-// groups: 96), its solver warpgroups take 96 (128) and the two service warpgroups (producer, MMA
-// issuer, gather warps) give theirs back down to SERVICE_REGS, the sum being exactly what the
-// launch holds (launch_regs_of x threads).
+// takes five, as many as its ring has stages; the Cholesky factor and LU (96 and more) two.  The
+// quad-blocked CG splits its registers (setmaxnreg): launched with six gather warps at 80 a thread
+// (FP = 128, three groups: 96), its solver warpgroups take 96 (128) and the two service warpgroups
+// (producer, MMA issuer, gather warps) give theirs back down to SERVICE_REGS, the sum being exactly
+// what the launch holds (launch_regs_of x threads).
 __host__ __device__ constexpr bool regsplit_of(int solver, int fp) {
     return cg_quad_rows(solver, fp);
 }
@@ -231,7 +231,7 @@ inline Geometry geometry(int f, int solver, bool f8 = false) {
     size_t bytes = (size_t)ns * stage_bytes(solver, g.fp, f8);                     // operand ring
     bytes += sizeof(float) * group_floats(g.fp, solver) * g.nepi;    // per-group scratch
     if (f8) bytes += sizeof(float) * MAXF;                            // per-feature scales
-    bytes += MRING_BYTES;                                            // metadata ring
+    bytes += MRING_BYTES;                                            // descriptors, ids
     bytes += 1024;                                                   // metas, barriers, scalars
     g.smem = bytes + 1024;                                           // 1024-B alignment slack
     return g;
@@ -1171,8 +1171,8 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                         if (lane < n) {
                             const uint32_t b = base + lane * KC;
                             const int flags = (b == beg ? 1 : 0) | (part_is_last(b, end, KC) ? 2 : 0);
-                            desc[(gen + lane) % MR] =
-                                make_int4(row, (int)b, (int)(end - beg), (int)part_ratings(b, end, KC) | flags << 16);
+                            desc[(gen + lane) % MR] = make_int4(
+                                row, (int)b, (int)(end - beg), (int)part_ratings(b, end, KC) | flags << 16);
                         }
                         __threadfence_block();
                         __syncwarp();
@@ -1349,7 +1349,8 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                         }
                     }
                 }
-                // lane 0's acquire, and its count, hold for every lane from here: all read one descriptor
+                // lane 0's acquire and its count hold for every lane from here: all read one
+                // descriptor (a lane with another would leave the warp's full-mask shuffles)
                 __syncwarp();
                 d = desc[t % MR];
                 __syncwarp();

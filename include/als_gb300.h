@@ -268,7 +268,10 @@ als_status als_get_tuning(const als_handle *h, int32_t side, float *ms_cg, float
  * user half-sweep given Y = V.  Computes X (written to the handle's U), L, dL/dY (n*f floats,
  * host) and dL/dlambda by solving A_u g_u = dL/dx_u with each row's L D L^T factor, in FP32.
  * dL/dY is summed per item over its ratings in a fixed order (deterministic).
- * `heldout` is a host COO view (rows index U, cols index V). */
+ * `heldout` is a host COO view (rows index U, cols index V).  The handle keeps the call's device
+ * workspace for the next one, up to the largest so far, until als_destroy: x_u, g_u and dL/dY with
+ * its partial sums, about 4 (2 m + 2 n) f bytes here (0.35 GB at 283,228 x 58,098, f = 128) and twice
+ * that in FP64, and 44 bytes a held-out rating. */
 als_status als_user_halfsweep_adjoint(als_handle *h, const als_coo_view *heldout, double *loss,
                                       float *dLdY, double *dLdlambda);
 
@@ -302,9 +305,10 @@ als_status als_csr_to_csc_device(const als_csr_view *csr, int32_t *col_ptrs, int
  * device memory (a plug-in inside an engine that owns all device memory, an allocation-free
  * latency-critical loop).  No counterpart in the reference.  Scratch is a fixed 16 MiB device
  * array inside this library; at most 593,856 ratings are accepted (28 bytes each plus 1 KiB per
- * 4,096) and larger inputs are rejected with ALS_ERR_INVALID_ARG.  The first call in each CUDA context looks the
- * array up (again after a device reset); all calls share the array, so calls that overlap on the
- * GPU race and must be serialised by the caller.  DEVICE pointers, enqueued on `stream`. */
+ * 4,096) and larger inputs are rejected with ALS_ERR_INVALID_ARG.  The first call in each CUDA
+ * context looks the array up (again after a device reset); all calls share the array, so calls that
+ * overlap on the GPU race and must be serialised by the caller.  DEVICE pointers, enqueued on
+ * `stream`. */
 als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int32_t *col_ptrs,
                                          int32_t *row_idxs, float *vals, void *stream);
 
@@ -342,9 +346,10 @@ als_status als_degree_order(int64_t rows, const int32_t *row_ptrs, int32_t *perm
  * row_weight (the solve's cost in rating-equivalents; 0 = balance ratings only).  Part k gets rows
  * [bounds[k], bounds[k+1]), bounds[0] = 0, bounds[nparts] = rows; boundary k falls where the
  * running weight crosses k/nparts of the total (a row goes to the earlier part when its midpoint
- * lies before that point), so every boundary is within half a row's weight of its target.  Replaces the reference's equal-count m_batches / n_batches split
- * (als_model.cu:1891-1896) for sharding a half-sweep over ranks.  Host work, HOST pointers:
- * row_ptrs (rows + 1) in, bounds (nparts + 1) out. */
+ * lies before that point), so every boundary is within half a row's weight of its target.  Replaces
+ * the reference's equal-count m_batches / n_batches split (als_model.cu:1891-1896) for sharding a
+ * half-sweep over ranks.  Host work, HOST pointers: row_ptrs (rows + 1) in, bounds (nparts + 1)
+ * out. */
 als_status als_partition_rows(int64_t rows, const int32_t *row_ptrs, int32_t nparts,
                               double row_weight, int64_t *bounds);
 
