@@ -30,6 +30,7 @@
 #include <stdint.h>
 
 #include "internal.h"
+#include "ratings.h"
 #include "solvers.cuh"
 #include "sweep_fp32_tile.cuh"
 
@@ -120,8 +121,9 @@ __device__ void accumulate(const SweepArgs &a, int FP, int beg, int end, const T
                            int32_t *scol, float *sval) {
     const int f = a.f;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    for (int left = end - beg; left > 0; left -= KC) {
-        const int cnt = min(KC, left), base = end - left;
+    int base = beg;
+    for (int n = (int)parts_of(beg, end, KC); n > 0; --n, base = (int)((uint32_t)base + KC)) {
+        const int cnt = min(KC, end - base);
         if (tid < KC) {
             scol[tid] = tid < cnt ? a.idx[base + tid] : -1;
             sval[tid] = tid < cnt ? a.val[base + tid] : 0.f;
