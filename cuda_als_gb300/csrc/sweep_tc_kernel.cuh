@@ -307,7 +307,8 @@ __device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, vol
         }
     }
 }
-// A shared-memory word written after what it announces (__threadfence_block before the store).
+// A shared-memory word written after what it announces (st_release, or __threadfence_block before
+// the store).
 __device__ __forceinline__ uint32_t ld_acquire(const volatile int *word) {
     uint32_t v;
     asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];"
@@ -315,6 +316,11 @@ __device__ __forceinline__ uint32_t ld_acquire(const volatile int *word) {
                  : "r"(smem_u32(const_cast<const int *>(word)))
                  : "memory");
     return v;
+}
+__device__ __forceinline__ void st_release(volatile int *word, int v) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(const_cast<const int *>(word))),
+                 "r"(v)
+                 : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -957,7 +963,7 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
     // (ng = 128) has no free column: a second, N = 16 MMA against the rating tile.  FP8 stages
     // take the e4m3 rating into byte ng of each 128-byte row: one MMA per 32 ratings.
     constexpr bool FUSED = fused_of(FP);
-    static_assert(NGATHER <= MAX_NGATHER && NGATHER <= NSTAGE, "");
+    static_assert(NGATHER <= MAX_NGATHER && NGATHER <= NSTAGE && NSTAGE + 2 * NGATHER <= MR, "");
     // Register split: setmaxnreg acts per warpgroup, so the solver warps and the service warps
     // each form whole warpgroups, and the registers the solvers take are exactly those the
     // service warps give back out of the launch's own (a larger .inc would wait forever; the host
@@ -1353,11 +1359,6 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                 // descriptor (a lane with another would leave the warp's full-mask shuffles)
                 __syncwarp();
                 d = desc[t % MR];
-                __syncwarp();
-                if (lane == 0) {  // read by every lane: the slot may be refilled
-                    __threadfence_block();
-                    done[h] = (int)(t + NGATHER);
-                }
                 const int cnt = d.w & 0xffff;  // the ragged tail gathers the all-zero row
                 const int32_t *ip = p.idx + d.y + lane;
                 const float *vp = p.val + d.y + lane;
@@ -1397,6 +1398,11 @@ __global__ void __launch_bounds__(nthreads_of(SOLVER, FP), 1)
                     rv[e] = vv[e];
                 }
                 __syncwarp();
+                // Every lane has read stage t's descriptor: the producer may refill its slot.  (Here
+                // and by st.release: a __threadfence_block directly behind the read cost the
+                // Cholesky's two gather warps 4%, FP8 at f = 48 397 -> 414 us.  A stage still waiting
+                // for its ring slot is at most NSTAGE - 1 behind, so MR leaves the others room.)
+                if (lane == 0) st_release(done + h, (int)(t + NGATHER));
                 go = take(t + NGATHER);  // the next stage's ids and ratings, behind this one
                 uint8_t *tile = ring + s * SBYTES;
                 // the MMA reads ratings [0, 16 n16) (the ragged tail's column ids point at the
