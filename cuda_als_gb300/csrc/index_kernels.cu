@@ -15,6 +15,7 @@
 #include <mutex>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "internal.h"
 
@@ -637,10 +638,11 @@ cudaError_t count_bad_entries(int64_t nnz, const int32_t *idx, int32_t limit, co
 // In host code the array's name is only a host-side stand-in, so the device address is looked up
 // with cudaGetSymbolAddress (with the device current) on the first call made in each CUDA
 // context, and looked up again when the device's context changes (after cudaDeviceReset the
-// module reloads at another address).  Every call shares the one array: calls whose work
-// overlaps on the GPU (different streams, or several threads) race on it and must be serialised
-// by the caller.  The transpose writes every scratch word before it reads it, so no clearing is
-// needed between calls.
+// module reloads at another address).  Every call shares the one array, so each waits on the GPU for
+// the one before, whatever its stream or thread: an event recorded behind every call (two calls
+// that overlapped could take places from each other's counters, past the end of the outputs).  A call
+// under stream capture is not ordered that way; replays of its graph must not overlap other calls.
+// The transpose writes every scratch word before it reads it, so no clearing is needed between calls.
 // ---------------------------------------------------------------------------------------------
 
 namespace {
@@ -651,9 +653,14 @@ constexpr int NOALLOC_MAX_DEVICES = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
+// A device's array as one CUDA context sees it (an entry of a context that is gone never matches).
+struct NoallocSite {
+    unsigned long long ctx;  // cuCtxGetId; 0 where it is unavailable: looked up again each time
+    void *addr;
+    cudaEvent_t done;        // behind the last call's work (none without an id)
+};
 std::mutex g_noalloc_mu;
-void *g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};
-unsigned long long g_noalloc_ctx[NOALLOC_MAX_DEVICES] = {};  // cuCtxGetId of the lookup's context
+std::vector<NoallocSite> g_noalloc_sites[NOALLOC_MAX_DEVICES];
 
 // The unique id of the calling thread's current CUDA context (cuCtxGetCurrent + cuCtxGetId
 // through the runtime's driver entry points; no link against libcuda); 0 if unavailable.
@@ -707,27 +714,36 @@ extern "C" als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int
         return set_global_error(ALS_ERR_NO_DEVICE, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     if (dev < 0 || dev >= NOALLOC_MAX_DEVICES)
         return set_global_error(ALS_ERR_UNSUPPORTED, "device ordinal beyond 63");
-    void *scratch = nullptr;
-    {
-        // cudaGetDevice made the device's primary context current if it was not yet
-        const unsigned long long ctx = current_context_id();
-        std::lock_guard<std::mutex> lock(g_noalloc_mu);
-        if (!g_noalloc_addr[dev] || ctx == 0 || ctx != g_noalloc_ctx[dev]) {
-            // set-up, once per device and context, with that device current
-            void *addr = nullptr;
-            e = cudaGetSymbolAddress(&addr, g_noalloc_scratch);
-            if (e != cudaSuccess || !addr)
-                return set_global_error(ALS_ERR_CUDA,
-                                        std::string("cudaGetSymbolAddress: ") +
-                                            cudaGetErrorString(e));
-            g_noalloc_addr[dev] = addr;
-            g_noalloc_ctx[dev] = ctx;
-        }
-        scratch = g_noalloc_addr[dev];
+    cudaStream_t st = (cudaStream_t)stream;
+    // cudaGetDevice made the device's primary context current if it was not yet
+    const unsigned long long ctx = current_context_id();
+    std::lock_guard<std::mutex> lock(g_noalloc_mu);  // until the call is enqueued
+    NoallocSite site{0, nullptr, nullptr};
+    for (const NoallocSite &k : g_noalloc_sites[dev])
+        if (ctx != 0 && k.ctx == ctx) site = k;
+    if (!site.addr) {  // set-up, once per device and context, with that device current
+        e = cudaGetSymbolAddress(&site.addr, g_noalloc_scratch);
+        if (e == cudaSuccess && ctx != 0) e = cudaEventCreateWithFlags(&site.done, cudaEventDisableTiming);
+        if (e != cudaSuccess || !site.addr)
+            return set_global_error(ALS_ERR_CUDA, std::string("the scratch array's address: ") +
+                                                      cudaGetErrorString(e));
+        site.ctx = ctx;
+        if (ctx != 0) g_noalloc_sites[dev].push_back(site);
     }
-    e = csr_to_csc_device(csr->rows, csr->cols, csr->nnz, csr->row_ptrs, csr->col_idxs,
-                          csr->vals, col_ptrs, row_idxs, vals, scratch, (cudaStream_t)stream,
-                          nullptr, nullptr, false, in_place);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool known = cudaStreamIsCapturing(st, &capture) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    const bool ordered = site.done && known && capture == cudaStreamCaptureStatusNone;
+    if (ordered) e = cudaStreamWaitEvent(st, site.done, 0);
+    if (e == cudaSuccess)
+        e = csr_to_csc_device(csr->rows, csr->cols, csr->nnz, csr->row_ptrs, csr->col_idxs,
+                              csr->vals, col_ptrs, row_idxs, vals, site.addr, st, nullptr, nullptr,
+                              false, in_place);
+    // (behind whatever was enqueued, also when a later launch failed)
+    if (ordered) {
+        const cudaError_t r = cudaEventRecord(site.done, st);
+        if (e == cudaSuccess) e = r;
+    }
     if (e != cudaSuccess)
         return set_global_error(ALS_ERR_CUDA, std::string("csr_to_csc: ") + cudaGetErrorString(e));
     return ALS_OK;

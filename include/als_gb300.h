@@ -306,9 +306,10 @@ als_status als_csr_to_csc_device(const als_csr_view *csr, int32_t *col_ptrs, int
  * latency-critical loop).  No counterpart in the reference.  Scratch is a fixed 16 MiB device
  * array inside this library; at most 593,856 ratings are accepted (28 bytes each plus 1 KiB per
  * 4,096) and larger inputs are rejected with ALS_ERR_INVALID_ARG.  The first call in each CUDA
- * context looks the array up (again after a device reset); all calls share the array, so calls that
- * overlap on the GPU race and must be serialised by the caller.  DEVICE pointers, enqueued on
- * `stream`. */
+ * context looks the array up (again after a device reset); all calls share the array, so each waits
+ * on the GPU for the one before, whatever its stream or thread.  Calls under stream capture are not
+ * ordered: replays of their graph must be serialised with other calls by the caller.  DEVICE
+ * pointers, enqueued on `stream`. */
 als_status als_csr_to_csc_device_noalloc(const als_csr_view *csr, int32_t *col_ptrs,
                                          int32_t *row_idxs, float *vals, void *stream);
 
